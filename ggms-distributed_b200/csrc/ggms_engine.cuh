@@ -15,6 +15,8 @@
 #pragma once
 #include "ggms_host.cuh"
 #include "ggms_kernels.cuh"
+#include "ggms_refine.cuh"
+#include "ggms_direct.cuh"
 #include "ggms_learned.cuh"
 #include "ggms_window.cuh"
 
@@ -50,21 +52,22 @@ struct Workspace {
   uint32_t* knext;        // per k: next k in its segment's list
   uint32_t* smalls;       // ids of the small segments the current level created
   uint32_t* tinies;       // ids of the tiny segments the current level created
-  uint32_t* bigs[2];      // per pool: the segments a level refines (batched level 0: quantile ones)
+  uint32_t* bigs[2];      // per pool: the segments a level refines, by row (batched level 0: quantile ones)
   K* qtab;                // ... their boundaries [cap_q][QB]
   uint16_t* qdir;         // ... their directories [cap_q][QDS]
   K* points;
   K* cand[2];
-  void* out_dev;
   size_t bytes;
 };
 
 
 template <typename K>
-static Workspace<K> layout(const Plan& p, size_t out_elem_bytes, uint8_t* base) {
+static Workspace<K> layout(const Plan& p, uint8_t* base) {
   Bump b;
   Workspace<K> w;
+  static_assert(sizeof(Counters) <= ARENA_BAR, "the barrier word follows the counters");
   size_t o_C = b.take(sizeof(Counters));
+  b.take(256);  // ARENA_BAR
   size_t o_kin = b.take(4ull * p.nk);
   size_t o_krank = b.take(4ull * p.nk);
   size_t o_kseg = b.take(4ull * p.nk);
@@ -87,7 +90,7 @@ static Workspace<K> layout(const Plan& p, size_t out_elem_bytes, uint8_t* base) 
   size_t o_smalls = b.take(4ull * p.cap_seg);
   size_t o_tinies = b.take(4ull * p.cap_seg);
   size_t o_bigs[2];
-  for (int i = 0; i < 2; ++i) o_bigs[i] = b.take(4ull * p.cap_seg);
+  for (int i = 0; i < 2; ++i) o_bigs[i] = b.take(4ull * p.cap_rows);
   size_t o_qtab = b.take(sizeof(K) * QB * p.cap_q);
   size_t o_qdir = b.take(2ull * QDS * p.cap_q);
   for (int i = 0; i < 2; ++i) {
@@ -95,12 +98,11 @@ static Workspace<K> layout(const Plan& p, size_t out_elem_bytes, uint8_t* base) 
     o_segs[i] = b.take(sizeof(Seg<K>) * p.cap_seg);
     o_cur[i] = b.take(4ull * p.cap_seg);
     o_tiles[i] = b.take(sizeof(TileRef) * p.cap_tiles);
-    o_rows[i] = b.take(4ull * NBIN * p.cap_seg);
-    o_af[i] = b.take(4ull * NBIN_WORDS * p.cap_seg);
+    o_rows[i] = b.take(4ull * NBIN * p.cap_rows);
+    o_af[i] = b.take(4ull * NBIN_WORDS * p.cap_rows);
   }
   size_t o_pts = b.take(sizeof(K) * p.nk);
   for (int i = 0; i < 2; ++i) o_cand[i] = b.take(sizeof(K) * p.n);
-  size_t o_out = b.take(out_elem_bytes * p.nk);
   w.bytes = b.take(0) + 256;
   if (!base) return w;
   w.C = (Counters*)(base + o_C);
@@ -138,78 +140,46 @@ static Workspace<K> layout(const Plan& p, size_t out_elem_bytes, uint8_t* base) 
   w.qtab = (K*)(base + o_qtab);
   w.qdir = (uint16_t*)(base + o_qdir);
   w.points = (K*)(base + o_pts);
-  w.out_dev = (void*)(base + o_out);
   return w;
 }
 
 
-// The refinement levels first..maxlev (1-based) of the single-vector path.
-// Captured into a graph, level l becomes an IF node and level l + 1 is nested
-// inside its body, so a level without segments skips every later level at
-// the cost of one conditional node.  The condition of the first level is set
-// by an earlier kernel (handle `first`, created by level_handle()); the later
-// ones by lvl_gate at the end of the enclosing level.  Run directly, the
-// levels' kernels are launched as they are (each returns at once when there
-// is no work).  body(stream, l) enqueues level l's kernels.
-static int level_handle(cudaStream_t s, cudaGraphConditionalHandle* h) {
-  *h = 0;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  GGMS_CU(cudaStreamIsCapturing(s, &cs));
-  if (cs != cudaStreamCaptureStatusActive) return GGMS_OK;
-  cudaGraph_t g = nullptr;
-  GGMS_CU(cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, nullptr, nullptr));
-  GGMS_CU(cudaGraphConditionalHandleCreate(h, g, 0u, cudaGraphCondAssignDefault));
-  return GGMS_OK;
-}
-
-template <typename F>
-static int enqueue_levels(Context* c, cudaStream_t s, Counters* C, int l, int maxlev,
-                          cudaGraphConditionalHandle first, F&& body) {
-  if (l > maxlev) return GGMS_OK;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  GGMS_CU(cudaStreamIsCapturing(s, &cs));
-  if (cs != cudaStreamCaptureStatusActive) {
-    const int rc = body(s, l);
-    if (rc) return rc;
-    return enqueue_levels(c, s, C, l + 1, maxlev, 0, body);
+// The arguments of refine_levels over a workspace: the levels from 1 on, then
+// the answers to `out` (device or pinned memory).
+template <typename T>
+static RefineArgs<T> refine_args(const Workspace<typename KeyOf<T>::K>& w, const Context* c, uint32_t nk, Caps caps,
+                                 T* out, Counters* report) {
+  RefineArgs<T> a;
+  a.C = w.C;
+  a.bar = (uint32_t*)(c->arena + ARENA_BAR);
+  for (int i = 0; i < 2; ++i) {
+    a.cand[i] = w.cand[i];
+    a.segs[i] = w.segs[i];
+    a.tiles[i] = w.tiles[i];
+    a.rows[i] = w.rows[i];
+    a.aflag[i] = w.aflag[i];
+    a.bigs[i] = w.bigs[i];
+    a.cursor[i] = w.cursor[i];
+    a.khead[i] = w.khead[i];
   }
-  if (l > Context::MAX_NEST) return GGMS_E_INTERNAL;
-  cudaGraph_t g = nullptr;
-  const cudaGraphNode_t* deps = nullptr;
-  size_t nd = 0;
-  cudaGraphConditionalHandle h = first;
-  if (!h) {
-    GGMS_CU(cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, &nd));
-    GGMS_CU(cudaGraphConditionalHandleCreate(&h, g, 0u, cudaGraphCondAssignDefault));
-    ++c->launches;
-    lvl_gate<<<1, 1, 0, s>>>(C, l & 1, h);
-  }
-  GGMS_CU(cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, &nd));
-  cudaGraphNodeParams np = {};
-  np.type = cudaGraphNodeTypeConditional;
-  np.conditional.handle = h;
-  np.conditional.type = cudaGraphCondTypeIf;
-  np.conditional.size = 1;
-  cudaGraphNode_t cn;
-  GGMS_CU(cudaGraphAddNode(&cn, g, deps, nd, &np));
-  cudaStream_t& bs = c->bodies[l - 1];
-  if (!bs) GGMS_CU(cudaStreamCreateWithFlags(&bs, cudaStreamNonBlocking));
-  GGMS_CU(cudaStreamBeginCaptureToGraph(bs, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                        cudaStreamCaptureModeThreadLocal));
-  int rc = body(bs, l);
-  if (!rc) rc = enqueue_levels(c, bs, C, l + 1, maxlev, 0, body);
-  cudaGraph_t out = nullptr;
-  const cudaError_t e = cudaStreamEndCapture(bs, &out);
-  if (rc) return rc;
-  GGMS_CU(e);
-  GGMS_CU(cudaStreamUpdateCaptureDependencies(s, &cn, 1, cudaStreamSetCaptureDependencies));
-  return GGMS_OK;
+  a.knext = w.knext;
+  a.smalls = w.smalls;
+  a.tinies = w.tinies;
+  a.krank = w.krank;
+  a.kseg = w.kseg;
+  a.kbin = w.kbin;
+  a.points = w.points;
+  a.kkey = w.kkey;
+  a.nk = nk;
+  a.caps = caps;
+  a.caps.tiny_keys = RF_TINY / sizeof(typename KeyOf<T>::K);  // of the levels' children
+  a.out = out;
+  a.report = report;
+  return a;
 }
 
 // ------------------------------------------------------------------ kernel configs
 constexpr int LV_NT = 256;
-constexpr int MAX_LEVELS_32 = 3;
-constexpr int MAX_LEVELS_64 = 6;
 
 template <typename T>
 static size_t l0_count_smem(uint32_t B, int nt, int unroll, uint32_t nst) {
@@ -334,7 +304,7 @@ static int launch_small_select(Context* ctx, const InT* src, const Seg<K>* segs_
                                const Workspace<K>& w, const Caps& caps, cudaStream_t st,
                                const int64_t* k_off = nullptr) {
   static bool attr = false;
-  const size_t sm = SMALL_SMEM + (size_t)SS_GROUP * 256 * 4;
+  const size_t sm = SMALL_SELECT_SMEM;
   if (!attr) {
     GGMS_CU(cudaFuncSetAttribute(small_select<InT, SS_NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)sm));
@@ -414,6 +384,102 @@ static int sort_cluster_ctas(uint32_t S) {
   return S >= cs_min_s(8) ? 8 : 0;
 }
 
+// The one-launch path (ggms_direct.cuh) takes calls that leave everything to
+// the library: AUTO with no tuning field set, no statistics and no profiling
+// (those describe the two-pass pipeline), on a vector of up to
+// DIRECT_MAX_BYTES.  The lines below, and where they lie (us per call, one
+// launch / pipeline, B200, device ks and answers, normal values):
+//   bytes: the second read has to come from L2 (126 MB).  2^24 fp32: 90 / 189
+//     for 5 random ks, 154 / 260 for 1000, 132 / 164 for 1000 in the top 1 %;
+//     2^24 fp64 (128 MB): 175 / 285, 231 / 396, 190 / 244; 2^26 fp32 (256 MB):
+//     229 / 335, 401 / 472, but 295 / 238 and 1895 / 1230 for 2^14 random ks.
+//   ks: every k costs each CTA a search up to DIRECT_SLICE_KS; beyond, each CTA
+//     searches its own (one more barrier): 2^14 ks took 50 us of searching
+//     without it, 10 with it.  DIRECT_MAX_KS is the largest count measured.
+//   buckets: one per 8 keys keeps the children of a short vector short (2^16
+//     fp32, 1000 ks: 38 us, 45 with one per 32); 16384 instead of 8192 halve
+//     the copied keys of a long one (2^24, 1000 ks) and cost a short one 2 us.
+//   focus (most buckets to clustered ks): costs 3 us of the map, saves 25 of
+//     the copy and sort at 2^22 and 100 at 2^24 with 1000 ks in the top 1 %.
+constexpr uint64_t DIRECT_MAX_BYTES = 128ull << 20;
+constexpr uint32_t DIRECT_MAX_KS = 65536;
+constexpr uint64_t DIRECT_CTA_KEYS = 1024;    // keys that repay another CTA
+constexpr uint64_t DIRECT_BUCKET_KEYS = 8;
+constexpr uint64_t DIRECT_WIDE_N = 1u << 23;  // vectors that get all DIRECT_MAX_B buckets
+constexpr uint64_t DIRECT_FOCUS_N = 1u << 18;
+constexpr uint32_t DIRECT_FOCUS_KS = 16;
+constexpr uint32_t DIRECT_SLICE_KS = 2048;
+
+static bool direct_ok(const Context* ctx, const ggms_opts& o, uint64_t n, uint64_t nk, size_t elem) {
+  return n * elem <= DIRECT_MAX_BYTES && nk <= DIRECT_MAX_KS && !ctx->profile && !o.stats && !o.autotune &&
+         o.assigner == GGMS_ASSIGNER_AUTO && !o.num_buckets && !o.sample_size && o.train_steps <= 0 &&
+         !o.pass_threads && !o.pass_unroll && o.window_z == 0.0f && !o.pl_knots;
+}
+
+template <typename T>
+static int run_direct(Context* ctx, const T* d_in, uint64_t n, const uint32_t* ks, uint32_t nk, T* out,
+                      const ggms_opts& o, cudaStream_t st, bool topk) {
+  using K = typename KeyOf<T>::K;
+  ggms_opts od = o;
+  od.num_buckets = (int32_t)std::min<uint64_t>(n < DIRECT_WIDE_N ? DIRECT_MAX_B / 2 : DIRECT_MAX_B,
+                                                  std::max<uint64_t>(1024, pow2_floor(n / DIRECT_BUCKET_KEYS)));
+  od.sample_size = 1024;  // this path's sample stays in shared memory
+  Plan p;
+  int rc = make_plan(&p, n, nk, od);
+  if (rc) return rc;
+  GGMS_CU(cudaSetDevice(ctx->device));
+  rc = ensure_arena(ctx, layout<K>(p, nullptr).bytes);
+  if (rc) return rc;
+  const Workspace<K> w = layout<K>(p, ctx->arena);
+  const bool host_k = !o.ks_on_device && !topk, host_out = !o.out_on_device;
+  const size_t k_bytes = host_k ? ((4ull * nk + 63) & ~(size_t)63) : 0;
+  rc = ensure_pinned(ctx, sizeof(Counters) + 64 + k_bytes + (host_out ? sizeof(T) * nk : 0) + 64);
+  if (rc) return rc;
+  Counters* pin_C = (Counters*)ctx->pinned;
+  uint8_t* pin_k = ctx->pinned + ((sizeof(Counters) + 63) & ~(size_t)63);
+  T* pin_out = (T*)(pin_k + k_bytes);
+  if (host_k) {
+    if (ctx->pin_busy) GGMS_CU(cudaEventSynchronize(ctx->pin_busy));
+    memcpy(pin_k, ks, 4ull * nk);
+  }
+  const Caps caps{p.cap_seg, p.cap_tiles, p.nk, (uint32_t)(SMALL_SMEM / sizeof(K)), 0u, p.cap_rows};
+  const unsigned ctas = (unsigned)std::min<uint64_t>((n + DIRECT_CTA_KEYS - 1) / DIRECT_CTA_KEYS, 1u << 16);
+  auto enqueue = [&](cudaStream_t s) -> int {
+    DirectArgs<T> a;
+    a.in = d_in;
+    a.n = n;
+    a.ks = topk ? nullptr : (host_k ? (const uint32_t*)pin_k : ks);
+    a.seed = p.seed;
+    a.B = p.B;
+    a.slices = nk > DIRECT_SLICE_KS ? 1u : 0u;
+    a.focus = n >= DIRECT_FOCUS_N && nk >= DIRECT_FOCUS_KS && !a.slices ? 1u : 0u;
+    a.gact = w.aflag0;
+    a.ghist = w.hist0;
+    a.gcur = w.cmap0;
+    a.r = refine_args<T>(w, ctx, nk, caps, host_out ? pin_out : out, host_out ? pin_C : nullptr);
+    return launch_direct<T>(ctx, a, ctas, s);
+  };
+  const uint64_t key[] = {0xD17ull + sizeof(T) + (topk ? 256u : 0u) + (std::is_signed<T>::value ? 16u : 0u) +
+                              (std::is_floating_point<T>::value ? 32u : 0u),
+                          (uint64_t)(uintptr_t)d_in, n, host_k ? 1ull : (uint64_t)(uintptr_t)ks, nk,
+                          host_out ? 1ull : (uint64_t)(uintptr_t)out, p.seed, (uint64_t)(uintptr_t)ctx->arena,
+                          (uint64_t)(uintptr_t)ctx->pinned};
+  rc = run_graphed(ctx, key, (int)(sizeof(key) / sizeof(key[0])), st, enqueue);
+  if (rc) return rc;
+  rc = mark_done(ctx, st);
+  if (rc) return rc;
+  if (!host_out) {  // nothing waits for this call: the next one must not overwrite its ks
+    if (host_k) {
+      if (!ctx->pin_busy) GGMS_CU(cudaEventCreateWithFlags(&ctx->pin_busy, cudaEventDisableTiming));
+      GGMS_CU(cudaEventRecord(ctx->pin_busy, st));
+    }
+    return GGMS_OK;
+  }
+  GGMS_CU(cudaStreamSynchronize(st));
+  memcpy(out, pin_out, sizeof(T) * nk);
+  return (int)pin_C->status;
+}
+
 template <typename T>
 static int run_single(Context* ctx, const T* d_in, uint64_t n, const uint32_t* ks, uint64_t nk64,
                       T* out, const ggms_opts& o_in, cudaStream_t st, bool topk = false) {
@@ -430,6 +496,7 @@ static int run_single(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
     for (uint32_t i = 0; i < nk; ++i)
       if (ks[i] < 1u || (uint64_t)ks[i] > n) return GGMS_E_INVALID_ARG;
   }
+  if (direct_ok(ctx, o, n, nk, sizeof(T))) return run_direct<T>(ctx, d_in, n, ks, nk, out, o, st, topk);
   Plan p;
   int rc = make_plan(&p, n, nk, o);
   if (rc) return rc;
@@ -440,10 +507,10 @@ static int run_single(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
   pass_stages<T>(ctx, pv, p.B, p.ring_st);
   rc = l0_ncta<T>(ctx, pv, p.B, p.ring_st, &p.ncta);
   if (rc) return rc;
-  Workspace<K> w0 = layout<K>(p, sizeof(T), nullptr);
+  Workspace<K> w0 = layout<K>(p, nullptr);
   rc = ensure_arena(ctx, w0.bytes);
   if (rc) return rc;
-  Workspace<K> w = layout<K>(p, sizeof(T), ctx->arena);
+  Workspace<K> w = layout<K>(p, ctx->arena);
   const bool host_k = !o.ks_on_device && !topk, host_out = !o.out_on_device;
   const size_t pin_bytes = (host_k ? 4ull * nk : 0) + (host_out ? sizeof(T) * nk : 0) + sizeof(Counters) + 64;
   rc = ensure_pinned(ctx, pin_bytes);
@@ -453,7 +520,7 @@ static int run_single(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
   uint8_t* pin_k = pin + ((sizeof(Counters) + 63) & ~(size_t)63);
   uint8_t* pin_out = pin_k + (host_k ? ((4ull * nk + 63) & ~(size_t)63) : 0);
 
-  const Caps caps{p.cap_seg, p.cap_tiles, p.nk, (uint32_t)(SMALL_SMEM / sizeof(K)), 0u};
+  const Caps caps{p.cap_seg, p.cap_tiles, p.nk, (uint32_t)(SMALL_SMEM / sizeof(K)), 0u, p.cap_rows};
   if (host_k && !topk) {
     // host side, every call: the previous call's upload from the same pinned
     // buffer may still be queued (calls with device-resident answers return
@@ -466,11 +533,7 @@ static int run_single(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
   auto enqueue = [&](cudaStream_t s) -> int {
     prof_rec(prof, 0, s);
     GGMS_CU(cudaMemsetAsync(w.C, 0, sizeof(Counters), s));
-    const uint32_t* d_k = ks;
-    if (host_k && !topk) {
-      GGMS_CU(cudaMemcpyAsync(w.kin, pin_k, 4ull * nk, cudaMemcpyHostToDevice, s));
-      d_k = w.kin;
-    }
+    const uint32_t* d_k = host_k ? (const uint32_t*)pin_k : ks;  // host ks: read once, from the pinned copy
     ++ctx->launches;
     if (topk)
       k_init_topk<<<cdiv(nk, 256), 256, 0, s>>>(nk, n, w.krank, w.kseg);
@@ -550,7 +613,7 @@ static int run_single(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
       ++ctx->launches;
       l0_scan<K><<<1, 1024, 4u * p.B, s>>>(w.hist0, p.B, w.C, w.win, w.aflagc);
       ++ctx->launches;
-      lvl_locate_rows<<<cdiv(nk, 256), 256, 0, s>>>(w.hist0, p.B, nk, w.krank, w.kseg, w.kbin,
+      lvl_locate_rows<<<cdiv(nk, 256), 256, 0, s>>>(w.hist0, p.B, nk, w.krank, w.kseg, nullptr, 0u, w.kbin,
                                                        w.aflag0, p.B / 32, w.C, w.kcnt0);
       // most buckets hold a k: copy groups of buckets instead (coarse mode)
       ++ctx->launches;
@@ -561,14 +624,9 @@ static int run_single(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
     GGMS_CU(launch_pdl(l0_children<K>, cdiv(p.B, 256), 256, 0, s, w.hist0, w.aflag0, p.B, w.grid, w.C, w.win,
                        w.cmap0, w.segs[1], w.cursor[1], w.tiles[1], w.points, w.khead[1], w.smalls, w.bigs[1], caps,
                        w.ic, w.aflagc, w.kcnt0, tiny_keys<K>(), w.tinies));
-    // the first refinement level runs only when a level-0 child needs it: the
-    // kernel that relabels the ks after l0_children sets that condition
-    cudaGraphConditionalHandle lev1 = 0;
-    rc = level_handle(s, &lev1);
-    if (rc) return rc;
     ++ctx->launches;
     GGMS_CU(launch_pdl(l0_relabel_bases<K>, ctx->sms * 4, 256, 0, s, w.cmap0, nk, w.kbin, w.kseg, w.kkey, w.points,
-                       w.C, w.segs[1], w.khead[1], w.knext, w.crow, p.B, p.ncta, caps, lev1));
+                       w.C, w.segs[1], w.khead[1], w.knext, w.crow, p.B, p.ncta, caps));
     // ---- PASS 2: compact the buckets that still need refinement
     prof_rec(prof, 3, s);
     ++ctx->launches;
@@ -588,51 +646,12 @@ static int run_single(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
     }
     if (rc) return rc;
 
-    // ---- refinement levels over candidates
-    const int maxlev = (sizeof(K) == 4) ? MAX_LEVELS_32 : MAX_LEVELS_64;
-    const int lv_grid = ctx->sms * 8;
-    const int seg_grid = std::min<int>((int)p.cap_seg, ctx->sms * 2);
-    rc = enqueue_levels(ctx, s, w.C, 1, maxlev, lev1, [&](cudaStream_t s, int l) -> int {
-      const int pp = l & 1, q = pp ^ 1;
-      const K* src = w.cand[(l - 1) & 1];
-      K* dst = w.cand[l & 1];
-      ++ctx->launches;
-      lvl_prep<<<ctx->sms * 2, 256, 0, s>>>(w.rows[pp], w.aflag[pp], w.bigs[pp], w.C, pp, caps);
-      ++ctx->launches;
-      lvl_count<K, LV_NT><<<lv_grid, LV_NT, 0, s>>>(src, w.segs[pp], w.tiles[pp], w.C, pp, w.rows[pp], caps,
-                                                     nullptr, nullptr);
-      ++ctx->launches;
-      lvl_scan<<<seg_grid, 1024, 0, s>>>(w.rows[pp], w.bigs[pp], w.C, pp, caps);
-      ++ctx->launches;
-      lvl_locate_rows<<<cdiv(nk, 256), 256, 0, s>>>(w.rows[pp], NBIN, nk, w.krank, w.kseg, w.kbin,
-                                                       w.aflag[pp], NBIN_WORDS, w.C);
-      ++ctx->launches;
-      lvl_children<K, 1024><<<seg_grid, 1024, 0, s>>>(w.rows[pp], w.aflag[pp], w.segs[pp], w.C, pp,
-                                                       w.segs[q], w.cursor[q], w.tiles[q], w.points,
-                                                       w.khead[q], w.smalls, w.tinies, w.bigs[pp],
-                                                       w.bigs[q], caps, nullptr);
-      ++ctx->launches;
-      lvl_relabel<K><<<cdiv(nk, 256), 256, 0, s>>>(w.rows[pp], NBIN, nk, w.kbin, w.kseg, w.kkey,
-                                                      w.points, w.C, w.segs[q], w.khead[q], w.knext);
-      if (l < maxlev) {
-        ++ctx->launches;
-        lvl_compact<K, LV_NT><<<lv_grid, LV_NT, 0, s>>>(src, w.segs[pp], w.tiles[pp], w.C, pp,
-                                                         w.rows[pp], w.segs[q], w.cursor[q], dst, caps,
-                                                         nullptr, nullptr);
-        return launch_small_select<K>(ctx, dst, w.segs[q], w.khead[q], w, caps, s);
-      }
-      return GGMS_OK;
-    });
-    if (rc) return rc;
-
-    // ---- answers
+    // ---- refinement levels over candidates, answers
     prof_rec(prof, 8, s);
-    T* d_out = host_out ? (T*)w.out_dev : out;
-    ++ctx->launches;
-    write_out<T><<<cdiv(nk, 256), 256, 0, s>>>(w.kkey, w.kseg, nk, d_out, w.C);
+    rc = launch_refine<T>(ctx, refine_args<T>(w, ctx, nk, caps, host_out ? (T*)pin_out : out,
+                                              host_out || o.stats ? pin_C : nullptr), s);
+    if (rc) return rc;
     if (cudaGetLastError() != cudaSuccess) return GGMS_E_CUDA;
-    if (host_out) GGMS_CU(cudaMemcpyAsync(pin_out, d_out, sizeof(T) * nk, cudaMemcpyDeviceToHost, s));
-    if (host_out || o.stats) GGMS_CU(cudaMemcpyAsync(pin_C, w.C, sizeof(Counters), cudaMemcpyDeviceToHost, s));
     prof_rec(prof, 5, s);
     return GGMS_OK;
   };
@@ -818,11 +837,12 @@ static int run_segmented(Context* ctx, const T* d_in, const int64_t* seg_off, in
   p.cap_seg = std::max<uint32_t>(nk, nseg) + 1;
   p.cap_tiles = (uint32_t)((n + TILE - 1) / TILE) + p.cap_seg;
   p.cap_q = (uint32_t)std::min<uint64_t>(nseg, n / QSAMP) + 1;
-  Workspace<K> w0 = layout<K>(p, sizeof(T), nullptr);
+  p.cap_rows = std::max(p.cap_q, (uint32_t)p.cap_rows);
+  Workspace<K> w0 = layout<K>(p, nullptr);
   rc = ensure_arena(ctx, w0.bytes);
   if (rc) return rc;
-  Workspace<K> w = layout<K>(p, sizeof(T), ctx->arena);
-  const Caps caps{p.cap_seg, p.cap_tiles, p.nk, small_keys, tiny_keys<K>()};
+  Workspace<K> w = layout<K>(p, ctx->arena);
+  const Caps caps{p.cap_seg, p.cap_tiles, p.nk, small_keys, tiny_keys<K>(), p.cap_rows};
   // the stream-ordered part: captured once and replayed when the call repeats
   auto enqueue = [&](cudaStream_t s) -> int {
     GGMS_CU(cudaMemsetAsync(w.C, 0, sizeof(Counters), s));
@@ -841,59 +861,34 @@ static int run_segmented(Context* ctx, const T* d_in, const int64_t* seg_off, in
     seg_sample<T><<<ctx->sms * 2, 1024, 0, s>>>(d_in, w.segs[0], w.bigs[0], w.C, p.cap_q, w.qtab, w.qdir,
                                                  p.seed ^ 0x5E6A11ull);
     // level 0 over the input with quantile bins; then radix levels over candidates
-    // (a child range of up to 2^bits keys needs ceil(bits / 11) more levels)
-    const int maxlev = 1 + (KeyBits<K>::value + RADIX_BITS - 1) / RADIX_BITS;
     const int lv_grid = ctx->sms * lv_mult;
     const int seg_grid = ctx->sms * 2;
-    for (int l = 0; l < maxlev; ++l) {
-      const int pp = l & 1, q = pp ^ 1;
-      K* dst = w.cand[l & 1];
-      const K* src = w.cand[(l + 1) & 1];  // the previous level's candidates (l >= 1)
-      ++ctx->launches;
-      lvl_prep<<<ctx->sms * 2, 256, 0, s>>>(w.rows[pp], w.aflag[pp], w.bigs[pp], w.C, pp, caps);
-      ++ctx->launches;
-      if (l == 0)
-        lvl_count<T, LV_NT, true><<<lv_grid, LV_NT, 0, s>>>(d_in, w.segs[pp], w.tiles[pp], w.C, pp, w.rows[pp],
-                                                             caps, w.qtab, w.qdir);
-      else
-        lvl_count<K, LV_NT><<<lv_grid, LV_NT, 0, s>>>(src, w.segs[pp], w.tiles[pp], w.C, pp, w.rows[pp], caps,
-                                                       nullptr, nullptr);
-      ++ctx->launches;
-      lvl_scan<<<seg_grid, 1024, 0, s>>>(w.rows[pp], w.bigs[pp], w.C, pp, caps);
-      ++ctx->launches;
-      lvl_locate_rows<<<cdiv(nk, 256), 256, 0, s>>>(w.rows[pp], NBIN, nk, w.krank, w.kseg, w.kbin,
-                                                       w.aflag[pp], NBIN_WORDS, w.C);
-      ++ctx->launches;
-      if (l == 0)
-        lvl_children<K, 1024, true><<<seg_grid, 1024, 0, s>>>(w.rows[pp], w.aflag[pp], w.segs[pp], w.C, pp,
-                                                               w.segs[q], w.cursor[q], w.tiles[q], w.points,
-                                                               w.khead[q], w.smalls, w.tinies, w.bigs[pp],
-                                                               w.bigs[q], caps, w.qtab);
-      else
-        lvl_children<K, 1024><<<seg_grid, 1024, 0, s>>>(w.rows[pp], w.aflag[pp], w.segs[pp], w.C, pp,
-                                                         w.segs[q], w.cursor[q], w.tiles[q], w.points,
-                                                         w.khead[q], w.smalls, w.tinies, w.bigs[pp],
-                                                         w.bigs[q], caps, nullptr);
-      ++ctx->launches;
-      lvl_relabel<K><<<cdiv(nk, 256), 256, 0, s>>>(w.rows[pp], NBIN, nk, w.kbin, w.kseg, w.kkey,
-                                                      w.points, w.C, w.segs[q], w.khead[q], w.knext);
-      if (l + 1 < maxlev) {
-        ++ctx->launches;
-        if (l == 0)
-          lvl_compact<T, LV_NT, true><<<lv_grid, LV_NT, 0, s>>>(d_in, w.segs[pp], w.tiles[pp], w.C, pp,
-                                                                 w.rows[pp], w.segs[q], w.cursor[q], dst, caps,
-                                                                 w.qtab, w.qdir);
-        else
-          lvl_compact<K, LV_NT><<<lv_grid, LV_NT, 0, s>>>(src, w.segs[pp], w.tiles[pp], w.C, pp,
-                                                           w.rows[pp], w.segs[q], w.cursor[q], dst, caps,
-                                                           nullptr, nullptr);
-        rc = launch_small_select<K>(ctx, dst, w.segs[q], w.khead[q], w, caps, s);
-        if (rc) return rc;
-      }
-    }
     ++ctx->launches;
-    write_out<T><<<cdiv(nk, 256), 256, 0, s>>>(w.kkey, w.kseg, nk, out, w.C);
-  return cudaGetLastError() == cudaSuccess ? GGMS_OK : GGMS_E_CUDA;
+    lvl_prep<<<ctx->sms * 2, 256, 0, s>>>(w.rows[0], w.aflag[0], w.C, 0, caps);
+    ++ctx->launches;
+    lvl_count<T, LV_NT, true><<<lv_grid, LV_NT, 0, s>>>(d_in, w.segs[0], w.tiles[0], w.C, 0, w.rows[0], caps, w.qtab,
+                                                         w.qdir);
+    ++ctx->launches;
+    lvl_scan<<<seg_grid, 1024, 0, s>>>(w.rows[0], w.C, 0, caps);
+    ++ctx->launches;
+    lvl_locate_rows<<<cdiv(nk, 256), 256, 0, s>>>(w.rows[0], NBIN, nk, w.krank, w.kseg, &w.segs[0]->row,
+                                                     (uint32_t)(sizeof(Seg<K>) / 4), w.kbin, w.aflag[0], NBIN_WORDS,
+                                                     w.C);
+    ++ctx->launches;
+    lvl_children<K, 1024, true><<<seg_grid, 1024, 0, s>>>(w.rows[0], w.aflag[0], w.segs[0], w.C, 0, w.segs[1],
+                                                           w.cursor[1], w.tiles[1], w.points, w.khead[1], w.smalls,
+                                                           w.tinies, w.bigs[0], w.bigs[1], caps, w.qtab);
+    ++ctx->launches;
+    lvl_relabel<K><<<cdiv(nk, 256), 256, 0, s>>>(w.rows[0], NBIN, nk, w.segs[0], w.kbin, w.kseg, w.kkey, w.points, w.C,
+                                                    w.segs[1], w.khead[1], w.knext);
+    ++ctx->launches;
+    lvl_compact<T, LV_NT, true><<<lv_grid, LV_NT, 0, s>>>(d_in, w.segs[0], w.tiles[0], w.C, 0, w.rows[0], w.segs[1],
+                                                           w.cursor[1], w.cand[0], caps, w.qtab, w.qdir);
+    rc = launch_small_select<K>(ctx, w.cand[0], w.segs[1], w.khead[1], w, caps, s);
+    if (rc) return rc;
+    rc = launch_refine<T>(ctx, refine_args<T>(w, ctx, nk, caps, out, nullptr), s);
+    if (rc) return rc;
+    return cudaGetLastError() == cudaSuccess ? GGMS_OK : GGMS_E_CUDA;
   };
   if (o.stats || ctx->profile) {
     rc = enqueue(st);

@@ -5,6 +5,7 @@
 // live in ggms_engine.cuh, compiled once per value type (ggms_f32.cu, ...).
 #pragma once
 #include <algorithm>
+#include <atomic>
 #include <cstddef>
 #include <cstdio>
 #include <cstdlib>
@@ -18,6 +19,8 @@
 #include "../../include/ggms.h"
 
 namespace ggms {
+
+constexpr int MAX_DEVICES = 64;
 
 // ------------------------------------------------------------------ context
 struct Context {
@@ -54,8 +57,6 @@ struct Context {
   uint64_t clock = 0;
   cudaStream_t capture = nullptr;  // private stream the graphs are captured on
   cudaEvent_t pin_busy = nullptr;  // recorded after the last call's uploads from the pinned buffer
-  static constexpr int MAX_NEST = 8;
-  cudaStream_t bodies[MAX_NEST] = {};  // private streams the nested level bodies are captured on
   cudaStream_t side = nullptr;     // the sampled assigner's build next to the learned one; the warp finisher
   cudaEvent_t fork = nullptr, join = nullptr, fork2 = nullptr, join2 = nullptr;
   // autotuner: launch shapes and bucket counts picked per shape class
@@ -78,6 +79,10 @@ static int cuda_status(cudaError_t e) {
     if (e_ != cudaSuccess) return cuda_status(e_);  \
   } while (0)
 
+// Every layout of the arena begins with the call's counters and, at
+// ARENA_BAR, the word the grid barriers count on.
+constexpr size_t ARENA_BAR = 256;
+
 static int ensure_arena(Context* c, size_t bytes) {
   if (c->arena_bytes >= bytes) return GGMS_OK;
   if (c->arena) {
@@ -89,6 +94,11 @@ static int ensure_arena(Context* c, size_t bytes) {
   size_t want = bytes + bytes / 8;
   GGMS_CU(cudaMalloc(&c->arena, want));
   c->arena_bytes = want;
+  // the grid barriers' word is zeroed here once (it needs no reset between
+  // launches), on the context's own stream: the caller's may be capturing
+  if (!c->query) GGMS_CU(cudaStreamCreateWithFlags(&c->query, cudaStreamNonBlocking));
+  GGMS_CU(cudaMemsetAsync(c->arena + ARENA_BAR, 0, 256, c->query));
+  GGMS_CU(cudaStreamSynchronize(c->query));
   return GGMS_OK;
 }
 
@@ -112,9 +122,9 @@ static int create_context(Context** out, int device) {
   c->device = device;
   cudaError_t e = cudaSetDevice(device);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
-  if (e != cudaSuccess) {
+  if (e != cudaSuccess || device >= MAX_DEVICES) {
     delete c;
-    return cuda_status(e);
+    return e != cudaSuccess ? cuda_status(e) : GGMS_E_UNSUPPORTED;
   }
   *out = c;
   return GGMS_OK;
@@ -137,8 +147,6 @@ static void destroy_context(Context* c) {
     if (g.exec) cudaGraphExecDestroy(g.exec);
   if (c->capture) cudaStreamDestroy(c->capture);
   if (c->pin_busy) cudaEventDestroy(c->pin_busy);
-  for (auto& b : c->bodies)
-    if (b) cudaStreamDestroy(b);
   if (c->side) cudaStreamDestroy(c->side);
   for (cudaEvent_t e : {c->fork, c->join, c->fork2, c->join2})
     if (e) cudaEventDestroy(e);
@@ -165,6 +173,24 @@ static cudaError_t launch_pdl(void (*k)(P...), unsigned grid, unsigned block, si
   return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
 }
 
+// Launch whose CTAs meet at grid barriers: all of them are resident at once, or
+// the launch waits until they can be (or fails when they never can).
+template <typename... P, typename... A>
+static cudaError_t launch_coop(void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                               A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
+}
+
 // The side stream and its fork / join events (created on first use).
 static int ensure_side(Context* c) {
   if (!c->side) GGMS_CU(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
@@ -175,12 +201,12 @@ static int ensure_side(Context* c) {
 
 // default contexts of the drop-in entry points, one per device
 inline std::mutex g_default_mu;
-inline Context* g_default[64];
+inline Context* g_default[MAX_DEVICES];
 
 inline int default_context(Context** out) {
   int dev = 0;
   GGMS_CU(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64) return GGMS_E_UNSUPPORTED;
+  if (dev < 0 || dev >= MAX_DEVICES) return GGMS_E_UNSUPPORTED;
   std::lock_guard<std::mutex> lk(g_default_mu);
   if (!g_default[dev]) {
     int rc = create_context(&g_default[dev], dev);
@@ -208,6 +234,7 @@ struct Plan {
   uint32_t S;        // sample size
   uint32_t cap_seg;
   uint32_t cap_tiles;
+  uint32_t cap_rows; // segments a refinement level can hold
   uint32_t ncta;     // CTAs of the two passes (identical grids)
   int assigner;
   int train_steps;
@@ -247,6 +274,9 @@ static int make_plan(Plan* p, uint64_t n, uint32_t nk, const ggms_opts& o) {
   p->ncta = 0;
   p->cap_seg = nk + 1;
   p->cap_tiles = (uint32_t)((n + TILE - 1) / TILE) + p->cap_seg;
+  // a level refines segments of more than 4096 keys (the one-launch path's
+  // 64-bit ones; the other segments that come to a level have more)
+  p->cap_rows = (uint32_t)std::min<uint64_t>(p->cap_seg, n / 4096 + 1);
   p->train_steps = o.train_steps > 0 ? o.train_steps : 0;
   p->bound = o.imbalance_bound > 0.0f ? o.imbalance_bound : 3.0f;
   p->window_z = o.window_z == 0.0f ? 6.0f : o.window_z;

@@ -388,9 +388,11 @@ struct Seg {
   uint32_t shift;
   K lo;
   K hi;
-  uint32_t small; // finished by small_select (in shared memory), not by another level
+  uint32_t row;   // its histogram row (position in the level's list), or SEG_SMALL
   uint32_t pad;
 };
+
+constexpr uint32_t SEG_SMALL = 0xFFFFFFFFu;    // Seg::row: finished in shared memory, not by another level
 
 constexpr uint32_t K_NIL = 0xFFFFFFFFu;        // end of a per-segment k list
 constexpr size_t SMALL_SMEM = 64 * 1024;         // keys of one small segment in shared memory (a power of two)
@@ -416,11 +418,11 @@ struct Counters {
   unsigned long long refine_elems;
   uint32_t asg_choice;        // index of the assigner in use (0 sampled, 1 learned)
   uint32_t win_runs;          // PASS 1 window runs in use (0: no windows)
-  uint32_t done;              // a refinement level found no segment: later levels are skipped
   uint32_t ntiny;             // tiny segments created by the current level (batched path)
   uint32_t nbig[2];           // segments of pool p that a level refines (listed in bigs[p])
   uint32_t coarse;            // level 0 copies NGRP groups of buckets (most buckets hold a k)
   uint32_t passes;            // launches that read the whole input (counted by the kernels themselves)
+  uint32_t ticket;            // CTAs of the call's last kernel that are done (the last one reports)
 };
 
 // PASS 1 windows (l0_window).  From the sample, every requested k gets a
@@ -469,6 +471,7 @@ struct Caps {
   uint32_t points;
   uint32_t small_keys;        // a child with at most this many keys is finished by small_select
   uint32_t tiny_keys;         // ... and with at most this many by tiny_select (one warp); 0: never
+  uint32_t rows;              // segments a level can refine at once (its histogram rows)
 };
 
 // Level 0 of the batched path: a caller segment too large for small_select

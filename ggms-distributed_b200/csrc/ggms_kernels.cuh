@@ -1193,16 +1193,16 @@ __device__ __forceinline__ uint32_t locate_one(const uint32_t* I, uint32_t row_l
   return lo;
 }
 
-// With kcnt (level 0 of one vector), the ks of each bucket are also counted.
-__global__ void lvl_locate_rows(const uint32_t* __restrict__ rows, uint32_t row_len, uint32_t nk,
-                                uint32_t* k_rank, const uint32_t* __restrict__ k_seg,
-                                uint32_t* k_bin, uint32_t* aflag, uint32_t flag_words,
-                                Counters* C, uint32_t* kcnt = nullptr) {
-  pdl_entry();
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nk) return;
-  const uint32_t s = k_seg[i];
+// The row of segment s is s itself, or row_of[s * row_stride] (Seg::row of the
+// level's segments, a strided array of words).  With kcnt (level 0 of one
+// vector), the ks of each bucket are also counted.
+__device__ __forceinline__ void locate_in_row(uint32_t i, const uint32_t* rows, uint32_t row_len, uint32_t* k_rank,
+                                              const uint32_t* k_seg, const uint32_t* row_of, uint32_t row_stride,
+                                              uint32_t* k_bin, uint32_t* aflag, uint32_t flag_words, Counters* C,
+                                              uint32_t* kcnt) {
+  uint32_t s = k_seg[i];
   if (s == K_DONE) return;
+  if (row_of) s = row_of[(size_t)s * row_stride];
   uint32_t r = k_rank[i];
   const uint32_t lo = locate_one(rows + (size_t)s * row_len, row_len, r, C);
   if (lo == K_NIL) return;
@@ -1210,6 +1210,17 @@ __global__ void lvl_locate_rows(const uint32_t* __restrict__ rows, uint32_t row_
   k_rank[i] = r;
   atomicOr(&aflag[(size_t)s * flag_words + (lo >> 5)], 1u << (lo & 31));
   if (kcnt) atomicAdd(&kcnt[lo], 1u);
+}
+
+__global__ void lvl_locate_rows(const uint32_t* __restrict__ rows, uint32_t row_len, uint32_t nk,
+                                uint32_t* k_rank, const uint32_t* __restrict__ k_seg,
+                                const uint32_t* __restrict__ row_of, uint32_t row_stride,
+                                uint32_t* k_bin, uint32_t* aflag, uint32_t flag_words,
+                                Counters* C, uint32_t* kcnt = nullptr) {
+  pdl_entry();
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < nk)
+    locate_in_row(i, rows, row_len, k_rank, k_seg, row_of, row_stride, k_bin, aflag, flag_words, C, kcnt);
 }
 
 // Active level-0 buckets -> refinement segments (or points).  In the coarse
@@ -1322,7 +1333,7 @@ __global__ __launch_bounds__(1024) void l0_children(const uint32_t* __restrict__
   sg.lo = lo;
   sg.hi = hi;
   sg.shift = (uint32_t)max(0, bitlen((K)(hi - lo)) - RADIX_BITS);
-  sg.small = kind != C_BIG ? 1u : 0u;
+  sg.row = kind != C_BIG ? SEG_SMALL : cbase[N_BIG] + li;
   sg.pad = b;  // the level-0 bucket or group (l0_bases needs it)
   segs1[id] = sg;
   cursor1[id] = 0u;
@@ -1333,8 +1344,8 @@ __global__ __launch_bounds__(1024) void l0_children(const uint32_t* __restrict__
     if (si < caps.segs) (kind == C_TINY ? tinies : smalls)[si] = id; else set_status(C, GGMS_E_INTERNAL);
     return;
   }
-  const uint32_t bi = cbase[N_BIG] + li;
-  if (bi < caps.segs) bigs1[bi] = id; else set_status(C, GGMS_E_INTERNAL);
+  if (sg.row >= caps.rows) { set_status(C, GGMS_E_INTERNAL); return; }
+  bigs1[sg.row] = id;
   const uint32_t t0 = cbase[N_TILE] + lt;
   if (t0 + nt > caps.tiles || t0 + nt < t0) { set_status(C, GGMS_E_INTERNAL); return; }
   for (uint32_t t = 0; t < nt; ++t) tiles1[t0 + t] = TileRef{id, t};
@@ -1343,9 +1354,8 @@ __global__ __launch_bounds__(1024) void l0_children(const uint32_t* __restrict__
 // ks follow their bin: resolved (single key) or the id of the next segment.
 template <typename K>
 __device__ __forceinline__ void relabel_one(uint32_t i, uint32_t e, uint32_t* k_seg, K* k_key,
-                                            const K* __restrict__ points, Counters* C,
-                                            const Seg<K>* __restrict__ segs_q, uint32_t* khead_q,
-                                            uint32_t* knext) {
+                                            const K* points, Counters* C, const Seg<K>* segs_q,
+                                            uint32_t* khead_q, uint32_t* knext) {
   if (e == CM_NONE) {
     set_status(C, GGMS_E_INTERNAL);
     k_seg[i] = K_DONE;
@@ -1356,21 +1366,21 @@ __device__ __forceinline__ void relabel_one(uint32_t i, uint32_t e, uint32_t* k_
     k_seg[i] = K_DONE;
   } else {
     k_seg[i] = e;
-    if (segs_q[e].small) knext[i] = atomicExch(&khead_q[e], i);  // lock-free push
+    if (segs_q[e].row == SEG_SMALL) knext[i] = atomicExch(&khead_q[e], i);  // lock-free push
   }
 }
 
 template <typename K>
 __global__ void lvl_relabel(const uint32_t* __restrict__ cmap, uint32_t row_len, uint32_t nk,
-                            const uint32_t* __restrict__ k_bin, uint32_t* k_seg, K* k_key,
-                            const K* __restrict__ points, Counters* C,
+                            const Seg<K>* __restrict__ segs, const uint32_t* __restrict__ k_bin,
+                            uint32_t* k_seg, K* k_key, const K* __restrict__ points, Counters* C,
                             const Seg<K>* __restrict__ segs_q, uint32_t* khead_q, uint32_t* knext) {
   pdl_entry();
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nk) return;
   const uint32_t s = k_seg[i];
   if (s == K_DONE) return;
-  relabel_one<K>(i, cmap[(size_t)s * row_len + k_bin[i]], k_seg, k_key, points, C, segs_q, khead_q, knext);
+  relabel_one<K>(i, cmap[(size_t)segs[s].row * row_len + k_bin[i]], k_seg, k_key, points, C, segs_q, khead_q, knext);
 }
 
 // The first steps between PASS 1 and PASS 2 of one vector in ONE CTA (1024
@@ -1535,17 +1545,14 @@ __global__ void l0_bases(uint32_t* crow, uint32_t B, uint32_t ncta, const Seg<K>
 // After l0_children: the ks follow their level-0 child (lvl_relabel) and the
 // per-CTA write cursors of PASS 2 are formed (l0_bases), in one launch --
 // threads [0, nk) relabel, all warps then take children for the cursors.
-// In a captured graph it also sets the condition of the first refinement
-// level (lev1, nonzero): whether some level-0 child needs one.
 template <typename K>
 __global__ void l0_relabel_bases(const uint32_t* __restrict__ cmap0, uint32_t nk,
                                  const uint32_t* __restrict__ k_bin, uint32_t* k_seg, K* k_key,
                                  const K* __restrict__ points, Counters* C, const Seg<K>* __restrict__ segs1,
                                  uint32_t* khead1, uint32_t* knext, uint32_t* crow, uint32_t B, uint32_t ncta,
-                                 Caps caps, cudaGraphConditionalHandle lev1) {
+                                 Caps caps) {
   pdl_entry();
   GGMS_TRACE(60);
-  if (lev1 && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(lev1, C->nbig[1] ? 1u : 0u);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nk; i += gridDim.x * blockDim.x) {
     const uint32_t s = k_seg[i];
     if (s == K_DONE) continue;
@@ -2081,29 +2088,22 @@ __global__ __launch_bounds__(NT, PASS_MIN_CTAS(NT)) void l0_compact_coarse(const
 // ------------------------------------------------------------------ refinement levels
 // Level l works on the segments of pool p = l & 1 and creates children in pool
 // q = p ^ 1.  Keys are read from `src` and children are written to `dst`.
-
-// Gate of a refinement level inside a captured CUDA graph: the level (an IF
-// node) runs only while every level so far had segments to refine.
-__global__ void lvl_gate(Counters* C, int p, cudaGraphConditionalHandle h) {
-  pdl_entry();
-  GGMS_TRACE(41 + p);
-  if (C->nbig[p] == 0u) C->done = 1u;
-  cudaGraphSetConditional(h, C->done ? 0u : 1u);
-}
+// The steps are device functions over (cta, ncta), so that the batched level 0
+// can launch them as kernels and refine_levels runs them all in one launch.
+// In that launch one step reads what another CTA wrote in an earlier one, so
+// their pointers to scratch are not __restrict__ (no non-coherent loads).
 
 // zero this level's histogram rows / flags (segments that small_select or
 // tiny_select finished have none); reset the child pool's counters
-__global__ void lvl_prep(uint32_t* rows, uint32_t* aflag, const uint32_t* __restrict__ bigs, Counters* C,
-                         int p, Caps caps) {
-  pdl_entry();
-  const uint32_t nb = min(C->nbig[p], caps.segs);
-  for (uint32_t j = blockIdx.x; j < nb; j += gridDim.x) {
-    const uint32_t sid = bigs[j];
-    uint32_t* row = rows + (size_t)sid * NBIN;
+__device__ __forceinline__ void prep_body(uint32_t* rows, uint32_t* aflag, Counters* C, int p, const Caps& caps,
+                                          uint32_t cta, uint32_t ncta) {
+  const uint32_t nb = min(C->nbig[p], caps.rows);
+  for (uint32_t j = cta; j < nb; j += ncta) {
+    uint32_t* row = rows + (size_t)j * NBIN;
     for (uint32_t i = threadIdx.x; i < NBIN; i += blockDim.x) row[i] = 0u;
-    for (uint32_t i = threadIdx.x; i < NBIN_WORDS; i += blockDim.x) aflag[(size_t)sid * NBIN_WORDS + i] = 0u;
+    for (uint32_t i = threadIdx.x; i < NBIN_WORDS; i += blockDim.x) aflag[(size_t)j * NBIN_WORDS + i] = 0u;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  if (cta == 0 && threadIdx.x == 0) {
     C->nsegs[p ^ 1] = 0u;
     C->ntiles[p ^ 1] = 0u;
     C->nbig[p ^ 1] = 0u;
@@ -2111,6 +2111,11 @@ __global__ void lvl_prep(uint32_t* rows, uint32_t* aflag, const uint32_t* __rest
     C->ntiny = 0u;
     if (nb) C->levels_run += 1u;
   }
+}
+
+__global__ void lvl_prep(uint32_t* rows, uint32_t* aflag, Counters* C, int p, Caps caps) {
+  pdl_entry();
+  prep_body(rows, aflag, C, p, caps, blockIdx.x, gridDim.x);
 }
 
 // Bin of a key in a quantile segment: the number of boundaries <= key.  The
@@ -2208,35 +2213,64 @@ __global__ __launch_bounds__(1024) void seg_sample(const T* __restrict__ in, Seg
   }
 }
 
+// Elements [beg, end) of a candidate buffer, 16 bytes at a time: every thread
+// calls f(keys, mask) for its vectors, U of them in flight; bit t of mask says
+// that keys[t] is one of the elements (the first and last vector may reach
+// past them, into the same allocation).  All threads make the same number of
+// calls (those past the end with mask 0).
+template <typename K, int NT, typename F>
+__device__ __forceinline__ void tile_stream(const K* src, uint64_t beg, uint64_t end, F&& f) {
+  constexpr int N = 16 / (int)sizeof(K), U = 4;
+  const uint64_t v0 = beg / N, v1 = (end + N - 1) / N;
+  const uint4* vp = reinterpret_cast<const uint4*>(src);
+  for (uint64_t r = v0; r < v1; r += NT * U) {
+    uint4 q[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint64_t v = r + threadIdx.x + (uint64_t)u * NT;
+      if (v < v1) q[u] = vp[v];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint64_t v = r + threadIdx.x + (uint64_t)u * NT;
+      if (r + (uint64_t)u * NT >= v1) break;  // the same for every thread
+      uint32_t mask = v < v1 ? (1u << N) - 1u : 0u;
+      if (mask && v * N < beg) mask &= ~0u << (uint32_t)(beg - v * N);
+      if (mask && v * N + N > end) mask &= (1u << (uint32_t)(end - v * N)) - 1u;
+      K k[N];
+      unpack16<K>(q[u], k);
+      f(k, mask);
+    }
+  }
+}
+
 // Histogram of radix bins, one tile of one segment per iteration.
 // Q: the level's segments have quantile bins (batched level 0), else radix
 // bins (key - lo) >> shift.
+// h: NBIN words of shared memory.
 template <typename InT, int NT, bool Q = false>
-__global__ __launch_bounds__(NT) void lvl_count(const InT* __restrict__ src,
-                                               const Seg<typename KeyOf<InT>::K>* __restrict__ segs,
-                                               const TileRef* __restrict__ tiles,
-                                               Counters* C, int p, uint32_t* rows, Caps caps,
-                                               const typename KeyOf<InT>::K* __restrict__ qtab,
-                                               const uint16_t* __restrict__ qdir) {
-  pdl_entry();
+__device__ __forceinline__ void count_body(const InT* src, const Seg<typename KeyOf<InT>::K>* segs,
+                                           const TileRef* tiles, Counters* C, int p, uint32_t* rows,
+                                           const Caps& caps, const typename KeyOf<InT>::K* qtab,
+                                           const uint16_t* qdir, uint32_t* h, uint32_t cta, uint32_t ncta) {
   using K = typename KeyOf<InT>::K;
-  __shared__ uint32_t h[NBIN];
   __shared__ __align__(16) K qb[Q ? QB : 1];
   __shared__ __align__(16) uint16_t qd[Q ? QDS : 8];
   const uint32_t nt = min(C->ntiles[p], caps.tiles);
   const uint32_t ns = min(C->nsegs[p], caps.segs);
-  if (Q && nt && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&C->passes, 1u);  // level 0 reads the input
+  if (Q && nt && cta == 0 && threadIdx.x == 0) atomicAdd(&C->passes, 1u);  // level 0 reads the input
   // Each CTA takes a contiguous range of the tile list, where a segment's tiles
   // are consecutive: the histogram of one segment's run of tiles stays in
   // shared memory and is added to the segment's row once per run, not once
   // per tile (a row holds NBIN bins for TILE keys), and the quantile table is
   // loaded once per run.
-  const uint32_t per = (nt + gridDim.x - 1) / gridDim.x;
-  const uint32_t t_beg = min(blockIdx.x * per, nt), t_end = min(t_beg + per, nt);
+  const uint32_t per = (nt + ncta - 1) / ncta;
+  const uint32_t t_beg = min(cta * per, nt), t_end = min(t_beg + per, nt);
   uint32_t open = 0xFFFFFFFFu;  // segment whose counts the shared histogram holds
+  uint32_t open_row = 0;
   unsigned long long open_keys = 0;
   auto flush = [&]() {  // all threads, after a barrier
-    uint32_t* row = rows + (size_t)open * NBIN;
+    uint32_t* row = rows + (size_t)open_row * NBIN;
     for (uint32_t i = threadIdx.x; i < NBIN; i += NT) {
       const uint32_t v = h[i];
       if (v) atomicAdd(&row[i], v);
@@ -2255,27 +2289,34 @@ __global__ __launch_bounds__(NT) void lvl_count(const InT* __restrict__ src,
       if (Q) qtab_to_smem<K>(qtab, qdir, s.pad, qb, qd);
       for (uint32_t i = threadIdx.x; i < NBIN; i += NT) h[i] = 0u;
       open = tr.seg;
+      open_row = s.row;
       open_keys = 0;
       __syncthreads();
     }
     const uint64_t beg = s.off + (uint64_t)tr.no * TILE;
     const uint64_t end = min(beg + TILE, s.off + s.cnt);
-    constexpr int U = 8;  // independent loads in flight per thread
-    for (uint64_t o = beg + threadIdx.x; o < end; o += (uint64_t)NT * U) {
-      K kk[U];
+    if constexpr (Q) {
+      constexpr int U = 8;  // independent loads in flight per thread
+      for (uint64_t o = beg + threadIdx.x; o < end; o += (uint64_t)NT * U) {
+        K kk[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const uint64_t i = o + (uint64_t)u * NT;
-        kk[u] = i < end ? KeyOf<InT>::to(src[i]) : (K)0;
-      }
+        for (int u = 0; u < U; ++u) {
+          const uint64_t i = o + (uint64_t)u * NT;
+          kk[u] = i < end ? KeyOf<InT>::to(src[i]) : (K)0;
+        }
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (o + (uint64_t)u * NT >= end) break;
-        uint32_t bin;
-        if (Q) bin = qbin<K>(kk[u], s.lo, s.shift, qb, qd);
-        else bin = min((uint32_t)((K)(kk[u] - s.lo) >> s.shift), (uint32_t)NBIN - 1u);
-        atomicAdd(&h[bin], 1u);
+        for (int u = 0; u < U; ++u) {
+          if (o + (uint64_t)u * NT >= end) break;
+          atomicAdd(&h[qbin<K>(kk[u], s.lo, s.shift, qb, qd)], 1u);
+        }
       }
+    } else {
+      tile_stream<K, NT>(src, beg, end, [&](const K* k, uint32_t mask) {
+#pragma unroll
+        for (int t = 0; t < 16 / (int)sizeof(K); ++t)
+          if ((mask >> t) & 1u)
+            atomicAdd(&h[min((uint32_t)((K)(k[t] - s.lo) >> s.shift), (uint32_t)NBIN - 1u)], 1u);
+      });
     }
     open_keys += end - beg;
     __syncthreads();
@@ -2283,34 +2324,48 @@ __global__ __launch_bounds__(NT) void lvl_count(const InT* __restrict__ src,
   if (open != 0xFFFFFFFFu) flush();  // the last tile ended with a barrier
 }
 
-__global__ __launch_bounds__(1024) void lvl_scan(uint32_t* rows, const uint32_t* __restrict__ bigs,
-                                                  const Counters* __restrict__ C, int p, Caps caps) {
+template <typename InT, int NT, bool Q = false>
+__global__ __launch_bounds__(NT) void lvl_count(const InT* __restrict__ src,
+                                               const Seg<typename KeyOf<InT>::K>* __restrict__ segs,
+                                               const TileRef* __restrict__ tiles,
+                                               Counters* C, int p, uint32_t* rows, Caps caps,
+                                               const typename KeyOf<InT>::K* __restrict__ qtab,
+                                               const uint16_t* __restrict__ qdir) {
+  pdl_entry();
+  __shared__ uint32_t h[NBIN];
+  count_body<InT, NT, Q>(src, segs, tiles, C, p, rows, caps, qtab, qdir, h, blockIdx.x, gridDim.x);
+}
+
+// w: 72 words of shared memory
+template <int NT>
+__device__ __forceinline__ void scan_body(uint32_t* rows, const Counters* C, int p, const Caps& caps, uint32_t* w,
+                                          uint32_t cta, uint32_t ncta) {
+  const uint32_t nb = min(C->nbig[p], caps.rows);
+  for (uint32_t j = cta; j < nb; j += ncta)
+    block_inclusive_scan_global<NT>(rows + (size_t)j * NBIN, NBIN, w, nullptr);
+}
+
+__global__ __launch_bounds__(1024) void lvl_scan(uint32_t* rows, const Counters* __restrict__ C, int p, Caps caps) {
   pdl_entry();
   __shared__ uint32_t w[72];
-  const uint32_t nb = min(C->nbig[p], caps.segs);
-  for (uint32_t j = blockIdx.x; j < nb; j += gridDim.x)
-    block_inclusive_scan_global<1024>(rows + (size_t)bigs[j] * NBIN, NBIN, w, nullptr);
+  scan_body<1024>(rows, C, p, caps, w, blockIdx.x, gridDim.x);
 }
 
 // Active bins of each segment -> child segments (pool q) or points.  One CTA
 // per segment; the row holding the inclusive counts is overwritten by the
 // child map (each entry read before any is written).
 template <typename K, int NT, bool Q = false>
-__global__ __launch_bounds__(NT) void lvl_children(uint32_t* rows, const uint32_t* __restrict__ aflag,
-                                                  const Seg<K>* __restrict__ segs, Counters* C, int p,
-                                                  Seg<K>* segs_q, uint32_t* cursor_q, TileRef* tiles_q,
-                                                  K* points, uint32_t* khead_q, uint32_t* smalls,
-                                                  uint32_t* tinies, const uint32_t* __restrict__ bigs,
-                                                  uint32_t* bigs_q, Caps caps, const K* __restrict__ qtab) {
-  pdl_entry();
+__device__ __forceinline__ void children_body(uint32_t* rows, const uint32_t* aflag, const Seg<K>* segs,
+                                              Counters* C, int p, Seg<K>* segs_q, uint32_t* cursor_q,
+                                              TileRef* tiles_q, K* points, uint32_t* khead_q, uint32_t* smalls,
+                                              uint32_t* tinies, const uint32_t* bigs, uint32_t* bigs_q,
+                                              const Caps& caps, const K* qtab, uint32_t cta, uint32_t ncta) {
   constexpr int PER = NBIN / NT;
-  const uint32_t nb = min(C->nbig[p], caps.segs);
-  for (uint32_t j = blockIdx.x; j < nb; j += gridDim.x) {
-    const uint32_t sid = bigs[j];
-    const Seg<K> s = segs[sid];
-    if (s.small) continue;  // finished by small_select
-    uint32_t* I = rows + (size_t)sid * NBIN;
-    const uint32_t* F = aflag + (size_t)sid * NBIN_WORDS;
+  const uint32_t nb = min(C->nbig[p], caps.rows);
+  for (uint32_t j = cta; j < nb; j += ncta) {
+    const Seg<K> s = segs[bigs[j]];
+    uint32_t* I = rows + (size_t)j * NBIN;
+    const uint32_t* F = aflag + (size_t)j * NBIN_WORDS;
     uint32_t out[PER];
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
@@ -2349,23 +2404,26 @@ __global__ __launch_bounds__(NT) void lvl_children(uint32_t* rows, const uint32_
       c.lo = blo;
       c.hi = bhi;
       c.shift = (uint32_t)max(0, bitlen((K)(bhi - blo)) - RADIX_BITS);
-      c.small = cnt <= caps.small_keys ? 1u : 0u;
+      const bool small = cnt <= caps.small_keys;
+      c.row = SEG_SMALL;
+      if (!small) {
+        c.row = atomicAdd(&C->nbig[p ^ 1], 1u);
+        if (c.row < caps.rows) bigs_q[c.row] = id; else set_status(C, GGMS_E_INTERNAL);
+      }
       c.pad = 0u;
       segs_q[id] = c;
       cursor_q[id] = 0u;
       khead_q[id] = K_NIL;
       out[u] = id;
-      if (c.small) {
+      if (small) {
         const bool tiny = cnt <= caps.tiny_keys;
         const uint32_t si = atomicAdd(tiny ? &C->ntiny : &C->nsmall, 1u);
         if (si < caps.segs) (tiny ? tinies : smalls)[si] = id; else set_status(C, GGMS_E_INTERNAL);
         continue;
       }
-      const uint32_t bi = atomicAdd(&C->nbig[p ^ 1], 1u);
-      if (bi < caps.segs) bigs_q[bi] = id; else set_status(C, GGMS_E_INTERNAL);
       const uint32_t nt = (cnt + TILE - 1) / TILE;
       const uint32_t t0 = atomicAdd(&C->ntiles[p ^ 1], nt);
-      if (t0 + nt > caps.tiles || t0 + nt < t0) { set_status(C, GGMS_E_INTERNAL); continue; }
+      if (c.row >= caps.rows || t0 + nt > caps.tiles || t0 + nt < t0) { set_status(C, GGMS_E_INTERNAL); continue; }
       for (uint32_t t = 0; t < nt; ++t) tiles_q[t0 + t] = TileRef{id, t};
     }
     __syncthreads();
@@ -2375,10 +2433,163 @@ __global__ __launch_bounds__(NT) void lvl_children(uint32_t* rows, const uint32_
   }
 }
 
+template <typename K, int NT, bool Q = false>
+__global__ __launch_bounds__(NT) void lvl_children(uint32_t* rows, const uint32_t* __restrict__ aflag,
+                                                  const Seg<K>* __restrict__ segs, Counters* C, int p,
+                                                  Seg<K>* segs_q, uint32_t* cursor_q, TileRef* tiles_q,
+                                                  K* points, uint32_t* khead_q, uint32_t* smalls,
+                                                  uint32_t* tinies, const uint32_t* __restrict__ bigs,
+                                                  uint32_t* bigs_q, Caps caps, const K* __restrict__ qtab) {
+  pdl_entry();
+  children_body<K, NT, Q>(rows, aflag, segs, C, p, segs_q, cursor_q, tiles_q, points, khead_q, smalls, tinies,
+                          bigs, bigs_q, caps, qtab, blockIdx.x, gridDim.x);
+}
+
 // Copies each key whose bin became a child segment into that child's region.
 // Tiles go to CTAs grid-stride, so the CTAs running at one time fill the same
 // children side by side and L2 merges their partial sectors (contiguous tile
 // ranges per CTA measured 24 % slower on the 4096-segment batch).
+// A tile's hits (3 % of its keys in a typical level) go through a per-warp
+// queue and are written 32 at a time, one per lane: the cursor reservations of
+// 32 hits are then one round trip to L2, where reserving each hit as it was
+// found paid a trip per hit.  (The batched level 0, where 12 % are hits, has
+// enough of them in flight without the queue: 13.9 ms with it, 13.2 without.)
+// cm: NBIN words of shared memory, then the queues (COMPACT_SMEM bytes in all).
+template <typename K, int NT>
+constexpr size_t COMPACT_SMEM = 4u * NBIN + (NT / 32) * WQ_DEPTH * (sizeof(K) + 4u);
+
+template <typename InT, int NT, bool Q = false>
+__device__ __forceinline__ void compact_body(const InT* src, const Seg<typename KeyOf<InT>::K>* segs,
+                                             const TileRef* tiles, const Counters* C, int p, const uint32_t* rows,
+                                             const Seg<typename KeyOf<InT>::K>* segs_q, uint32_t* cursor_q,
+                                             typename KeyOf<InT>::K* dst, const Caps& caps,
+                                             const typename KeyOf<InT>::K* qtab, const uint16_t* qdir,
+                                             uint32_t* cm, uint32_t cta, uint32_t ncta) {
+  using K = typename KeyOf<InT>::K;
+  __shared__ __align__(16) K qb[Q ? QB : 1];
+  __shared__ __align__(16) uint16_t qd[Q ? QDS : 8];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lt = lanemask_lt();
+  K* qk = reinterpret_cast<K*>(cm + NBIN) + warp * WQ_DEPTH;
+  uint32_t* qc = reinterpret_cast<uint32_t*>(reinterpret_cast<K*>(cm + NBIN) + (NT / 32) * WQ_DEPTH) + warp * WQ_DEPTH;
+  uint32_t qn = 0;  // warp-uniform queue fill
+  // the lanes of `mask` write one hit each: one reservation per group of lanes
+  // with the same child
+  auto emit = [&](uint32_t mask, K key, uint32_t c) {
+    const uint32_t peers = __match_any_sync(mask, c);
+    const int leader = __ffs(peers) - 1;
+    uint32_t base = 0;
+    if ((int)lane == leader) base = atomicAdd(&cursor_q[c], (uint32_t)__popc(peers));
+    base = __shfl_sync(peers, base, leader);
+    const uint32_t slot = base + __popc(peers & lt);
+    const Seg<K>& sg = segs_q[c];
+    if (slot < sg.cnt) dst[sg.off + slot] = key;
+    else set_status(const_cast<Counters*>(C), GGMS_E_INTERNAL);
+  };
+  const uint32_t nt = min(C->ntiles[p], caps.tiles);
+  const uint32_t ns = min(C->nsegs[p], caps.segs);
+  if (Q && nt && cta == 0 && threadIdx.x == 0)  // level 0 reads the input
+    atomicAdd(&const_cast<Counters*>(C)->passes, 1u);
+  uint32_t loaded = 0xFFFFFFFFu;  // segment whose child map (and table) is in shared memory
+  for (uint32_t t = cta; t < nt; t += ncta) {
+    const TileRef tr = tiles[t];
+    if (tr.seg >= ns) continue;  // only after a capacity error (status already set)
+    const Seg<K> s = segs[tr.seg];
+    if (tr.seg != loaded) {  // the previous tile ended with a barrier
+      const uint32_t* row = rows + (size_t)s.row * NBIN;
+      for (uint32_t i = threadIdx.x; i < NBIN; i += NT) cm[i] = row[i];
+      if (Q) qtab_to_smem<K>(qtab, qdir, s.pad, qb, qd);
+      loaded = tr.seg;
+    }
+    __syncthreads();
+    const uint64_t beg = s.off + (uint64_t)tr.no * TILE;
+    const uint64_t end = min(beg + TILE, s.off + s.cnt);
+    if constexpr (Q) {
+      constexpr int U = 4;  // loads in flight per thread before the warp-synchronous part
+      const uint64_t span = ((end - beg + NT * U - 1) / (NT * U)) * (NT * U);
+      for (uint64_t o = threadIdx.x; o < span; o += NT * U) {
+        K kk[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const uint64_t i = beg + o + (uint64_t)u * NT;
+          kk[u] = i < end ? KeyOf<InT>::to(src[i]) : (K)0;
+        }
+        // each key's child (CM_NONE when its bin is not copied)
+        uint32_t cc[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          cc[u] = beg + o + (uint64_t)u * NT < end ? cm[qbin<K>(kk[u], s.lo, s.shift, qb, qd)] : CM_NONE;
+        // one cursor reservation per group of lanes with the same child, for
+        // all U keys before any result is used
+        uint32_t peers[U], base[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const bool hit = cc[u] < CM_POINT;
+          const uint32_t hm = __ballot_sync(FULL, hit);
+          peers[u] = 0u;
+          base[u] = 0u;
+          if (hit) {
+            peers[u] = __match_any_sync(hm, cc[u]);
+            if ((int)lane == __ffs(peers[u]) - 1) base[u] = atomicAdd(&cursor_q[cc[u]], (uint32_t)__popc(peers[u]));
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (peers[u]) {
+            const uint32_t b0 = __shfl_sync(peers[u], base[u], __ffs(peers[u]) - 1);
+            const uint32_t slot = b0 + __popc(peers[u] & lt);
+            const Seg<K>& sg = segs_q[cc[u]];
+            if (slot < sg.cnt) dst[sg.off + slot] = kk[u];
+            else set_status(const_cast<Counters*>(C), GGMS_E_INTERNAL);
+          }
+        }
+      }
+    } else {
+      tile_stream<K, NT>(src, beg, end, [&](const K* k, uint32_t mask) {
+        constexpr int N = 16 / (int)sizeof(K);
+        uint32_t cc[N];
+        bool any = false;
+#pragma unroll
+        for (int t = 0; t < N; ++t) {
+          cc[t] = cm[min((uint32_t)((K)(k[t] - s.lo) >> s.shift), (uint32_t)NBIN - 1u)];
+          if (!((mask >> t) & 1u)) cc[t] = CM_NONE;
+          any = any || cc[t] < CM_POINT;
+        }
+        if (!__any_sync(FULL, any)) return;
+#pragma unroll
+        for (int t = 0; t < N; ++t) {
+          const bool hit = cc[t] < CM_POINT;
+          const uint32_t hm = __ballot_sync(FULL, hit);
+          if (hit) {
+            const uint32_t at = qn + __popc(hm & lt);
+            qk[at] = k[t];
+            qc[at] = cc[t];
+          }
+          qn += __popc(hm);
+          if (qn >= 32u) {
+            __syncwarp();
+            const K k0 = qk[lane];
+            const uint32_t c0 = qc[lane];
+            const bool more = lane + 32u < qn;
+            const K k1 = more ? qk[lane + 32u] : (K)0;
+            const uint32_t c1 = more ? qc[lane + 32u] : 0u;
+            __syncwarp();
+            if (more) {
+              qk[lane] = k1;
+              qc[lane] = c1;
+            }
+            qn -= 32u;
+            __syncwarp();
+            emit(FULL, k0, c0);
+          }
+        }
+      });
+    }
+    __syncthreads();
+  }
+  __syncwarp();
+  if (lane < qn) emit((1u << qn) - 1u, qk[lane], qc[lane]);  // qn < 32
+}
+
 template <typename InT, int NT, bool Q = false>
 __global__ __launch_bounds__(NT) void lvl_compact(const InT* __restrict__ src,
                                                  const Seg<typename KeyOf<InT>::K>* __restrict__ segs,
@@ -2390,82 +2601,10 @@ __global__ __launch_bounds__(NT) void lvl_compact(const InT* __restrict__ src,
                                                  Caps caps, const typename KeyOf<InT>::K* __restrict__ qtab,
                                                  const uint16_t* __restrict__ qdir) {
   pdl_entry();
-  using K = typename KeyOf<InT>::K;
-  __shared__ uint32_t cm[NBIN];
-  __shared__ __align__(16) K qb[Q ? QB : 1];
-  __shared__ __align__(16) uint16_t qd[Q ? QDS : 8];
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t nt = min(C->ntiles[p], caps.tiles);
-  const uint32_t ns = min(C->nsegs[p], caps.segs);
-  if (Q && nt && blockIdx.x == 0 && threadIdx.x == 0)  // level 0 reads the input
-    atomicAdd(&const_cast<Counters*>(C)->passes, 1u);
-  uint32_t loaded = 0xFFFFFFFFu;  // segment whose child map (and table) is in shared memory
-  for (uint32_t t = blockIdx.x; t < nt; t += gridDim.x) {
-    const TileRef tr = tiles[t];
-    if (tr.seg >= ns) continue;  // only after a capacity error (status already set)
-    const Seg<K> s = segs[tr.seg];
-    if (tr.seg != loaded) {  // the previous tile ended with a barrier
-      const uint32_t* row = rows + (size_t)tr.seg * NBIN;
-      for (uint32_t i = threadIdx.x; i < NBIN; i += NT) cm[i] = row[i];
-      if (Q) qtab_to_smem<K>(qtab, qdir, s.pad, qb, qd);
-      loaded = tr.seg;
-    }
-    __syncthreads();
-    const uint64_t beg = s.off + (uint64_t)tr.no * TILE;
-    const uint64_t end = min(beg + TILE, s.off + s.cnt);
-    constexpr int U = 4;  // loads in flight per thread before the warp-synchronous part
-    const uint64_t span = ((end - beg + NT * U - 1) / (NT * U)) * (NT * U);
-    for (uint64_t o = threadIdx.x; o < span; o += NT * U) {
-      K kk[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const uint64_t i = beg + o + (uint64_t)u * NT;
-        kk[u] = i < end ? KeyOf<InT>::to(src[i]) : (K)0;
-      }
-      // 1. each key's child (CM_NONE when its bin is not copied)
-      uint32_t cc[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        cc[u] = CM_NONE;
-        if (beg + o + (uint64_t)u * NT < end) {
-          uint32_t bin;
-          if (Q) bin = qbin<K>(kk[u], s.lo, s.shift, qb, qd);
-          else bin = min((uint32_t)((K)(kk[u] - s.lo) >> s.shift), (uint32_t)NBIN - 1u);
-          cc[u] = cm[bin];
-        }
-      }
-      // 2. one cursor reservation per group of lanes with the same child, for
-      // all U keys before any result is used: the U global atomics of a warp
-      // are in flight together instead of one round trip after another
-      uint32_t peers[U], base[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const bool hit = cc[u] < CM_POINT;
-        const uint32_t hm = __ballot_sync(FULL, hit);
-        peers[u] = 0u;
-        base[u] = 0u;
-        if (hit) {
-          peers[u] = __match_any_sync(hm, cc[u]);
-          if ((int)lane == __ffs(peers[u]) - 1) base[u] = atomicAdd(&cursor_q[cc[u]], (uint32_t)__popc(peers[u]));
-        }
-      }
-      // 3. the stores
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (peers[u]) {
-          const uint32_t b0 = __shfl_sync(peers[u], base[u], __ffs(peers[u]) - 1);
-          const uint32_t slot = b0 + __popc(peers[u] & lanemask_lt());
-          const Seg<K>& sg = segs_q[cc[u]];
-          if (slot < sg.cnt) dst[sg.off + slot] = kk[u];
-          else set_status(const_cast<Counters*>(C), GGMS_E_INTERNAL);
-        }
-      }
-    }
-    __syncthreads();
-  }
+  __shared__ __align__(16) uint32_t cm[Q ? NBIN : COMPACT_SMEM<typename KeyOf<InT>::K, NT> / 4];
+  compact_body<InT, NT, Q>(src, segs, tiles, C, p, rows, segs_q, cursor_q, dst, caps, qtab, qdir, cm, blockIdx.x,
+                           gridDim.x);
 }
-
-
 
 // ------------------------------------------------------------------ small segments
 // One CTA finishes a whole small segment in shared memory: its keys (as
@@ -2478,21 +2617,17 @@ constexpr int SS_GROUP = 16;
 constexpr int SS_MAXK = 256;
 constexpr int SS_SORT_ABOVE = 64;   // more ks than this in one segment: bitonic sort instead
 
+// smem: SMALL_SELECT_SMEM bytes of dynamic shared memory.
+constexpr size_t SMALL_SELECT_SMEM = SMALL_SMEM + (size_t)SS_GROUP * 256 * 4;
+
 template <typename InT, int NT>
-__global__ __launch_bounds__(NT) void small_select(const InT* __restrict__ src,
-                                                  const Seg<typename KeyOf<InT>::K>* __restrict__ segs_q,
-                                                  const uint32_t* __restrict__ smalls,
-                                                  const Counters* __restrict__ C_,
-                                                  const uint32_t* __restrict__ khead_q,
-                                                  const uint32_t* __restrict__ knext,
-                                                  const int64_t* __restrict__ k_off,
-                                                  const uint32_t* __restrict__ k_rank, uint32_t* k_seg,
+__device__ __forceinline__ void small_select_body(const InT* src, const Seg<typename KeyOf<InT>::K>* segs_q,
+                                                  const uint32_t* smalls, Counters* C, const uint32_t* khead_q,
+                                                  const uint32_t* knext, const int64_t* k_off,
+                                                  const uint32_t* k_rank, uint32_t* k_seg,
                                                   typename KeyOf<InT>::K* k_key, uint32_t small_keys,
-                                                  Caps caps) {
-  pdl_entry();
+                                                  const Caps& caps, uint8_t* smem, uint32_t cta, uint32_t ncta) {
   using K = typename KeyOf<InT>::K;
-  Counters* C = const_cast<Counters*>(C_);
-  extern __shared__ __align__(128) uint8_t smem[];
   K* vals = (K*)smem;
   uint32_t* hist = (uint32_t*)(smem + SMALL_SMEM);           // [SS_GROUP][256]
   __shared__ uint32_t kid[SS_MAXK];
@@ -2502,10 +2637,11 @@ __global__ __launch_bounds__(NT) void small_select(const InT* __restrict__ src,
   __shared__ K upk[SS_GROUP];       // distinct prefixes of the current round
   __shared__ uint32_t hmap[SS_GROUP];  // k -> its prefix's histogram
   __shared__ uint32_t nuniq;
+  __shared__ K rng[2][NT / 32];
   GGMS_TRACE(35);
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t ns = min(C->nsmall, caps.segs);
-  for (uint32_t t = blockIdx.x; t < ns; t += gridDim.x) {
+  for (uint32_t t = cta; t < ns; t += ncta) {
     const uint32_t id = smalls[t];
     const Seg<K> s = segs_q[id];
     const uint32_t cnt = min(s.cnt, small_keys);
@@ -2523,7 +2659,31 @@ __global__ __launch_bounds__(NT) void small_select(const InT* __restrict__ src,
         if (i < cnt) vals[i] = (K)(v[q] - s.lo);
       }
     }
-    const int bits = bitlen((K)(s.hi - s.lo));
+    // the keys' true range: a radix round less for every 8 bits it saves
+    K mn = key_max<K>(), mx = 0;
+    for (uint32_t i = tid; i < cnt; i += NT) {  // this thread's own keys
+      mn = min(mn, vals[i]);
+      mx = max(mx, vals[i]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const K x = __shfl_xor_sync(FULL, mn, o), y = __shfl_xor_sync(FULL, mx, o);
+      mn = min(mn, x);
+      mx = max(mx, y);
+    }
+    if (lane == 0) {
+      rng[0][warp] = mn;
+      rng[1][warp] = mx;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < NT / 32; ++w) {
+      mn = min(mn, rng[0][w]);
+      mx = max(mx, rng[1][w]);
+    }
+    const K base = (K)(s.lo + mn);
+    for (uint32_t i = tid; i < cnt; i += NT) vals[i] = (K)(vals[i] - mn);
+    const int bits = bitlen((K)(mx - mn));
     bool sorted_seg = false;
     if (tid == 0) {  // the ks: the segment's list, or (k_off: a caller segment) its k range
       if (k_off) {
@@ -2577,7 +2737,7 @@ __global__ __launch_bounds__(NT) void small_select(const InT* __restrict__ src,
         for (uint32_t j = tid; j < m; j += NT) {
           const uint32_t k = kid[j];
           const uint32_t r = k_rank[k];
-          if (r < cnt) k_key[k] = (K)(s.lo + vals[r]);
+          if (r < cnt) k_key[k] = (K)(base + vals[r]);
           else set_status(C, GGMS_E_INTERNAL);
           k_seg[k] = K_DONE;
         }
@@ -2653,7 +2813,7 @@ __global__ __launch_bounds__(NT) void small_select(const InT* __restrict__ src,
         __syncthreads();
         if (tid < g) {
           const uint32_t k = kid[g0 + tid];
-          k_key[k] = (K)(s.lo + pk[tid]);
+          k_key[k] = (K)(base + pk[tid]);
           k_seg[k] = K_DONE;
         }
         __syncthreads();
@@ -2664,6 +2824,23 @@ __global__ __launch_bounds__(NT) void small_select(const InT* __restrict__ src,
   }
   GGMS_TRACE(36);
   GGMS_TRACE_CTA(4);
+}
+
+template <typename InT, int NT>
+__global__ __launch_bounds__(NT) void small_select(const InT* __restrict__ src,
+                                                  const Seg<typename KeyOf<InT>::K>* __restrict__ segs_q,
+                                                  const uint32_t* __restrict__ smalls,
+                                                  const Counters* __restrict__ C_,
+                                                  const uint32_t* __restrict__ khead_q,
+                                                  const uint32_t* __restrict__ knext,
+                                                  const int64_t* __restrict__ k_off,
+                                                  const uint32_t* __restrict__ k_rank, uint32_t* k_seg,
+                                                  typename KeyOf<InT>::K* k_key, uint32_t small_keys,
+                                                  Caps caps) {
+  pdl_entry();
+  extern __shared__ __align__(128) uint8_t smem[];
+  small_select_body<InT, NT>(src, segs_q, smalls, const_cast<Counters*>(C_), khead_q, knext, k_off, k_rank, k_seg,
+                             k_key, small_keys, caps, smem, blockIdx.x, gridDim.x);
 }
 
 // One warp finishes a whole tiny segment (at most tiny_keys<K>() keys, as
@@ -2730,38 +2907,46 @@ __device__ __forceinline__ K warp_radix_select(const K* v, uint32_t cnt, int bit
   return pre;
 }
 
-template <typename InT, int NT>
-__global__ __launch_bounds__(NT) void tiny_select(const InT* __restrict__ src,
-                                                 const Seg<typename KeyOf<InT>::K>* __restrict__ segs_q,
-                                                 const uint32_t* __restrict__ tinies,
-                                                 const Counters* __restrict__ C_,
-                                                 const uint32_t* __restrict__ khead_q,
-                                                 const uint32_t* __restrict__ knext,
-                                                 const int64_t* __restrict__ k_off,
-                                                 const uint32_t* __restrict__ k_rank, uint32_t* k_seg,
-                                                 typename KeyOf<InT>::K* k_key, Caps caps) {
-  // Launched right after small_select, whose output it does not read: it lets
-  // its successor launch and runs beside small_select, and waits for it only
-  // at its end (so that it completes after its predecessor).
-  pdl_trigger();
+// buf, hist: TK keys (a power of two) and 256 words of shared memory per warp.
+template <typename InT, int NW, uint32_t TK>
+__device__ __forceinline__ void tiny_select_body(const InT* src, const Seg<typename KeyOf<InT>::K>* segs_q,
+                                                 const uint32_t* tinies, Counters* C, const uint32_t* khead_q,
+                                                 const uint32_t* knext, const int64_t* k_off,
+                                                 const uint32_t* k_rank, uint32_t* k_seg,
+                                                 typename KeyOf<InT>::K* k_key, const Caps& caps,
+                                                 typename KeyOf<InT>::K* buf, uint32_t* hist, uint32_t cta,
+                                                 uint32_t ncta) {
   using K = typename KeyOf<InT>::K;
-  constexpr uint32_t TK = tiny_keys<K>();
-  constexpr int NW = NT / 32;
-  __shared__ K buf[NW][TK];
-  __shared__ uint32_t hist[NW][256];
-  Counters* C = const_cast<Counters*>(C_);
   const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  K* v = buf[wid];
-  uint32_t* h = hist[wid];
+  K* v = buf + wid * TK;
+  uint32_t* h = hist + wid * 256u;
+  auto sort_slice = [&](uint32_t cnt) {  // bitonic; N <= TK
+    uint32_t N = 32;
+    while (N < cnt) N <<= 1;
+    for (uint32_t i = cnt + lane; i < N; i += 32) v[i] = key_max<K>();
+    __syncwarp();
+    for (uint32_t kk = 2; kk <= N; kk <<= 1) {
+      for (uint32_t jj = kk >> 1; jj > 0; jj >>= 1) {
+        for (uint32_t i = lane; i < N; i += 32) {
+          const uint32_t ixj = i ^ jj;
+          if (ixj > i) {
+            const K a = v[i], b = v[ixj];
+            if ((a > b) == ((i & kk) == 0)) { v[i] = b; v[ixj] = a; }
+          }
+        }
+        __syncwarp();
+      }
+    }
+  };
   const uint32_t nt = min(C->ntiny, caps.segs);
   // a warp takes up to 32 list entries at a time (fewer when the list is short,
   // so that every warp gets work): lane j loads entry j's descriptor and k-list
   // head -- the chain of dependent loads is paid once per batch -- then the warp
   // finishes the segments one by one
   GGMS_TRACE(39);
-  const uint32_t nwarps = gridDim.x * NW;
+  const uint32_t nwarps = ncta * NW;
   const uint32_t batch = max(1u, min(32u, nt / nwarps));
-  for (uint32_t t0 = (blockIdx.x * NW + wid) * batch; t0 < nt; t0 += nwarps * batch) {
+  for (uint32_t t0 = (cta * NW + wid) * batch; t0 < nt; t0 += nwarps * batch) {
     const uint32_t tj = t0 + lane;
     uint32_t pid = 0u, pkh = K_NIL;
     Seg<K> ps{};
@@ -2839,22 +3024,7 @@ __global__ __launch_bounds__(NT) void tiny_select(const InT* __restrict__ src,
       } else if (k_off) {
         const int64_t k0 = k_off[id], k1 = k_off[id + 1];
         if ((uint64_t)(k1 - k0) > TS_SORT_ABOVE) {
-          uint32_t N = 32;
-          while (N < cnt) N <<= 1;
-          for (uint32_t i = cnt + lane; i < N; i += 32) v[i] = key_max<K>();
-          __syncwarp();
-          for (uint32_t kk = 2; kk <= N; kk <<= 1) {
-            for (uint32_t jj = kk >> 1; jj > 0; jj >>= 1) {
-              for (uint32_t i = lane; i < N; i += 32) {
-                const uint32_t ixj = i ^ jj;
-                if (ixj > i) {
-                  const K a = v[i], b = v[ixj];
-                  if ((a > b) == ((i & kk) == 0)) { v[i] = b; v[ixj] = a; }
-                }
-              }
-              __syncwarp();
-            }
-          }
+          sort_slice(cnt);
           for (int64_t k = k0 + lane; k < k1; k += 32) {
             if (k_seg[k] == K_DONE) continue;  // an invalid k (status already set)
             const uint32_t r = k_rank[k];
@@ -2874,11 +3044,17 @@ __global__ __launch_bounds__(NT) void tiny_select(const InT* __restrict__ src,
           }
         }
       } else {
+        uint32_t some = 0;  // ks, up to TS_SORT_ABOVE + 1 of them
+        if (!by_rank)
+          for (uint32_t k = khead; k != K_NIL && some <= TS_SORT_ABOVE; k = knext[k]) ++some;
+        const bool sorted = some > TS_SORT_ABOVE;
+        if (sorted) sort_slice(cnt);
         for (uint32_t k = khead; k != K_NIL; k = knext[k]) {
           bool ok = false;
           const uint32_t r = k_rank[k];
-          const K pre = by_rank ? rank_pick(r, &ok)
-                                : (r < cnt ? warp_radix_select<K>(v, cnt, bits, r, h, lane, &ok) : (K)0);
+          K pre = 0;
+          if (by_rank) pre = rank_pick(r, &ok);
+          else if ((ok = r < cnt)) pre = sorted ? v[r] : warp_radix_select<K>(v, cnt, bits, r, h, lane, &ok);
           if (lane == 0) {
             if (ok) k_key[k] = (K)(s.lo + pre); else set_status(C, GGMS_E_INTERNAL);
             k_seg[k] = K_DONE;
@@ -2891,6 +3067,27 @@ __global__ __launch_bounds__(NT) void tiny_select(const InT* __restrict__ src,
   }
   GGMS_TRACE(40);
   GGMS_TRACE_CTA(5);
+}
+
+template <typename InT, int NT>
+__global__ __launch_bounds__(NT) void tiny_select(const InT* __restrict__ src,
+                                                 const Seg<typename KeyOf<InT>::K>* __restrict__ segs_q,
+                                                 const uint32_t* __restrict__ tinies,
+                                                 const Counters* __restrict__ C,
+                                                 const uint32_t* __restrict__ khead_q,
+                                                 const uint32_t* __restrict__ knext,
+                                                 const int64_t* __restrict__ k_off,
+                                                 const uint32_t* __restrict__ k_rank, uint32_t* k_seg,
+                                                 typename KeyOf<InT>::K* k_key, Caps caps) {
+  // Launched right after small_select, whose output it does not read: it lets
+  // its successor launch and runs beside small_select, and waits for it only
+  // at its end (so that it completes after its predecessor).
+  pdl_trigger();
+  using K = typename KeyOf<InT>::K;
+  __shared__ K buf[NT / 32 * tiny_keys<K>()];
+  __shared__ uint32_t hist[NT / 32 * 256];
+  tiny_select_body<InT, NT / 32, tiny_keys<K>()>(src, segs_q, tinies, const_cast<Counters*>(C), khead_q, knext, k_off,
+                                                 k_rank, k_seg, k_key, caps, buf, hist, blockIdx.x, gridDim.x);
   pdl_wait();
 }
 
@@ -2915,17 +3112,15 @@ __global__ void seg_init(const int64_t* __restrict__ seg_off, uint32_t nseg,
   d.lo = 0;
   d.hi = key_max<K>();
   d.shift = 0u;
-  d.small = 0u;
+  d.row = SEG_SMALL;
   d.pad = 0u;
   khead0[s] = K_NIL;
   if (b < a) set_status(C, GGMS_E_INVALID_ARG);
-  if (k_off[s + 1] == k_off[s] || d.cnt == 0) {  // nothing to select here
-    d.small = 1u;  // no row, no tiles
+  if (k_off[s + 1] == k_off[s] || d.cnt == 0) {  // nothing to select here: no row, no tiles
     segs0[s] = d;
     return;
   }
   if (d.cnt <= caps.tiny_keys || d.cnt < QSAMP) {
-    d.small = 1u;
     segs0[s] = d;
     const bool tiny = d.cnt <= caps.tiny_keys;
     const uint32_t si = atomicAdd(tiny ? &C->ntiny : &C->nsmall, 1u);
@@ -2933,13 +3128,13 @@ __global__ void seg_init(const int64_t* __restrict__ seg_off, uint32_t nseg,
     return;
   }
   const uint32_t q = atomicAdd(&C->nbig[0], 1u);  // its quantile table: q
-  if (q < caps.segs) bigs0[q] = s;
-  if (q >= cap_q) {  // cannot happen: cap_q bounds the segments of QSAMP keys or more
+  if (q >= cap_q) {  // cannot happen: cap_q (<= caps.rows) bounds the segments of QSAMP keys or more
     set_status(C, GGMS_E_INTERNAL);
-    d.small = 1u;
     segs0[s] = d;
     return;
   }
+  bigs0[q] = s;
+  d.row = q;
   d.pad = q;
   segs0[s] = d;
   const uint32_t nt = (d.cnt + TILE - 1) / TILE;
@@ -2976,19 +3171,7 @@ __global__ void k_init_seg(const uint32_t* __restrict__ ks, uint32_t nk,
   }
   k_rank[i] = (uint32_t)(len - k);
   k_seg[i] = lo;
-  if (segs0[lo].small) knext[i] = atomicExch(&khead0[lo], i);  // lock-free push
-}
-
-// ------------------------------------------------------------------ outputs
-template <typename T>
-__global__ void write_out(const typename KeyOf<T>::K* __restrict__ k_key,
-                          const uint32_t* __restrict__ k_seg, uint32_t nk, T* out, Counters* C) {
-  pdl_entry();
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  GGMS_TRACE(37);
-  if (i >= nk) return;
-  if (k_seg[i] != K_DONE) set_status(C, GGMS_E_NOT_CONVERGED);
-  out[i] = KeyOf<T>::from(k_key[i]);
+  if (segs0[lo].row == SEG_SMALL) knext[i] = atomicExch(&khead0[lo], i);  // lock-free push
 }
 
 GGMS_END
