@@ -1,0 +1,412 @@
+// ggms_batch.cuh -- the batched path: thousands of vectors of uneven length,
+// each with its own ks.
+//
+// batch_init sorts the segments into classes by length, each with a persistent
+// kernel of one CTA per SM:
+//
+//   teams    a segment long against an equal share of the batch goes to a team
+//            of CTAs (half, a quarter, ... of the grid): the one-vector steps of
+//            ggms_direct.cuh with the barriers among the team;
+//   singles  a segment beyond one CTA's sort: the same steps by one CTA (its
+//            barriers are CTA barriers), taken from a shared list, longer ones
+//            first, so that the CTAs end together;
+//   sorts    a segment of up to 32 KB: one CTA sorts it;
+//   rows     up to 16 KB: one warp each.
+//
+// Children that are still large go to the refinement levels, which write the
+// answers.
+//
+// What bounds it: a single CTA counts and copies with private shared-memory
+// histograms and cursors, so the streams are bound by shared-memory bandwidth
+// (the bucket lookup and the histogram atomic, ~9 cycles per 32 keys and SM) and
+// not by a global cursor atomic per copied key as when tiles of a segment were
+// spread over CTAs: 2^30 fp32 in 4096 segments, 1 M ks: 13.3 ms then.
+#pragma once
+#include "ggms_direct.cuh"
+
+namespace ggms {
+
+// Keys of a segment that one warp finishes (32-bit keys): three classes, whose
+// warps hold 1024, 2048 and 4096 keys.
+constexpr uint32_t BT_ROW0 = 1024;
+
+template <typename T>
+struct BatchArgs {
+  using K = typename KeyOf<T>::K;
+  const T* in;
+  const int64_t *seg_off, *k_off;
+  const uint32_t* ks;
+  uint32_t nseg;
+  uint64_t n;
+  uint64_t seed;
+  uint32_t* lists;             // [BT_CLASSES][nseg] segments of each class
+  uint32_t* scratch;           // per CTA: BT_SCRATCH words (a team uses its first CTA's)
+  RefineArgs<T> r;
+};
+constexpr uint32_t BT_SCRATCH = 2 * DIRECT_MAX_B + DIRECT_MAX_B / 32 + 32;
+
+// Enqueues batch_init and the classes' kernels (ggms_batch.cu).
+template <typename T>
+int launch_batch(Context* ctx, const BatchArgs<T>& a, cudaStream_t s);
+
+}  // namespace ggms
+
+GGMS_BEGIN
+
+constexpr uint32_t NONE_YET = 0xFFFFFFFFu;
+
+// A segment's keys and ks; every range is clamped into its array.
+struct SegRange {
+  uint64_t off;
+  uint32_t cnt, k0, nk;
+};
+template <typename T>
+__device__ __forceinline__ SegRange seg_range(const BatchArgs<T>& a, uint32_t s, bool* bad) {
+  const int64_t o0 = a.seg_off[s], o1 = a.seg_off[s + 1], q0 = a.k_off[s], q1 = a.k_off[s + 1];
+  *bad = o1 < o0 || o0 < 0 || (uint64_t)o1 > a.n || q1 < q0 || q0 < 0 || q1 > (int64_t)a.r.nk;
+  SegRange g{0, 0u, 0u, 0u};
+  if (!*bad) g = SegRange{(uint64_t)o0, (uint32_t)(o1 - o0), (uint32_t)q0, (uint32_t)(q1 - q0)};
+  return g;
+}
+
+// A CTA's equal share of the batch, but no fewer keys than repay a team's
+// barriers.
+__device__ __forceinline__ uint64_t batch_share(uint64_t n, uint32_t ncta) {
+  return max((uint64_t)(1u << 18), n / ncta);
+}
+// Team level of a segment (BT_TEAMS: a single CTA): CTAs for about a share
+// each.  A single CTA is the cheapest per key (no barriers, no global
+// histogram); it takes segments of up to two shares, the longest first.
+__device__ __forceinline__ uint32_t team_level(uint64_t cnt, uint64_t n, uint32_t ncta) {
+  const uint64_t t = cnt / batch_share(n, ncta);
+  if (t <= 1u) return BT_TEAMS;
+  uint32_t l = 0;
+  while (l + 1u < BT_TEAMS && (uint64_t)(ncta >> (l + 1u)) >= t) ++l;
+  return l;
+}
+
+// Every segment into its class's list; an unresolved k counts as an error, so
+// the ks start as resolved to key 0 and invalid ones stay that way.
+template <typename T>
+__global__ void batch_init(const __grid_constant__ BatchArgs<T> a, uint32_t ncta) {
+  Counters* C = a.r.C;
+  const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x, gs = gridDim.x * blockDim.x;
+  for (uint32_t i = gt; i < a.r.nk; i += gs) {
+    a.r.kseg[i] = K_DONE;
+    a.r.kkey[i] = 0;
+  }
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t end = (a.nseg + 31u) & ~31u;  // whole warps: the appends below are per warp
+  for (uint32_t s = gt; s < end; s += gs) {
+    bool bad = false;
+    uint32_t cls = BT_CLASSES;
+    if (s < a.nseg) {
+      const SegRange g = seg_range(a, s, &bad);
+      if (bad) set_status(C, GGMS_E_INVALID_ARG);
+      if (g.nk) {
+        constexpr uint32_t CAP = direct_cap<typename KeyOf<T>::K>();
+        if (g.cnt <= BT_ROW0 << 2) {
+          cls = BT_WARP + (g.cnt > BT_ROW0) + (g.cnt > BT_ROW0 << 1);
+        } else if (g.cnt <= CAP) {
+          cls = BT_SORT;
+        } else {
+          cls = team_level(g.cnt, a.n, ncta);
+          if (cls == BT_TEAMS) {  // single: halves of the longest a single CTA gets
+            const uint64_t most = 2u * batch_share(a.n, ncta);
+            while (cls + 1u < BT_SORT && (uint64_t)g.cnt << (cls + 1u - BT_TEAMS) <= most) ++cls;
+          }
+        }
+      }
+    }
+    const uint32_t peers = __match_any_sync(FULL, cls);
+    if (cls < BT_CLASSES) {
+      uint32_t base = 0;
+      const int leader = __ffs(peers) - 1;
+      if ((int)lane == leader) base = atomicAdd(&C->nlist[cls], (uint32_t)__popc(peers));
+      base = __shfl_sync(peers, base, leader);
+      a.lists[(size_t)cls * a.nseg + base + __popc(peers & lanemask_lt())] = s;
+    }
+  }
+}
+
+// direct_body's task for one segment (thread 0 fills it in shared memory: its
+// fields are read where they are used and hold no registers through the streams).
+template <typename T>
+__device__ __forceinline__ void batch_task(const BatchArgs<T>& a, uint32_t s, uint32_t first, uint32_t cta,
+                                           uint32_t ncta, uint32_t* bar, DirectTask<T>& t) {
+  bool bad = false;
+  const SegRange g = seg_range(a, s, &bad);
+  t.in = a.in + g.off;
+  t.n = g.cnt;
+  t.ks = a.ks + g.k0;
+  t.nk = g.nk;
+  t.seed = a.seed ^ ((uint64_t)s << 32);
+  uint32_t B = g.cnt < (1u << 20) ? DIRECT_MAX_B / 2 : DIRECT_MAX_B;
+  while (B > 1024u && B > g.cnt / 8u) B >>= 1;
+  t.B = B;
+  t.focus = 0u;
+  t.slices = ncta > 1u && g.nk > 2048u ? 1u : 0u;
+  t.ghist = a.scratch + (size_t)first * BT_SCRATCH;
+  t.gcur = t.ghist + DIRECT_MAX_B;
+  t.gact = t.gcur + DIRECT_MAX_B;
+  t.bar = bar;
+  t.cta = cta;
+  t.ncta = ncta;
+  t.off = g.off;
+  t.k0 = g.k0;
+}
+
+// What batch_teams hands to team_vector, behind direct_body's shared memory.
+template <typename T>
+struct TeamShared {
+  DirectTask<T> task;
+  RefineArgs<T> r;
+  uint32_t cls, next;  // the loop's state
+};
+template <typename T>
+constexpr size_t team_smem() {
+  return direct_smem<typename KeyOf<T>::K>() + sizeof(TeamShared<T>);
+}
+
+// A function of its own, so that the loop over the segments holds no registers
+// while a segment is worked on.  It names the shared memory itself: handed a
+// pointer, every access would be a generic one (the count ran at half speed).
+template <typename T>
+__device__ __noinline__ bool team_vector() {
+  extern __shared__ __align__(128) uint8_t smem[];
+  const TeamShared<T>& b = *reinterpret_cast<const TeamShared<T>*>(smem + direct_smem<typename KeyOf<T>::K>());
+  return direct_body<T, false>(b.task, b.r, smem);
+}
+
+// Segments of teams: a cooperative launch of gridDim.x CTAs.  Level l has 2^l
+// teams; team i is the CTAs [gridDim.x i / 2^l, gridDim.x (i + 1) / 2^l): every
+// team lies inside one team of the level above, so its CTAs come to it together
+// and no barrier waits for a CTA that is still in another team's segment.
+template <typename T>
+__global__ __launch_bounds__(DR_NT, 1) void batch_teams(const __grid_constant__ BatchArgs<T> a) {
+  using K = typename KeyOf<T>::K;
+  extern __shared__ __align__(128) uint8_t smem[];
+  TeamShared<T>& sh = *reinterpret_cast<TeamShared<T>*>(smem + direct_smem<K>());
+  Counters* C = a.r.C;
+  if (threadIdx.x == 0) {
+    sh.r = a.r;
+    sh.cls = 0u;
+    sh.next = NONE_YET;
+    if (blockIdx.x == 0) {  // the count and the copy read the segments beyond one CTA's sort
+      uint32_t m = 0;
+      for (uint32_t c = 0; c < BT_SORT; ++c) m += C->nlist[c];
+      if (m) atomicAdd(&C->passes, 2u);
+    }
+  }
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const uint32_t me = blockIdx.x, nc = gridDim.x;
+      for (; sh.cls < BT_TEAMS; ++sh.cls, sh.next = NONE_YET) {
+        const uint32_t cls = sh.cls, teams = 1u << cls, i = ((me + 1u) * teams - 1u) / nc;
+        const uint32_t j = sh.next == NONE_YET ? i : sh.next;
+        if (j >= C->nlist[cls]) continue;
+        sh.next = j + teams;
+        const uint32_t first = nc * i / teams, size = nc * (i + 1u) / teams - first;
+        batch_task<T>(a, a.lists[(size_t)cls * a.nseg + j], first, me - first, size, a.r.bar + cls * nc + first,
+                      sh.task);
+        break;
+      }
+    }
+    __syncthreads();
+    if (sh.cls == BT_TEAMS) return;
+    if (!team_vector<T>()) return;
+  }
+}
+
+// Segments of single CTAs: CTA j takes the j-th, longest class first, so the
+// hardware's scheduling deals them out as CTAs end.  (A persistent loop took
+// registers from the streams: 0.24 ns per key and CTA against 0.15.)
+template <typename T>
+__global__ __launch_bounds__(DR_NT, 1) void batch_singles(const __grid_constant__ BatchArgs<T> a) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ DirectTask<T> task;
+  uint32_t cls = BT_TEAMS, j = blockIdx.x;
+  for (; cls < BT_SORT; ++cls) {
+    const uint32_t m = a.r.C->nlist[cls];
+    if (j < m) break;
+    j -= m;
+  }
+  if (cls == BT_SORT) return;
+  if (threadIdx.x == 0) batch_task<T>(a, a.lists[(size_t)cls * a.nseg + j], 0u, 0u, 1u, a.r.bar, task);
+  __syncthreads();
+  direct_body<T, true>(task, a.r, smem);
+}
+
+// Segments of one CTA's sort.
+template <typename T>
+__global__ __launch_bounds__(DR_NT, 1) void batch_sorts(const __grid_constant__ BatchArgs<T> a) {
+  using K = typename KeyOf<T>::K;
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ K red_k[2][DR_NT / 32];
+  SortSmem<K>& sm = *reinterpret_cast<SortSmem<K>*>(smem);
+  K* sorted = reinterpret_cast<K*>(smem + sizeof(SortSmem<K>));
+  const uint32_t m = a.r.C->nlist[BT_SORT];
+  for (uint32_t j = blockIdx.x; j < m; j += gridDim.x) {
+    bool bad = false;
+    const SegRange g = seg_range(a, a.lists[(size_t)BT_SORT * a.nseg + j], &bad);
+    const T* in = a.in + g.off;
+    sort_keys<K>(sm, g.cnt, red_k, [&](uint32_t i) { return KeyOf<T>::to(in[i]); },
+                 [&](uint32_t i, K key) { sorted[i] = key; });
+    for (uint32_t i = threadIdx.x; i < g.nk; i += DR_NT) {
+      const uint32_t k = a.ks[g.k0 + i];
+      if (k >= 1u && k <= g.cnt) a.r.kkey[g.k0 + i] = sorted[g.cnt - k];
+      else set_status(a.r.C, GGMS_E_INVALID_ARG);
+    }
+    __syncthreads();
+  }
+}
+
+// One warp per segment of at most ROW keys: the keys are counted into ROW / 2
+// bins uniform in key between the segment's extremes (for floats without the
+// gap around zero, as in DirectMap), placed by bin, and each bin put in order
+// by one lane; every k then reads its rank.  The cost does not depend on the
+// number of ks, where a radix select pays four rounds per k (rows of 600 keys
+// with 4-5 ks: 386 us for 12 M keys).  Up to 64 keys: every key's rank by
+// comparison.  A bin that holds many different keys falls back to a bitonic
+// sort of the row.
+constexpr int RW_NT = 160;  // 5 warps: 4, 2 and 1 CTAs per SM by shared memory
+template <typename K, uint32_t ROW>
+struct RowSmem {
+  K v[ROW], w[ROW];
+  uint32_t h[ROW / 2];
+};
+
+template <typename T, uint32_t ROW>
+__global__ __launch_bounds__(RW_NT) void rows_select(const __grid_constant__ BatchArgs<T> a) {
+  pdl_entry();
+  using K = typename KeyOf<T>::K;
+  constexpr uint32_t RW_BINS = ROW / 2;
+  constexpr int RW_BITS = ROW == BT_ROW0 ? 9 : ROW == BT_ROW0 << 1 ? 10 : 11;
+  constexpr uint32_t CLS = BT_WARP + RW_BITS - 9;
+  constexpr bool FP = std::is_floating_point<T>::value;
+  constexpr K MID = (K)((K)1 << (sizeof(K) * 8 - 1));
+  extern __shared__ __align__(128) uint8_t smem[];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  RowSmem<K, ROW>& sm = reinterpret_cast<RowSmem<K, ROW>*>(smem)[warp];
+  Counters* C = a.r.C;
+  const uint32_t m = C->nlist[CLS];
+  const uint32_t* list = a.lists + (size_t)CLS * a.nseg;
+  const uint32_t gw = blockIdx.x * (RW_NT / 32) + warp, nw = gridDim.x * (RW_NT / 32);
+  for (uint32_t t0 = gw; t0 < m; t0 += 32u * nw) {
+    // lane j loads the j-th segment's ranges: the dependent loads once for 32
+    SegRange mine{0, 0u, 0u, 0u};
+    bool bad = false;
+    if ((uint64_t)t0 + (uint64_t)lane * nw < m) mine = seg_range(a, list[t0 + lane * nw], &bad);
+    for (uint32_t j = 0; j < 32u && (uint64_t)t0 + (uint64_t)j * nw < m; ++j) {
+      const uint64_t off = __shfl_sync(FULL, mine.off, j);
+      const uint32_t cnt = __shfl_sync(FULL, mine.cnt, j), k0 = __shfl_sync(FULL, mine.k0, j),
+                     nk = __shfl_sync(FULL, mine.nk, j);
+      const T* in = a.in + off;
+      K* sorted = sm.w;
+      if (cnt <= 64u) {
+        const K ka = lane < cnt ? KeyOf<T>::to(in[lane]) : key_max<K>();
+        const K kb = lane + 32u < cnt ? KeyOf<T>::to(in[lane + 32u]) : key_max<K>();
+        sm.v[lane] = ka;
+        sm.v[lane + 32u] = kb;
+        __syncwarp();
+        uint32_t ra = 0, rb = 0;
+        for (uint32_t i = 0; i < cnt; ++i) {
+          const K x = sm.v[i];
+          ra += (x < ka || (x == ka && i < lane)) ? 1u : 0u;
+          rb += (x < kb || (x == kb && i < lane + 32u)) ? 1u : 0u;
+        }
+        if (lane < cnt) sm.w[ra] = ka;
+        if (lane + 32u < cnt) sm.w[rb] = kb;
+        __syncwarp();
+      } else {
+        K lo = key_max<K>(), hi = 0, hn = 0, lp = key_max<K>();
+        for (uint32_t i0 = lane; i0 < cnt; i0 += 32u * 8u) {  // eight loads in flight
+          K x[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            x[q] = i0 + q * 32u < cnt ? KeyOf<T>::to(in[i0 + q * 32u]) : (K)0;
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            if (i0 + q * 32u < cnt) {
+              sm.v[i0 + q * 32u] = x[q];
+              lo = min(lo, x[q]);
+              hi = max(hi, x[q]);
+              if (FP && x[q] < MID) hn = max(hn, x[q]);
+              if (FP && x[q] >= MID) lp = min(lp, x[q]);
+            }
+        }
+        lo = warp_min(lo);
+        hi = warp_max(hi);
+        hn = warp_max(hn);
+        lp = warp_min(lp);
+        if (!FP || lo >= MID || hi < MID) hn = lp = hi;
+        for (uint32_t b = lane; b < RW_BINS; b += 32u) sm.h[b] = 0u;
+        __syncwarp();
+        const K range = (K)((hn - lo) + (hi - lp));
+        const uint32_t sh = (uint32_t)max(0, bitlen(range) - RW_BITS);
+        static_assert(RW_BINS == 1u << RW_BITS, "two keys a bin");
+        auto bin = [&](K k) -> uint32_t {
+          return FP ? (uint32_t)((K)((min(k, hn) - lo) + (max(k, lp) - lp)) >> sh) : (uint32_t)((K)(k - lo) >> sh);
+        };
+        for (uint32_t i = lane; i < cnt; i += 32u) atomicAdd(&sm.h[bin(sm.v[i])], 1u);
+        __syncwarp();
+        uint32_t run = 0, mx = 0;
+        for (uint32_t b0 = 0; b0 < RW_BINS; b0 += 32u) {
+          const uint32_t x = sm.h[b0 + lane];
+          mx = max(mx, x);
+          const uint32_t inc = warp_incl_scan_u32(x, lane);
+          sm.h[b0 + lane] = run + inc - x;
+          run += __shfl_sync(FULL, inc, 31);
+        }
+        __syncwarp();
+        for (uint32_t i = lane; i < cnt; i += 32u) {
+          const K k = sm.v[i];
+          sm.w[atomicAdd(&sm.h[bin(k)], 1u)] = k;
+        }
+        __syncwarp();
+        // h[b] is now the end of bin b.  One lane per bin: insertion sort; a
+        // bin of over 32 keys is fine when they are all equal
+        bool unsorted = false;
+        for (uint32_t b = lane; b < RW_BINS; b += 32u) {
+          const uint32_t e = sm.h[b], s0 = b ? sm.h[b - 1u] : 0u;
+          if (e - s0 > 32u) {
+            const K x = sm.w[s0];
+            for (uint32_t i = s0 + 1u; i < e && !unsorted; ++i) unsorted = sm.w[i] != x;
+            continue;
+          }
+          for (uint32_t i = s0 + 1u; i < e; ++i) {
+            const K x = sm.w[i];
+            uint32_t p = i;
+            for (; p > s0 && sm.w[p - 1u] > x; --p) sm.w[p] = sm.w[p - 1u];
+            sm.w[p] = x;
+          }
+        }
+        __syncwarp();
+        if (__any_sync(FULL, unsorted)) {
+          uint32_t N = 64;
+          while (N < cnt) N <<= 1;
+          for (uint32_t i = cnt + lane; i < N; i += 32u) sm.w[i] = key_max<K>();
+          __syncwarp();
+          for (uint32_t kk = 2; kk <= N; kk <<= 1)
+            for (uint32_t jj = kk >> 1; jj > 0; jj >>= 1) {
+              for (uint32_t t = lane; t < N / 2; t += 32u) {  // pair t: i has bit jj clear
+                const uint32_t i = ((t & ~(jj - 1u)) << 1) | (t & (jj - 1u));
+                const K x = sm.w[i], y = sm.w[i | jj];
+                if ((x > y) == ((i & kk) == 0)) { sm.w[i] = y; sm.w[i | jj] = x; }
+              }
+              __syncwarp();
+            }
+        }
+      }
+      for (uint32_t i = lane; i < nk; i += 32u) {
+        const uint32_t k = a.ks[k0 + i];
+        if (k >= 1u && k <= cnt) a.r.kkey[k0 + i] = sorted[cnt - k];
+        else set_status(C, GGMS_E_INVALID_ARG);
+      }
+      __syncwarp();
+    }
+  }
+}
+
+GGMS_END

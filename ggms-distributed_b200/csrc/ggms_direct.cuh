@@ -69,6 +69,7 @@ int launch_direct(Context* ctx, const DirectArgs<T>& a, unsigned ctas, cudaStrea
 GGMS_BEGIN
 
 constexpr int DR_NT = 1024;
+
 constexpr uint32_t K_SORTED = 0xFFFFFFFEu;   // k_seg value: the answer is at cand[k_rank] once that is sorted
 
 // Monotone map key -> bucket: keys are clamped to the sample's range; cell c
@@ -141,7 +142,8 @@ __device__ __forceinline__ void block_scan_regs(uint32_t (&v)[V], uint32_t* red)
   if (lane == 31) red[warp] = inc;
   __syncthreads();
   const uint32_t w = warp_incl_scan_u32(red[lane], lane);  // every warp scans the warp totals
-  const uint32_t before = inc - v[V - 1] + (warp ? __shfl_sync(FULL, w, warp - 1) : 0u);
+  const uint32_t prev = __shfl_sync(FULL, w, (warp + 31u) & 31u);
+  const uint32_t before = inc - v[V - 1] + (warp ? prev : 0u);
 #pragma unroll
   for (int i = 0; i < V; ++i) v[i] += before;
   __syncthreads();
@@ -154,10 +156,14 @@ __host__ __device__ constexpr uint32_t pz(uint32_t b) { return b + (b >> 5); }
 
 // Global counts [B] into their inclusive scan in shared memory: 16-byte loads,
 // all of a thread's in flight together, and one scan in registers.
+// (One CTA, g null: its own counts own[B].)
 template <int V>
-__device__ __forceinline__ void scan_counts(const uint32_t* g, uint32_t* I, uint32_t* red) {
+__device__ __forceinline__ void scan_counts(const uint32_t* g, const uint32_t* own, uint32_t* I, uint32_t* red) {
   uint32_t v[V];
-  if constexpr (V >= 4) {
+  if (!g) {
+#pragma unroll
+    for (int i = 0; i < V; ++i) v[i] = own[threadIdx.x * V + i];
+  } else if constexpr (V >= 4) {
 #pragma unroll
     for (int i = 0; i < V; i += 4) {
       const uint4 q = __ldcg(reinterpret_cast<const uint4*>(g + threadIdx.x * V + i));
@@ -309,7 +315,7 @@ __device__ K* cta_radix(SortSmem<K>& sm, K* A, K* Bf, uint32_t m, int sh0, int s
 // ranges; CTA 0 also takes the unaligned head and the tail.
 template <typename T, typename F>
 __device__ __forceinline__ void direct_stream(const T* in, uint64_t n, uint32_t cta, uint32_t ncta, F&& f) {
-  constexpr int EPV = Vec16<T>::N, U = 4;
+  constexpr int EPV = Vec16<T>::N, U = 2;
   const uint32_t tid = threadIdx.x;
   uint64_t head = ((16u - (uint32_t)((uintptr_t)in & 15u)) & 15u) / sizeof(T);
   if (head > n) head = n;
@@ -450,36 +456,61 @@ __global__ __launch_bounds__(DR_NT, 1) void direct_sort(const __grid_constant__ 
   }
 }
 
+// One vector for direct_body: its share of the grid, its workspace, its ks.
 template <typename T>
-__global__ __launch_bounds__(DR_NT, 1) void direct_select(const __grid_constant__ DirectArgs<T> a) {
+struct DirectTask {
+  using K = typename KeyOf<T>::K;
+  const T* in;
+  uint64_t n;
+  const uint32_t* ks;          // null: top-k
+  uint32_t nk;
+  uint64_t seed;
+  uint32_t B, focus, slices;
+  uint32_t *ghist, *gcur, *gact;  // [B], [B], [B / 32 + 1]; one CTA: unused
+  uint32_t* bar;               // the barrier word of the vector's CTAs
+  uint32_t cta, ncta;          // this CTA among them
+  uint64_t off;                // the vector's n candidates: r.cand[0] + off
+  uint64_t k0;                 // its ks in the per-k arrays: k0 ..
+};
+
+// Steps 1 to 5 for one vector.  On return its ks are resolved but for those in
+// large children, which are in pool 1 for the refinement levels, with their
+// true key ranges.  False after a barrier that ran out.  ONE: a single CTA's
+// vector (a.cta == 0, a.ncta == 1).
+template <typename T, bool ONE>
+__device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const RefineArgs<T>& r, uint8_t* smem) {
   using K = typename KeyOf<T>::K;
   constexpr bool FP = std::is_floating_point<T>::value, K64 = sizeof(K) == 8;
   constexpr uint32_t NONE = 0xFFFFFFFFu;
-  extern __shared__ __align__(128) uint8_t smem[];
   DirectSmem<K>& sm = *reinterpret_cast<DirectSmem<K>*>(smem);
   __shared__ K red_k[4][DR_NT / 32];
   __shared__ uint32_t red[72];
-  const RefineArgs<T>& r = a.r;
-  Counters* C = r.C;
-  const uint32_t cta = blockIdx.x, ncta = gridDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t cta = ONE ? 0u : a.cta, ncta = ONE ? 1u : a.ncta;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t gt = cta * DR_NT + tid, gs = ncta * DR_NT;
-  const uint32_t B = a.B, nk = r.nk;
+  const uint32_t B = a.B, nk = a.nk;
+  // the per-k arrays and the candidates, addressed where they are used: held
+  // from here on they would take ten registers through both streams
+  auto kbin = [&](uint32_t i) -> uint32_t& { return r.kbin[a.k0 + i]; };
+  auto krank = [&](uint32_t i) -> uint32_t& { return r.krank[a.k0 + i]; };
+  auto kseg = [&](uint32_t i) -> uint32_t& { return r.kseg[a.k0 + i]; };
+  auto kkey = [&](uint32_t i) -> K& { return r.kkey[a.k0 + i]; };
 
   GGMS_TRACE(0);
-  // ---- the call's counters, the global histogram
-  for (uint32_t i = gt; i < B; i += gs) {
-    a.ghist[i] = 0u;
-    a.gcur[i] = 0u;
-    if (i < B / 32) a.gact[i] = 0u;
-  }
-  if (cta == 0 && tid < sizeof(Counters) / 4) reinterpret_cast<uint32_t*>(C)[tid] = 0u;
+  // ---- the global histogram
+  if (ncta > 1u)
+    for (uint32_t i = gt; i < B; i += gs) {
+      a.ghist[i] = 0u;
+      a.gcur[i] = 0u;
+      if (i <= B / 32) a.gact[i] = 0u;
+    }
   // the ranks, staged in device memory (ks may be pinned host memory: each is read once)
   for (uint32_t i = gt; i < nk; i += gs) {
     const uint32_t k = a.ks ? a.ks[i] : i + 1u;
-    r.kbin[i] = k >= 1u && (uint64_t)k <= a.n ? (uint32_t)(a.n - k) : NONE;  // a rank is at most n - 1 < NONE
+    kbin(i) = k >= 1u && (uint64_t)k <= a.n ? (uint32_t)(a.n - k) : NONE;  // a rank is at most n - 1 < NONE
   }
   GridBarrier zeroed;
-  zeroed.arrive(r.bar, ncta);
+  zeroed.arrive(a.bar, ncta, cta == 0u);
 
   // ---- the map, from a sample every CTA draws for itself
   const uint32_t S = (uint32_t)min(a.n, (uint64_t)DIRECT_SAMPLE);
@@ -523,9 +554,12 @@ __global__ __launch_bounds__(DR_NT, 1) void direct_select(const __grid_constant_
   __syncthreads();
   lo = warp_min(red_k[0][lane]);
   hi = warp_max(red_k[1][lane]);
+  // (every lane takes part in every reduction: as arms of the selects below
+  // they gave the wrong arm in one kernel)
+  const K hn_all = warp_max(red_k[2][lane]), lp_all = warp_min(red_k[3][lane]);
   const bool two = FP && lo < MID && hi >= MID;
-  hn = two ? warp_max(red_k[2][lane]) : hi;
-  lp = two ? warp_min(red_k[3][lane]) : hi;
+  hn = two ? hn_all : hi;
+  lp = two ? lp_all : hi;
   // 64-bit keys: the high word alone when it resolves the sample
   const bool hi32 = K64 && (K)((hi - lo) - (two ? lp - hn : (K)0)) >> (K64 ? 32 : 0) >= (K)(1u << 16);
   auto dom = [&](K k) -> K { return hi32 ? (K)(k >> (K64 ? 32 : 0)) : k; };
@@ -565,11 +599,11 @@ __global__ __launch_bounds__(DR_NT, 1) void direct_select(const __grid_constant_
   uint32_t nfirst = w2[0] - own0;  // packed prefix before this thread's cells: hot | other << 16
   bool focus = false;
   if (a.focus) {
-    if (!zeroed.wait(r.bar, ncta, C)) return;
+    if (!zeroed.wait(a.bar, ncta, r.C)) return false;
     // clustered ks: their ranks occupy at most a quarter of 64 equal ranges
     unsigned long long occ = 0;
     for (uint32_t i = tid; i < nk; i += DR_NT) {
-      const uint32_t rank = __ldcg(&r.kbin[i]);
+      const uint32_t rank = __ldcg(&kbin(i));
       if (rank != NONE) occ |= 1ull << (uint32_t)(((uint64_t)rank * 64u) / a.n);
     }
     const uint32_t o0 = __reduce_or_sync(FULL, (uint32_t)occ), o1 = __reduce_or_sync(FULL, (uint32_t)(occ >> 32));
@@ -589,7 +623,7 @@ __global__ __launch_bounds__(DR_NT, 1) void direct_select(const __grid_constant_
     // m = z sqrt(S q (1 - q)) + z + 2 of S q (z = 6).  Cells of those positions,
     // as a difference array; a k outside them costs time, never exactness.
     for (uint32_t i = tid; i < nk; i += DR_NT) {
-      const uint32_t rank = __ldcg(&r.kbin[i]);
+      const uint32_t rank = __ldcg(&kbin(i));
       if (rank == NONE) continue;
       const float q = ((float)rank + 0.5f) / (float)a.n;
       const float pos = q * (float)S, m = 6.0f * sqrtf((float)S * q * fmaxf(1.0f - q, 0.0f)) + 8.0f;
@@ -664,13 +698,13 @@ __global__ __launch_bounds__(DR_NT, 1) void direct_select(const __grid_constant_
   });
   GGMS_TRACE(2);
   if (a.focus) __syncthreads();
-  else if (!zeroed.wait(r.bar, ncta, C)) return;  // (a CTA barrier too)
+  else if (!zeroed.wait(a.bar, ncta, r.C)) return false;  // (a CTA barrier too)
   if (ncta > 1u)
     for (uint32_t i = tid; i < B; i += DR_NT) {
       const uint32_t v = sm.hist[i];
       if (v) atomicAdd(&a.ghist[i], v);
     }
-  if (!grid_barrier(r.bar, ncta, C)) return;
+  if (!grid_barrier(a.bar, ncta, cta == 0u, r.C)) return false;
 
   GGMS_TRACE(3);
   // ---- scan, locate
@@ -678,17 +712,13 @@ __global__ __launch_bounds__(DR_NT, 1) void direct_select(const __grid_constant_
     sm.act[w] = 0u;
     sm.big[w] = 0u;
   }
-  if (ncta == 1u) {
-    // one CTA: its own counts (few buckets: the vector is short)
-    for (uint32_t i = tid; i < B; i += DR_NT) a.ghist[i] = sm.hist[i];
-    __syncthreads();
-  }
+  const uint32_t* counts = ncta > 1u ? a.ghist : nullptr;
   switch (B / DR_NT) {
-    case 1: scan_counts<1>(a.ghist, sm.I, red); break;
-    case 2: scan_counts<2>(a.ghist, sm.I, red); break;
-    case 4: scan_counts<4>(a.ghist, sm.I, red); break;
-    case 8: scan_counts<8>(a.ghist, sm.I, red); break;
-    default: scan_counts<16>(a.ghist, sm.I, red); break;
+    case 1: scan_counts<1>(counts, sm.hist, sm.I, red); break;
+    case 2: scan_counts<2>(counts, sm.hist, sm.I, red); break;
+    case 4: scan_counts<4>(counts, sm.hist, sm.I, red); break;
+    case 8: scan_counts<8>(counts, sm.hist, sm.I, red); break;
+    default: scan_counts<16>(counts, sm.hist, sm.I, red); break;
   }
   static_assert(DIRECT_MAX_B == 16 * DR_NT, "the largest scan above");
   auto bucket_of = [&](uint32_t rank) {  // the smallest b with I[b] > rank
@@ -701,19 +731,19 @@ __global__ __launch_bounds__(DR_NT, 1) void direct_select(const __grid_constant_
   };
   if (!a.slices) {  // every CTA locates every k
     for (uint32_t i = tid; i < nk; i += DR_NT) {
-      const uint32_t rank = __ldcg(&r.kbin[i]);
+      const uint32_t rank = __ldcg(&kbin(i));
       if (rank == NONE) continue;
       const uint32_t b = bucket_of(rank);
       atomicOr(&sm.act[b >> 5], 1u << (b & 31));
     }
   } else {  // many ks: every CTA locates its own, and they meet
     for (uint32_t i = gt; i < nk; i += gs) {
-      const uint32_t rank = r.kbin[i];
+      const uint32_t rank = kbin(i);
       if (rank == NONE) continue;
       const uint32_t b = bucket_of(rank);
       atomicOr(&a.gact[b >> 5], 1u << (b & 31));
     }
-    if (!grid_barrier(r.bar, ncta, C)) return;
+    if (!grid_barrier(a.bar, ncta, cta == 0u, r.C)) return false;
     for (uint32_t w = tid; w < B / 32; w += DR_NT) sm.act[w] = __ldcg(&a.gact[w]);
   }
   __syncthreads();
@@ -741,20 +771,6 @@ __global__ __launch_bounds__(DR_NT, 1) void direct_select(const __grid_constant_
   auto is_big = [&](uint32_t b) { return (sm.big[b >> 5] >> (b & 31)) & 1u; };
   auto big_of = [&](uint32_t b) { return sm.bpre[b >> 5] + __popc(sm.big[b >> 5] & ((1u << (b & 31)) - 1u)); };
   GGMS_TRACE(4);
-  // this CTA's slice of the ks
-  for (uint32_t i = gt; i < nk; i += gs) {
-    const uint32_t rank = __ldcg(&r.kbin[i]);
-    if (rank == NONE) {
-      set_status(C, GGMS_E_INVALID_ARG);
-      r.kseg[i] = K_DONE;
-      r.kkey[i] = 0;
-      continue;
-    }
-    const uint32_t b = bucket_of(rank), in = rank - (b ? sm.I[pz(b - 1)] : 0u);
-    const bool lg = is_big(b);
-    r.krank[i] = lg ? in : (b ? sm.J[pz(b - 1)] : 0u) + in;
-    r.kseg[i] = lg ? big_of(b) : K_SORTED;
-  }
   for (uint32_t b0 = tid; b0 < B; b0 += 8u * DR_NT) {
     // this CTA's range of every child it holds keys of: one reservation each,
     // eight in flight per thread
@@ -771,11 +787,54 @@ __global__ __launch_bounds__(DR_NT, 1) void direct_select(const __grid_constant_
       if (b >= B || !active(b)) continue;
       const uint32_t off = b ? sm.J[pz(b - 1)] : 0u;
       sm.hist[b] = off + base[u];
+    }
+  }
+  // ids of the large children: a range of the list of all vectors'
+  if (cta == 0 && tid == 0 && nbig) {
+    atomicAdd(&r.C->nsegs[1], nbig);
+    const uint32_t first = atomicAdd(&r.C->nbig[1], nbig);
+    if (ncta > 1u) a.gact[B / 32] = first;
+    red[69] = first;
+  }
+  __syncthreads();
+
+  GGMS_TRACE(5);
+  // ---- copy
+  with_map([&](const auto& m) {
+    K* cand = r.cand[0] + a.off;
+    direct_stream<T>(a.in, a.n, cta, ncta, [&](K key) {
+      const uint32_t b = m(key);
+      if (active(b)) cand[atomicAdd(&sm.hist[b], 1u)] = key;
+    });
+  });
+  GGMS_TRACE(6);
+  if (!grid_barrier(a.bar, ncta, cta == 0u, r.C)) return false;
+  GGMS_TRACE(7);
+  GGMS_TRACE_CTA(0);
+
+  // ---- this CTA's slice of the ks and of the large children
+  const uint32_t first_big = !nbig ? 0u : ncta > 1u ? __ldcg(&a.gact[B / 32]) : red[69];
+  for (uint32_t i = gt; i < nk; i += gs) {
+    const uint32_t rank = __ldcg(&kbin(i));
+    if (rank == NONE) {
+      set_status(r.C, GGMS_E_INVALID_ARG);
+      kseg(i) = K_DONE;
+      kkey(i) = 0;
+      continue;
+    }
+    const uint32_t b = bucket_of(rank), in = rank - (b ? sm.I[pz(b - 1)] : 0u);
+    const bool lg = is_big(b);
+    krank(i) = lg ? in : (b ? sm.J[pz(b - 1)] : 0u) + in;
+    kseg(i) = lg ? first_big + big_of(b) : K_SORTED;
+  }
+  if (nbig)
+    for (uint32_t b = tid; b < B; b += DR_NT) {
       if (!is_big(b)) continue;
-      const uint32_t id = big_of(b);
-      if (id % ncta != cta) continue;
+      const uint32_t at = big_of(b), id = first_big + at;
+      if (at % ncta != cta) continue;
+      const uint32_t off = b ? sm.J[pz(b - 1)] : 0u;
       Seg<K> sg;  // refined by levels, from its true key range (below)
-      sg.off = off;
+      sg.off = a.off + off;
       sg.cnt = sm.J[pz(b)] - off;
       sg.shift = 0u;
       sg.lo = key_max<K>();
@@ -783,9 +842,9 @@ __global__ __launch_bounds__(DR_NT, 1) void direct_select(const __grid_constant_
       sg.row = id;
       sg.pad = 0u;
       const uint32_t nt = (sg.cnt + TILE - 1) / TILE;
-      const uint32_t t0 = atomicAdd(&C->ntiles[1], nt);
-      if (id >= r.caps.rows || t0 + nt > r.caps.tiles) {  // cannot happen: the caps bound both
-        set_status(C, GGMS_E_INTERNAL);
+      const uint32_t t0 = atomicAdd(&r.C->ntiles[1], nt);
+      if (id >= r.caps.rows || id >= r.caps.segs || t0 + nt > r.caps.tiles) {  // cannot happen: the caps bound them
+        set_status(r.C, GGMS_E_INTERNAL);
         continue;
       }
       r.bigs[1][id] = id;
@@ -793,26 +852,6 @@ __global__ __launch_bounds__(DR_NT, 1) void direct_select(const __grid_constant_
       r.cursor[1][id] = 0u;
       for (uint32_t t = 0; t < nt; ++t) r.tiles[1][t0 + t] = TileRef{id, t};
     }
-  }
-  if (cta == 0 && tid == 0) {
-    C->nsegs[1] = nbig;
-    C->nbig[1] = min(nbig, r.caps.rows);
-  }
-  __syncthreads();
-
-  GGMS_TRACE(5);
-  // ---- copy
-  K* cand = r.cand[0];
-  with_map([&](const auto& m) {
-    direct_stream<T>(a.in, a.n, cta, ncta, [&](K key) {
-      const uint32_t b = m(key);
-      if (active(b)) cand[atomicAdd(&sm.hist[b], 1u)] = key;
-    });
-  });
-  GGMS_TRACE(6);
-  if (!grid_barrier(r.bar, ncta, C)) return;
-  GGMS_TRACE(7);
-  GGMS_TRACE_CTA(0);
 
   // ---- sort: whole children whose keys start in this CTA's part of the candidates
   auto boundary = [&](uint32_t x) -> uint32_t {  // the first child boundary at or after position x
@@ -836,7 +875,7 @@ __global__ __launch_bounds__(DR_NT, 1) void direct_select(const __grid_constant_
   for (uint32_t x = boundary((uint32_t)((uint64_t)total * cta / ncta)); x < x_end;) {
     const uint32_t y = min(x_end, last_boundary(x + CAP < x ? total : x + CAP));
     if (y > x) {
-      K* c = cand + x;
+      K* c = r.cand[0] + a.off + x;
       sort_keys<K>(sm.sort, y - x, red_k, [&](uint32_t i) { return c[i]; }, [&](uint32_t i, K key) { c[i] = key; });
       x = y;
     } else {  // a large child: the levels refine it
@@ -845,46 +884,74 @@ __global__ __launch_bounds__(DR_NT, 1) void direct_select(const __grid_constant_
   }
   GGMS_TRACE(8);
   GGMS_TRACE_CTA(1);
-  // ks of the sorted children (the barrier before makes every child's order
-  // visible; levels beyond the first reuse these buffers)
-  auto from_sorted = [&]() {
-    for (uint32_t i = gt; i < nk; i += gs) {
-      if (r.kseg[i] != K_SORTED) continue;
-      r.kkey[i] = cand[r.krank[i]];
-      r.kseg[i] = K_DONE;
-    }
-  };
-  if (nbig) {  // the same for every CTA
-    const uint32_t nt = min(C->ntiles[1], r.caps.tiles);
-    for (uint32_t t = cta; t < nt; t += ncta) {  // the true key range of the large children
-      const TileRef tr = r.tiles[1][t];
-      Seg<K>& s = r.segs[1][tr.seg];
-      const uint64_t beg = s.off + (uint64_t)tr.no * TILE, end = min(beg + TILE, s.off + s.cnt);
+  if (!grid_barrier(a.bar, ncta, cta == 0u, r.C)) return false;
+  GGMS_TRACE(9);
+  // ks of the sorted children (the barrier makes every child's order visible)
+  for (uint32_t i = gt; i < nk; i += gs) {
+    if (kseg(i) != K_SORTED) continue;
+    kkey(i) = r.cand[0][a.off + krank(i)];
+    kseg(i) = K_DONE;
+  }
+  if (!nbig) return true;
+  // the true key range of the large children: their tiles dealt to the CTAs
+  uint32_t dealt = 0;
+  for (uint32_t w = 0; w < B / 32; ++w)
+    for (uint32_t m = sm.big[w]; m; m &= m - 1u) {
+      const uint32_t b = w * 32u + __ffs(m) - 1u, id = first_big + big_of(b);
+      if (id >= r.caps.rows || id >= r.caps.segs) continue;
+      const uint32_t off = b ? sm.J[pz(b - 1)] : 0u, cnt = sm.J[pz(b)] - off;
+      const uint32_t nt = (cnt + TILE - 1) / TILE;
       K mn = key_max<K>(), mx = 0;
-      for (uint64_t i = beg + tid; i < end; i += DR_NT) {
-        mn = min(mn, cand[i]);
-        mx = max(mx, cand[i]);
-      }
+      for (uint32_t t = (cta + ncta - dealt % ncta) % ncta; t < nt; t += ncta)
+        for (uint32_t i = t * TILE + tid; i < min(cnt, (t + 1u) * TILE); i += DR_NT) {
+          const K x = r.cand[0][a.off + off + i];
+          mn = min(mn, x);
+          mx = max(mx, x);
+        }
+      dealt += nt;
       mn = warp_min(mn);
       mx = warp_max(mx);
       if (lane == 0 && mn <= mx) {
-        key_atomic_min(&s.lo, mn);
-        key_atomic_max(&s.hi, mx);
+        key_atomic_min(&r.segs[1][id].lo, mn);
+        key_atomic_max(&r.segs[1][id].hi, mx);
       }
     }
-    if (!grid_barrier(r.bar, ncta, C)) return;
-    from_sorted();
-    for (uint32_t j = gt; j < min(C->nbig[1], r.caps.rows); j += gs) {
-      Seg<K>& s = r.segs[1][r.bigs[1][j]];
-      s.shift = (uint32_t)max(0, bitlen((K)(__ldcg(&s.hi) - __ldcg(&s.lo))) - RADIX_BITS);
-    }
-    // (refine_body's first barrier orders the shifts before the count)
-    if (!refine_body<T, DR_NT>(r, smem)) return;
+  if (!grid_barrier(a.bar, ncta, cta == 0u, r.C)) return false;
+  for (uint32_t j = first_big + gt; j < min(first_big + nbig, min(r.caps.rows, r.caps.segs)); j += gs) {
+    Seg<K>& s = r.segs[1][j];
+    s.shift = (uint32_t)max(0, bitlen((K)(__ldcg(&s.hi) - __ldcg(&s.lo))) - RADIX_BITS);
   }
-  if (!grid_barrier(r.bar, ncta, C)) return;
-  GGMS_TRACE(9);
-  from_sorted();
-  write_out_body<T>(r.kkey, r.kseg, nk, r.out, C, cta, ncta);
+  return true;
+}
+
+template <typename T>
+__global__ __launch_bounds__(DR_NT, 1) void direct_select(const __grid_constant__ DirectArgs<T> a) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  const RefineArgs<T>& r = a.r;
+  Counters* C = r.C;
+  const uint32_t cta = blockIdx.x, ncta = gridDim.x;
+  // the call's counters (other CTAs touch them only after the body's first barrier)
+  if (cta == 0 && threadIdx.x < sizeof(Counters) / 4) reinterpret_cast<uint32_t*>(C)[threadIdx.x] = 0u;
+  DirectTask<T> t;
+  t.in = a.in;
+  t.n = a.n;
+  t.ks = a.ks;
+  t.nk = r.nk;
+  t.seed = a.seed;
+  t.B = a.B;
+  t.focus = a.focus;
+  t.slices = a.slices;
+  t.ghist = a.ghist;
+  t.gcur = a.gcur;
+  t.gact = a.gact;
+  t.bar = r.bar;
+  t.cta = cta;
+  t.ncta = ncta;
+  t.off = 0;
+  t.k0 = 0;
+  if (!direct_body<T, false>(t, r, smem)) return;
+  if (__ldcg(&C->nbig[1]) && (!refine_body<T, DR_NT>(r, smem) || !grid_barrier(r.bar, ncta, cta == 0u, C))) return;
+  write_out_body<T>(r.kkey, r.kseg, r.nk, r.out, C, cta, ncta);
   report_body(C, r.report, ncta);
   GGMS_TRACE(10);
 }

@@ -17,6 +17,7 @@
 #include "ggms_kernels.cuh"
 #include "ggms_refine.cuh"
 #include "ggms_direct.cuh"
+#include "ggms_batch.cuh"
 #include "ggms_learned.cuh"
 #include "ggms_window.cuh"
 
@@ -52,9 +53,9 @@ struct Workspace {
   uint32_t* knext;        // per k: next k in its segment's list
   uint32_t* smalls;       // ids of the small segments the current level created
   uint32_t* tinies;       // ids of the tiny segments the current level created
-  uint32_t* bigs[2];      // per pool: the segments a level refines, by row (batched level 0: quantile ones)
-  K* qtab;                // ... their boundaries [cap_q][QB]
-  uint16_t* qdir;         // ... their directories [cap_q][QDS]
+  uint32_t* bigs[2];      // per pool: the segments a level refines, by row
+  uint32_t* lists;        // batched path: segments by class [BT_CLASSES][nlist]
+  uint32_t* scratch;      // ... per CTA: a team's global histogram and cursors
   K* points;
   K* cand[2];
   size_t bytes;
@@ -67,7 +68,7 @@ static Workspace<K> layout(const Plan& p, uint8_t* base) {
   Workspace<K> w;
   static_assert(sizeof(Counters) <= ARENA_BAR, "the barrier word follows the counters");
   size_t o_C = b.take(sizeof(Counters));
-  b.take(256);  // ARENA_BAR
+  b.take(ARENA_BAR_BYTES);
   size_t o_kin = b.take(4ull * p.nk);
   size_t o_krank = b.take(4ull * p.nk);
   size_t o_kseg = b.take(4ull * p.nk);
@@ -91,8 +92,8 @@ static Workspace<K> layout(const Plan& p, uint8_t* base) {
   size_t o_tinies = b.take(4ull * p.cap_seg);
   size_t o_bigs[2];
   for (int i = 0; i < 2; ++i) o_bigs[i] = b.take(4ull * p.cap_rows);
-  size_t o_qtab = b.take(sizeof(K) * QB * p.cap_q);
-  size_t o_qdir = b.take(2ull * QDS * p.cap_q);
+  size_t o_lists = b.take(4ull * BT_CLASSES * p.nlist);
+  size_t o_scratch = b.take(p.nlist ? 4ull * BT_SCRATCH * p.sms : 0);
   for (int i = 0; i < 2; ++i) {
     o_kh[i] = b.take(4ull * p.cap_seg);
     o_segs[i] = b.take(sizeof(Seg<K>) * p.cap_seg);
@@ -137,8 +138,8 @@ static Workspace<K> layout(const Plan& p, uint8_t* base) {
   w.smalls = (uint32_t*)(base + o_smalls);
   w.tinies = (uint32_t*)(base + o_tinies);
   for (int i = 0; i < 2; ++i) w.bigs[i] = (uint32_t*)(base + o_bigs[i]);
-  w.qtab = (K*)(base + o_qtab);
-  w.qdir = (uint16_t*)(base + o_qdir);
+  w.lists = (uint32_t*)(base + o_lists);
+  w.scratch = (uint32_t*)(base + o_scratch);
   w.points = (K*)(base + o_pts);
   return w;
 }
@@ -179,7 +180,6 @@ static RefineArgs<T> refine_args(const Workspace<typename KeyOf<T>::K>& w, const
 }
 
 // ------------------------------------------------------------------ kernel configs
-constexpr int LV_NT = 256;
 
 template <typename T>
 static size_t l0_count_smem(uint32_t B, int nt, int unroll, uint32_t nst) {
@@ -301,8 +301,7 @@ constexpr int SS_NT = 512;
 
 template <typename InT, typename K = typename KeyOf<InT>::K>
 static int launch_small_select(Context* ctx, const InT* src, const Seg<K>* segs_q, const uint32_t* khead_q,
-                               const Workspace<K>& w, const Caps& caps, cudaStream_t st,
-                               const int64_t* k_off = nullptr) {
+                               const Workspace<K>& w, const Caps& caps, cudaStream_t st) {
   static bool attr = false;
   const size_t sm = SMALL_SELECT_SMEM;
   if (!attr) {
@@ -312,13 +311,13 @@ static int launch_small_select(Context* ctx, const InT* src, const Seg<K>* segs_
   }
   ++ctx->launches;
   GGMS_CU(launch_pdl(small_select<InT, SS_NT>, ctx->sms * 2, SS_NT, sm, st, src, segs_q, w.smalls, w.C, khead_q,
-                     w.knext, k_off, w.krank, w.kseg, w.kkey, caps.small_keys, caps));
+                     w.knext, w.krank, w.kseg, w.kkey, caps.small_keys, caps));
   // the warp finisher (its own list of segments) runs beside the CTA finisher:
   // it does not wait for it before its work (tiny_select)
   if (caps.tiny_keys) {
     ++ctx->launches;
     GGMS_CU(launch_pdl(tiny_select<InT, TS_NT>, ctx->sms * 8, TS_NT, 0, st, src, segs_q, w.tinies, w.C, khead_q,
-                       w.knext, k_off, w.krank, w.kseg, w.kkey, caps));
+                       w.knext, w.krank, w.kseg, w.kkey, caps));
   }
   return GGMS_OK;
 }
@@ -401,7 +400,7 @@ static int sort_cluster_ctas(uint32_t S) {
 //     the copied keys of a long one (2^24, 1000 ks) and cost a short one 2 us.
 //   focus (most buckets to clustered ks): costs 3 us of the map, saves 25 of
 //     the copy and sort at 2^22 and 100 at 2^24 with 1000 ks in the top 1 %.
-constexpr uint64_t DIRECT_MAX_BYTES = 128ull << 20;
+constexpr uint64_t DIRECT_MAX_BYTES = 160ull << 20;
 constexpr uint32_t DIRECT_MAX_KS = 65536;
 constexpr uint64_t DIRECT_CTA_KEYS = 1024;    // keys that repay another CTA
 constexpr uint64_t DIRECT_BUCKET_KEYS = 8;
@@ -731,7 +730,7 @@ static int run_single_tuned(Context* c, const T* d_in, uint64_t n, const uint32_
   static const int Bs[] = {4096, 8192, 16384};
   static const int shapes[][2] = {{1024, 4}, {1024, -2}, {512, 4}, {512, 8}};
   float best = 3.4e38f;
-  Context::Tuned pick{{key[0], key[1], key[2], key[3]}, 8192, DEFAULT_PASS_NT, DEFAULT_PASS_UNROLL, 8};
+  Context::Tuned pick{{key[0], key[1], key[2], key[3]}, 8192, DEFAULT_PASS_NT, DEFAULT_PASS_UNROLL};
   for (int B : Bs) {
     for (const auto& sh : shapes) {
       ggms_opts t = b;
@@ -800,29 +799,31 @@ static int ex(ggms_context* cx, const T* d_in, int64_t n, const uint32_t* ks, in
 
 
 // ------------------------------------------------------------------ batched segmented path
-// Every caller segment that holds a k: small ones are finished straight from
-// the input (one warp or one CTA each); the others get sample-quantile bins at
-// level 0, and the children of those bins go through radix levels (or
-// straight to the warp / CTA finishers) -- every level runs over all segments
-// at once.
+// Every segment by its length: a team of CTAs, one CTA or one warp
+// (ggms_batch.cuh); the children that are still large go through the refinement
+// levels, all segments' at once.
 template <typename T>
 static int run_segmented(Context* ctx, const T* d_in, const int64_t* seg_off, int64_t nseg64,
                          const uint32_t* ks, const int64_t* k_off, T* out, const ggms_opts& o,
-                         cudaStream_t st, int lv_mult = 8) {
+                         cudaStream_t st) {
   using K = typename KeyOf<T>::K;
   if (!d_in || !seg_off || !k_off || nseg64 <= 0 || nseg64 > (1 << 30)) return GGMS_E_INVALID_ARG;
   if ((uintptr_t)d_in % sizeof(T) != 0) return GGMS_E_INVALID_ARG;
   const uint32_t nseg = (uint32_t)nseg64;
-  int64_t h_tot[2], h_k[2];
   GGMS_CU(cudaSetDevice(ctx->device));
-  GGMS_CU(cudaMemcpyAsync(&h_tot[0], seg_off, 8, cudaMemcpyDeviceToHost, st));
-  GGMS_CU(cudaMemcpyAsync(&h_tot[1], seg_off + nseg, 8, cudaMemcpyDeviceToHost, st));
-  GGMS_CU(cudaMemcpyAsync(&h_k[0], k_off, 8, cudaMemcpyDeviceToHost, st));
-  GGMS_CU(cudaMemcpyAsync(&h_k[1], k_off + nseg, 8, cudaMemcpyDeviceToHost, st));
+  // the totals size the workspace: four words to pinned memory, one sync
+  int rc = ensure_pinned(ctx, 64);
+  if (rc) return rc;
+  if (ctx->pin_busy) GGMS_CU(cudaEventSynchronize(ctx->pin_busy));
+  int64_t* h = (int64_t*)ctx->pinned;
+  GGMS_CU(cudaMemcpyAsync(&h[0], seg_off, 8, cudaMemcpyDeviceToHost, st));
+  GGMS_CU(cudaMemcpyAsync(&h[1], seg_off + nseg, 8, cudaMemcpyDeviceToHost, st));
+  GGMS_CU(cudaMemcpyAsync(&h[2], k_off, 8, cudaMemcpyDeviceToHost, st));
+  GGMS_CU(cudaMemcpyAsync(&h[3], k_off + nseg, 8, cudaMemcpyDeviceToHost, st));
   GGMS_CU(cudaStreamSynchronize(st));
-  if (h_tot[0] != 0 || h_k[0] != 0 || h_tot[1] < 0 || h_k[1] < 0) return GGMS_E_INVALID_ARG;
-  const uint64_t n = (uint64_t)h_tot[1];
-  const uint64_t nk64 = (uint64_t)h_k[1];
+  if (h[0] != 0 || h[2] != 0 || h[1] < 0 || h[3] < 0) return GGMS_E_INVALID_ARG;
+  const uint64_t n = (uint64_t)h[1];
+  const uint64_t nk64 = (uint64_t)h[3];
   if (nk64 == 0) return GGMS_OK;
   if (n == 0 || n > 0xFFFFFFFFull || nk64 > 0x7FFFFFFFull || !ks || !out) return GGMS_E_INVALID_ARG;
   const uint32_t nk = (uint32_t)nk64;
@@ -831,64 +832,30 @@ static int run_segmented(Context* ctx, const T* d_in, const int64_t* seg_off, in
   oo.num_buckets = 1024;
   oo.sample_size = 1024;
   Plan p;
-  int rc = make_plan(&p, n, nk, oo);
+  rc = make_plan(&p, n, nk, oo);
   if (rc) return rc;
-  const uint32_t small_keys = (uint32_t)(SMALL_SMEM / sizeof(K));
-  p.cap_seg = std::max<uint32_t>(nk, nseg) + 1;
-  p.cap_tiles = (uint32_t)((n + TILE - 1) / TILE) + p.cap_seg;
-  p.cap_q = (uint32_t)std::min<uint64_t>(nseg, n / QSAMP) + 1;
-  p.cap_rows = std::max(p.cap_q, (uint32_t)p.cap_rows);
-  Workspace<K> w0 = layout<K>(p, nullptr);
-  rc = ensure_arena(ctx, w0.bytes);
+  p.nlist = nseg;
+  p.sms = (uint32_t)ctx->sms;
+  rc = ensure_arena(ctx, layout<K>(p, nullptr).bytes);
   if (rc) return rc;
-  Workspace<K> w = layout<K>(p, ctx->arena);
-  const Caps caps{p.cap_seg, p.cap_tiles, p.nk, small_keys, tiny_keys<K>(), p.cap_rows};
+  const Workspace<K> w = layout<K>(p, ctx->arena);
+  const Caps caps{p.cap_seg, p.cap_tiles, p.nk, (uint32_t)(SMALL_SMEM / sizeof(K)), 0u, p.cap_rows};
   // the stream-ordered part: captured once and replayed when the call repeats
   auto enqueue = [&](cudaStream_t s) -> int {
     GGMS_CU(cudaMemsetAsync(w.C, 0, sizeof(Counters), s));
-    ++ctx->launches;
-    seg_init<K><<<cdiv(nseg, 256), 256, 0, s>>>(seg_off, nseg, k_off, w.segs[0], w.tiles[0], w.khead[0],
-                                                 w.smalls, w.tinies, w.bigs[0], p.cap_q, w.C, caps);
-    ++ctx->launches;
-    seg_set_count<<<1, 1, 0, s>>>(w.C, nseg);
-    ++ctx->launches;
-    k_init_seg<K><<<cdiv(nk, 256), 256, 0, s>>>(ks, nk, seg_off, k_off, nseg, w.segs[0], w.khead[0], w.knext,
-                                                 w.krank, w.kseg, w.C);
-    // small caller segments, straight from the input
-    rc = launch_small_select<T>(ctx, d_in, w.segs[0], w.khead[0], w, caps, s, k_off);
-    if (rc) return rc;
-    ++ctx->launches;
-    seg_sample<T><<<ctx->sms * 2, 1024, 0, s>>>(d_in, w.segs[0], w.bigs[0], w.C, p.cap_q, w.qtab, w.qdir,
-                                                 p.seed ^ 0x5E6A11ull);
-    // level 0 over the input with quantile bins; then radix levels over candidates
-    const int lv_grid = ctx->sms * lv_mult;
-    const int seg_grid = ctx->sms * 2;
-    ++ctx->launches;
-    lvl_prep<<<ctx->sms * 2, 256, 0, s>>>(w.rows[0], w.aflag[0], w.C, 0, caps);
-    ++ctx->launches;
-    lvl_count<T, LV_NT, true><<<lv_grid, LV_NT, 0, s>>>(d_in, w.segs[0], w.tiles[0], w.C, 0, w.rows[0], caps, w.qtab,
-                                                         w.qdir);
-    ++ctx->launches;
-    lvl_scan<<<seg_grid, 1024, 0, s>>>(w.rows[0], w.C, 0, caps);
-    ++ctx->launches;
-    lvl_locate_rows<<<cdiv(nk, 256), 256, 0, s>>>(w.rows[0], NBIN, nk, w.krank, w.kseg, &w.segs[0]->row,
-                                                     (uint32_t)(sizeof(Seg<K>) / 4), w.kbin, w.aflag[0], NBIN_WORDS,
-                                                     w.C);
-    ++ctx->launches;
-    lvl_children<K, 1024, true><<<seg_grid, 1024, 0, s>>>(w.rows[0], w.aflag[0], w.segs[0], w.C, 0, w.segs[1],
-                                                           w.cursor[1], w.tiles[1], w.points, w.khead[1], w.smalls,
-                                                           w.tinies, w.bigs[0], w.bigs[1], caps, w.qtab);
-    ++ctx->launches;
-    lvl_relabel<K><<<cdiv(nk, 256), 256, 0, s>>>(w.rows[0], NBIN, nk, w.segs[0], w.kbin, w.kseg, w.kkey, w.points, w.C,
-                                                    w.segs[1], w.khead[1], w.knext);
-    ++ctx->launches;
-    lvl_compact<T, LV_NT, true><<<lv_grid, LV_NT, 0, s>>>(d_in, w.segs[0], w.tiles[0], w.C, 0, w.rows[0], w.segs[1],
-                                                           w.cursor[1], w.cand[0], caps, w.qtab, w.qdir);
-    rc = launch_small_select<K>(ctx, w.cand[0], w.segs[1], w.khead[1], w, caps, s);
-    if (rc) return rc;
-    rc = launch_refine<T>(ctx, refine_args<T>(w, ctx, nk, caps, out, nullptr), s);
-    if (rc) return rc;
-    return cudaGetLastError() == cudaSuccess ? GGMS_OK : GGMS_E_CUDA;
+    BatchArgs<T> a;
+    a.in = d_in;
+    a.seg_off = seg_off;
+    a.k_off = k_off;
+    a.ks = ks;
+    a.nseg = nseg;
+    a.n = n;
+    a.seed = p.seed ^ 0x5E6A11ull;
+    a.lists = w.lists;
+    a.scratch = w.scratch;
+    a.r = refine_args<T>(w, ctx, nk, caps, out, nullptr);
+    if (const int r = launch_batch<T>(ctx, a, s)) return r;
+    return launch_refine<T>(ctx, a.r, s);
   };
   if (o.stats || ctx->profile) {
     rc = enqueue(st);
@@ -896,7 +863,7 @@ static int run_segmented(Context* ctx, const T* d_in, const int64_t* seg_off, in
     const uint64_t key[] = {0x5E6ull + sizeof(T), (uint64_t)(uintptr_t)d_in, (uint64_t)(uintptr_t)seg_off, nseg,
                             (uint64_t)(uintptr_t)ks, (uint64_t)(uintptr_t)k_off, (uint64_t)(uintptr_t)out, n,
                             nk, (uint64_t)(uintptr_t)ctx->arena, (uint64_t)std::is_signed<T>::value,
-                            (uint64_t)std::is_floating_point<T>::value, (uint64_t)lv_mult};
+                            (uint64_t)std::is_floating_point<T>::value, p.seed};
     rc = run_graphed(ctx, key, (int)(sizeof(key) / sizeof(key[0])), st, enqueue);
   }
   if (rc) return rc;
@@ -916,42 +883,6 @@ static int run_segmented(Context* ctx, const T* d_in, const int64_t* seg_off, in
 }
 
 template <typename T>
-static int run_segmented_tuned(Context* c, const T* d_in, const int64_t* seg_off, int64_t nseg,
-                               const uint32_t* ks, const int64_t* k_off, T* out, const ggms_opts& o,
-                               cudaStream_t st) {
-  if (!o.autotune || o.stats) return run_segmented<T>(c, d_in, seg_off, nseg, ks, k_off, out, o, st);
-  // the class needs n and K: read the totals (run_segmented reads them again)
-  int64_t h[2] = {0, 0};
-  if (nseg <= 0 || !seg_off || !k_off) return GGMS_E_INVALID_ARG;
-  GGMS_CU(cudaSetDevice(c->device));
-  GGMS_CU(cudaMemcpyAsync(&h[0], seg_off + nseg, 8, cudaMemcpyDeviceToHost, st));
-  GGMS_CU(cudaMemcpyAsync(&h[1], k_off + nseg, 8, cudaMemcpyDeviceToHost, st));
-  GGMS_CU(cudaStreamSynchronize(st));
-  const uint64_t key[4] = {0x5E60000ull | sizeof(T) | (std::is_floating_point<T>::value ? 32u : 0u),
-                           (uint64_t)bitlen64((uint64_t)std::max<int64_t>(h[0], 0)) |
-                               ((uint64_t)bitlen64((uint64_t)std::max<int64_t>(h[1], 0)) << 8) |
-                               ((uint64_t)bitlen64((uint64_t)nseg) << 16),
-                           0ull, 0ull};
-  if (const Context::Tuned* t = tuned_find(c, key))
-    return run_segmented<T>(c, d_in, seg_off, nseg, ks, k_off, out, o, st, t->lv_mult);
-  static const int mults[] = {4, 8, 16};
-  float best = 3.4e38f;
-  Context::Tuned pick{{key[0], key[1], key[2], key[3]}, 0, 0, 0, 8};
-  for (int m : mults) {
-    float ms = 0.0f;
-    const int rc = time_calls(st, [&] { return run_segmented<T>(c, d_in, seg_off, nseg, ks, k_off, out, o, st, m); },
-                              &ms);
-    if (rc) return rc;
-    if (ms < best) {
-      best = ms;
-      pick.lv_mult = m;
-    }
-  }
-  c->tuned.push_back(pick);
-  return run_segmented<T>(c, d_in, seg_off, nseg, ks, k_off, out, o, st, pick.lv_mult);
-}
-
-template <typename T>
 static int segmented(ggms_context* cx, const T* d_in, const int64_t* seg_off, int64_t nseg,
                      const uint32_t* ks, const int64_t* k_off, T* out, const ggms_opts* opts,
                      void* stream) {
@@ -963,7 +894,7 @@ static int segmented(ggms_context* cx, const T* d_in, const int64_t* seg_off, in
     if (rc) return rc;
   }
   std::lock_guard<std::mutex> lk(c->mu);
-  return run_segmented_tuned<T>(c, d_in, seg_off, nseg, ks, k_off, out, o, (cudaStream_t)stream);
+  return run_segmented<T>(c, d_in, seg_off, nseg, ks, k_off, out, o, (cudaStream_t)stream);
 }
 
 

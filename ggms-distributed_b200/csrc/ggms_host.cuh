@@ -62,7 +62,7 @@ struct Context {
   // autotuner: launch shapes and bucket counts picked per shape class
   struct Tuned {
     uint64_t key[4];
-    int B, nt, unroll, lv_mult;
+    int B, nt, unroll;
   };
   std::vector<Tuned> tuned;
 };
@@ -80,8 +80,9 @@ static int cuda_status(cudaError_t e) {
   } while (0)
 
 // Every layout of the arena begins with the call's counters and, at
-// ARENA_BAR, the word the grid barriers count on.
-constexpr size_t ARENA_BAR = 256;
+// ARENA_BAR, the words the barriers of cooperative launches count on: one for
+// the whole grid, and one for every team of the batched path.
+constexpr size_t ARENA_BAR = 256, ARENA_BAR_BYTES = 8192;
 
 static int ensure_arena(Context* c, size_t bytes) {
   if (c->arena_bytes >= bytes) return GGMS_OK;
@@ -94,10 +95,10 @@ static int ensure_arena(Context* c, size_t bytes) {
   size_t want = bytes + bytes / 8;
   GGMS_CU(cudaMalloc(&c->arena, want));
   c->arena_bytes = want;
-  // the grid barriers' word is zeroed here once (it needs no reset between
+  // the barriers' words are zeroed here once (they need no reset between
   // launches), on the context's own stream: the caller's may be capturing
   if (!c->query) GGMS_CU(cudaStreamCreateWithFlags(&c->query, cudaStreamNonBlocking));
-  GGMS_CU(cudaMemsetAsync(c->arena + ARENA_BAR, 0, 256, c->query));
+  GGMS_CU(cudaMemsetAsync(c->arena + ARENA_BAR, 0, ARENA_BAR_BYTES, c->query));
   GGMS_CU(cudaStreamSynchronize(c->query));
   return GGMS_OK;
 }
@@ -241,7 +242,8 @@ struct Plan {
   float bound;
   float window_z;    // < 0: no PASS 1 windows
   uint64_t seed;
-  uint32_t cap_q;    // batched path: caller segments with quantile bins (0: single path)
+  uint32_t nlist;    // batched path: segments (0: the other paths)
+  uint32_t sms;      // ... and CTAs with scratch
   uint32_t pl_knots; // learned PL model: requested segments (0: the default)
   uint32_t ring_st[3];  // stages of the passes' TMA rings: count, compact, coarse (0: other streams)
 };
@@ -281,7 +283,8 @@ static int make_plan(Plan* p, uint64_t n, uint32_t nk, const ggms_opts& o) {
   p->bound = o.imbalance_bound > 0.0f ? o.imbalance_bound : 3.0f;
   p->window_z = o.window_z == 0.0f ? 6.0f : o.window_z;
   p->seed = o.seed;
-  p->cap_q = 0;
+  p->nlist = 0;
+  p->sms = 0;
   if (o.pl_knots != 0 && (o.pl_knots < 16 || o.pl_knots > 1024)) return GGMS_E_INVALID_ARG;
   p->pl_knots = (uint32_t)o.pl_knots;
   p->ring_st[0] = p->ring_st[1] = p->ring_st[2] = 0;
@@ -409,8 +412,8 @@ static int mark_done(Context* c, cudaStream_t st) {
 // where ks and answers live) times every candidate on the caller's own data --
 // each candidate a full, correct call: 1 warm-up + 2 timed with CUDA events on
 // the caller's stream -- and keeps the fastest in the context; later calls of
-// the class use it.  The batched path tunes the CTAs per SM of its level
-// kernels the same way (class: type, log2 n, log2 K, log2 segments).
+// the class use it.  (The batched path has nothing to tune: its launch shapes
+// follow the segments' lengths.)
 static const Context::Tuned* tuned_find(Context* c, const uint64_t* key) {
   for (const auto& t : c->tuned)
     if (!memcmp(t.key, key, sizeof(t.key))) return &t;

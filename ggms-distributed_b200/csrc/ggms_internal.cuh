@@ -402,6 +402,12 @@ struct TileRef {
   uint32_t no;    // tile number inside the segment
 };
 
+// Classes of caller segments in the batched path (ggms_batch.cuh): teams of
+// CTAs of BT_TEAMS sizes, single CTAs by length (BT_SINGLES lists), one CTA's
+// sort, one warp (three lengths).
+constexpr uint32_t BT_TEAMS = 7, BT_SINGLES = 4;
+constexpr uint32_t BT_SORT = BT_TEAMS + BT_SINGLES, BT_WARP = BT_SORT + 1, BT_CLASSES = BT_WARP + 3;
+
 // Device counters (one small block of memory, zeroed per call).
 struct Counters {
   uint32_t nsegs[2];          // segments of the level stored in pool p
@@ -418,11 +424,12 @@ struct Counters {
   unsigned long long refine_elems;
   uint32_t asg_choice;        // index of the assigner in use (0 sampled, 1 learned)
   uint32_t win_runs;          // PASS 1 window runs in use (0: no windows)
-  uint32_t ntiny;             // tiny segments created by the current level (batched path)
+  uint32_t ntiny;             // tiny segments created by the current level
   uint32_t nbig[2];           // segments of pool p that a level refines (listed in bigs[p])
   uint32_t coarse;            // level 0 copies NGRP groups of buckets (most buckets hold a k)
   uint32_t passes;            // launches that read the whole input (counted by the kernels themselves)
   uint32_t ticket;            // CTAs of the call's last kernel that are done (the last one reports)
+  uint32_t nlist[BT_CLASSES]; // batched path: segments per class
 };
 
 // PASS 1 windows (l0_window).  From the sample, every requested k gets a
@@ -473,18 +480,6 @@ struct Caps {
   uint32_t tiny_keys;         // ... and with at most this many by tiny_select (one warp); 0: never
   uint32_t rows;              // segments a level can refine at once (its histogram rows)
 };
-
-// Level 0 of the batched path: a caller segment too large for small_select
-// gets QB bins whose boundaries are every second key of a sorted sample of
-// QSAMP of its keys (equal-mass bins whatever the distribution), and a
-// directory of QD cells, uniform in key over the sample's range, that gives
-// for each cell the boundaries below its first key -- a key's bin is then a
-// short search between two directory entries.
-constexpr uint32_t QB = NBIN;                   // bins (QB - 1 boundaries)
-constexpr uint32_t QSAMP = 2 * QB;              // sampled keys per segment
-constexpr int QD_BITS = 12;
-constexpr uint32_t QD = 1u << QD_BITS;          // directory cells
-constexpr uint32_t QDS = QD + 8;                // directory stride (QD + 1 entries, 16-byte rows)
 
 // Coarse level 0 (single vector, most buckets hold a k): NGRP groups of
 // 2^coarse_shift(B) consecutive buckets (B a power of two >= 2 * NGRP).

@@ -1370,19 +1370,6 @@ __device__ __forceinline__ void relabel_one(uint32_t i, uint32_t e, uint32_t* k_
   }
 }
 
-template <typename K>
-__global__ void lvl_relabel(const uint32_t* __restrict__ cmap, uint32_t row_len, uint32_t nk,
-                            const Seg<K>* __restrict__ segs, const uint32_t* __restrict__ k_bin,
-                            uint32_t* k_seg, K* k_key, const K* __restrict__ points, Counters* C,
-                            const Seg<K>* __restrict__ segs_q, uint32_t* khead_q, uint32_t* knext) {
-  pdl_entry();
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nk) return;
-  const uint32_t s = k_seg[i];
-  if (s == K_DONE) return;
-  relabel_one<K>(i, cmap[(size_t)segs[s].row * row_len + k_bin[i]], k_seg, k_key, points, C, segs_q, khead_q, knext);
-}
-
 // The first steps between PASS 1 and PASS 2 of one vector in ONE CTA (1024
 // threads), through shared memory: the scan of the bucket counts, every k's
 // bucket and rank in it, and the coarse-mode decision with the groups' counts
@@ -2113,106 +2100,6 @@ __device__ __forceinline__ void prep_body(uint32_t* rows, uint32_t* aflag, Count
   }
 }
 
-__global__ void lvl_prep(uint32_t* rows, uint32_t* aflag, Counters* C, int p, Caps caps) {
-  pdl_entry();
-  prep_body(rows, aflag, C, p, caps, blockIdx.x, gridDim.x);
-}
-
-// Bin of a key in a quantile segment: the number of boundaries <= key.  The
-// directory cell of the key bounds the search: boundaries before qd[c] lie
-// below the cell's first key, those from qd[c + 1] on above its last.
-template <typename K>
-__device__ __forceinline__ uint32_t qbin(K key, K kmin, uint32_t dsh, const K* qb, const uint16_t* qd) {
-  const K d = key > kmin ? (K)(key - kmin) : (K)0;
-  const K cc = d >> dsh;
-  const uint32_t c = cc < (K)QD ? (uint32_t)cc : QD - 1u;
-  uint32_t lo = qd[c], hi = qd[c + 1];
-  while (lo < hi) {
-    const uint32_t m = (lo + hi) >> 1;
-    if (qb[m] <= key) lo = m + 1; else hi = m;
-  }
-  return lo;
-}
-
-// Boundaries and directory of quantile segment q into shared memory.
-template <typename K>
-__device__ __forceinline__ void qtab_to_smem(const K* __restrict__ qtab, const uint16_t* __restrict__ qdir,
-                                             uint32_t q, K* qb, uint16_t* qd) {
-  const K* tb = qtab + (size_t)q * QB;
-  for (uint32_t i = threadIdx.x; i < QB; i += blockDim.x) qb[i] = tb[i];
-  const uint4* dr = reinterpret_cast<const uint4*>(qdir + (size_t)q * QDS);
-  uint4* dd = reinterpret_cast<uint4*>(qd);
-  for (uint32_t i = threadIdx.x; i < QDS / 8; i += blockDim.x) dd[i] = dr[i];
-}
-
-// Sample-quantile bins of the batched level 0: one CTA per large caller
-// segment draws QSAMP keys (one from each of QSAMP equal strata, at a hashed
-// offset inside it), sorts them, and writes the QB - 1 boundaries and the
-// directory; the segment's lo / shift become the directory's origin / cell
-// shift and pad its table index.
-template <typename T>
-__global__ __launch_bounds__(1024) void seg_sample(const T* __restrict__ in, Seg<typename KeyOf<T>::K>* segs0,
-                                                   const uint32_t* __restrict__ qsegs,
-                                                   const Counters* __restrict__ C, uint32_t cap_q,
-                                                   typename KeyOf<T>::K* qtab, uint16_t* qdir, uint64_t seed) {
-  pdl_entry();
-  using K = typename KeyOf<T>::K;
-  __shared__ K sv[QSAMP];
-  const uint32_t tid = threadIdx.x;
-  const uint32_t nq = min(C->nbig[0], cap_q);
-  for (uint32_t q = blockIdx.x; q < nq; q += gridDim.x) {
-    const uint32_t sid = qsegs[q];
-    Seg<K> s = segs0[sid];
-    for (uint32_t i = tid; i < QSAMP; i += 1024) {
-      const uint64_t a = (uint64_t)s.cnt * i / QSAMP, b = (uint64_t)s.cnt * (i + 1) / QSAMP;
-      const uint64_t h = mix64(seed ^ ((uint64_t)sid << 32) ^ i);
-      const uint64_t pos = a + (((h >> 32) * (b - a)) >> 32);  // in [a, b) (b - a < 2^32), or a
-      sv[i] = KeyOf<T>::to(in[s.off + pos]);
-    }
-    __syncthreads();
-    for (uint32_t kk = 2; kk <= QSAMP; kk <<= 1) {
-      for (uint32_t jj = kk >> 1; jj > 0; jj >>= 1) {
-        for (uint32_t i = tid; i < QSAMP; i += 1024) {
-          const uint32_t ixj = i ^ jj;
-          if (ixj > i) {
-            const K a = sv[i], b = sv[ixj];
-            if ((a > b) == ((i & kk) == 0)) { sv[i] = b; sv[ixj] = a; }
-          }
-        }
-        // stages with jj < 32 stay inside a warp (i and i ^ jj: lanes l, l ^ jj)
-        const uint32_t nj = jj > 1 ? (jj >> 1) : kk;
-        if (nj >= 32u || (jj == 1 && kk == QSAMP)) __syncthreads(); else __syncwarp();
-      }
-    }
-    K* tb = qtab + (size_t)q * QB;
-    for (uint32_t j = tid; j < QB; j += 1024) tb[j] = (j + 1 < QB) ? sv[2 * j + 2] : key_max<K>();
-    const K kmin = sv[0], kmax = sv[QSAMP - 1];
-    const uint32_t dsh = (uint32_t)max(0, bitlen((K)(kmax - kmin)) - QD_BITS);
-    uint16_t* dr = qdir + (size_t)q * QDS;
-    for (uint32_t c = tid; c < QDS; c += 1024) {
-      uint32_t v = QB - 1u;  // past the range (or padding): every boundary is below
-      const K off = (K)((K)c << dsh);
-      if (c < QD && ((off >> dsh) == (K)c) && off <= (K)(key_max<K>() - kmin)) {
-        const K start = (K)(kmin + off);
-        uint32_t lo = 0, hi = QB - 1u;  // boundaries j < lo are < start
-        while (lo < hi) {
-          const uint32_t m = (lo + hi) >> 1;
-          if (sv[2 * m + 2] < start) lo = m + 1; else hi = m;
-        }
-        v = lo;
-      }
-      dr[c] = (uint16_t)v;
-    }
-    if (tid == 0) {
-      s.lo = kmin;
-      s.shift = dsh;
-      s.pad = q;
-      segs0[sid] = s;
-    }
-    __syncthreads();
-  }
-}
-
 // Elements [beg, end) of a candidate buffer, 16 bytes at a time: every thread
 // calls f(keys, mask) for its vectors, U of them in flight; bit t of mask says
 // that keys[t] is one of the elements (the first and last vector may reach
@@ -2244,26 +2131,18 @@ __device__ __forceinline__ void tile_stream(const K* src, uint64_t beg, uint64_t
   }
 }
 
-// Histogram of radix bins, one tile of one segment per iteration.
-// Q: the level's segments have quantile bins (batched level 0), else radix
-// bins (key - lo) >> shift.
-// h: NBIN words of shared memory.
-template <typename InT, int NT, bool Q = false>
-__device__ __forceinline__ void count_body(const InT* src, const Seg<typename KeyOf<InT>::K>* segs,
-                                           const TileRef* tiles, Counters* C, int p, uint32_t* rows,
-                                           const Caps& caps, const typename KeyOf<InT>::K* qtab,
-                                           const uint16_t* qdir, uint32_t* h, uint32_t cta, uint32_t ncta) {
-  using K = typename KeyOf<InT>::K;
-  __shared__ __align__(16) K qb[Q ? QB : 1];
-  __shared__ __align__(16) uint16_t qd[Q ? QDS : 8];
+// Histogram of radix bins (key - lo) >> shift, one tile of one segment per
+// iteration.  h: NBIN words of shared memory.
+template <typename K, int NT>
+__device__ __forceinline__ void count_body(const K* src, const Seg<K>* segs, const TileRef* tiles, Counters* C, int p,
+                                           uint32_t* rows, const Caps& caps, uint32_t* h, uint32_t cta,
+                                           uint32_t ncta) {
   const uint32_t nt = min(C->ntiles[p], caps.tiles);
   const uint32_t ns = min(C->nsegs[p], caps.segs);
-  if (Q && nt && cta == 0 && threadIdx.x == 0) atomicAdd(&C->passes, 1u);  // level 0 reads the input
   // Each CTA takes a contiguous range of the tile list, where a segment's tiles
   // are consecutive: the histogram of one segment's run of tiles stays in
   // shared memory and is added to the segment's row once per run, not once
-  // per tile (a row holds NBIN bins for TILE keys), and the quantile table is
-  // loaded once per run.
+  // per tile (a row holds NBIN bins for TILE keys).
   const uint32_t per = (nt + ncta - 1) / ncta;
   const uint32_t t_beg = min(cta * per, nt), t_end = min(t_beg + per, nt);
   uint32_t open = 0xFFFFFFFFu;  // segment whose counts the shared histogram holds
@@ -2286,7 +2165,6 @@ __device__ __forceinline__ void count_body(const InT* src, const Seg<typename Ke
         flush();
         __syncthreads();
       }
-      if (Q) qtab_to_smem<K>(qtab, qdir, s.pad, qb, qd);
       for (uint32_t i = threadIdx.x; i < NBIN; i += NT) h[i] = 0u;
       open = tr.seg;
       open_row = s.row;
@@ -2295,45 +2173,16 @@ __device__ __forceinline__ void count_body(const InT* src, const Seg<typename Ke
     }
     const uint64_t beg = s.off + (uint64_t)tr.no * TILE;
     const uint64_t end = min(beg + TILE, s.off + s.cnt);
-    if constexpr (Q) {
-      constexpr int U = 8;  // independent loads in flight per thread
-      for (uint64_t o = beg + threadIdx.x; o < end; o += (uint64_t)NT * U) {
-        K kk[U];
+    tile_stream<K, NT>(src, beg, end, [&](const K* k, uint32_t mask) {
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const uint64_t i = o + (uint64_t)u * NT;
-          kk[u] = i < end ? KeyOf<InT>::to(src[i]) : (K)0;
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          if (o + (uint64_t)u * NT >= end) break;
-          atomicAdd(&h[qbin<K>(kk[u], s.lo, s.shift, qb, qd)], 1u);
-        }
-      }
-    } else {
-      tile_stream<K, NT>(src, beg, end, [&](const K* k, uint32_t mask) {
-#pragma unroll
-        for (int t = 0; t < 16 / (int)sizeof(K); ++t)
-          if ((mask >> t) & 1u)
-            atomicAdd(&h[min((uint32_t)((K)(k[t] - s.lo) >> s.shift), (uint32_t)NBIN - 1u)], 1u);
-      });
-    }
+      for (int t = 0; t < 16 / (int)sizeof(K); ++t)
+        if ((mask >> t) & 1u)
+          atomicAdd(&h[min((uint32_t)((K)(k[t] - s.lo) >> s.shift), (uint32_t)NBIN - 1u)], 1u);
+    });
     open_keys += end - beg;
     __syncthreads();
   }
   if (open != 0xFFFFFFFFu) flush();  // the last tile ended with a barrier
-}
-
-template <typename InT, int NT, bool Q = false>
-__global__ __launch_bounds__(NT) void lvl_count(const InT* __restrict__ src,
-                                               const Seg<typename KeyOf<InT>::K>* __restrict__ segs,
-                                               const TileRef* __restrict__ tiles,
-                                               Counters* C, int p, uint32_t* rows, Caps caps,
-                                               const typename KeyOf<InT>::K* __restrict__ qtab,
-                                               const uint16_t* __restrict__ qdir) {
-  pdl_entry();
-  __shared__ uint32_t h[NBIN];
-  count_body<InT, NT, Q>(src, segs, tiles, C, p, rows, caps, qtab, qdir, h, blockIdx.x, gridDim.x);
 }
 
 // w: 72 words of shared memory
@@ -2345,21 +2194,15 @@ __device__ __forceinline__ void scan_body(uint32_t* rows, const Counters* C, int
     block_inclusive_scan_global<NT>(rows + (size_t)j * NBIN, NBIN, w, nullptr);
 }
 
-__global__ __launch_bounds__(1024) void lvl_scan(uint32_t* rows, const Counters* __restrict__ C, int p, Caps caps) {
-  pdl_entry();
-  __shared__ uint32_t w[72];
-  scan_body<1024>(rows, C, p, caps, w, blockIdx.x, gridDim.x);
-}
-
 // Active bins of each segment -> child segments (pool q) or points.  One CTA
 // per segment; the row holding the inclusive counts is overwritten by the
 // child map (each entry read before any is written).
-template <typename K, int NT, bool Q = false>
+template <typename K, int NT>
 __device__ __forceinline__ void children_body(uint32_t* rows, const uint32_t* aflag, const Seg<K>* segs,
                                               Counters* C, int p, Seg<K>* segs_q, uint32_t* cursor_q,
                                               TileRef* tiles_q, K* points, uint32_t* khead_q, uint32_t* smalls,
                                               uint32_t* tinies, const uint32_t* bigs, uint32_t* bigs_q,
-                                              const Caps& caps, const K* qtab, uint32_t cta, uint32_t ncta) {
+                                              const Caps& caps, uint32_t cta, uint32_t ncta) {
   constexpr int PER = NBIN / NT;
   const uint32_t nb = min(C->nbig[p], caps.rows);
   for (uint32_t j = cta; j < nb; j += ncta) {
@@ -2374,20 +2217,9 @@ __device__ __forceinline__ void children_body(uint32_t* rows, const uint32_t* af
       if (!((F[b >> 5] >> (b & 31)) & 1u)) continue;
       const uint32_t start = b ? I[b - 1] : 0u;
       const uint32_t cnt = I[b] - start;
-      K blo, bhi;
-      if (Q) {  // [boundary b - 1, boundary b - 1]; the outer bins reach the ends of the key space
-        const K* tb = qtab + (size_t)s.pad * QB;
-        blo = b ? tb[b - 1] : (K)0;
-        bhi = (b + 1u < QB) ? (K)(tb[b] - 1u) : key_max<K>();
-        if (b + 1u < QB && tb[b] <= blo) {  // an empty bin cannot hold a k
-          set_status(C, GGMS_E_INTERNAL);
-          continue;
-        }
-      } else {
-        blo = s.lo + ((K)b << s.shift);
-        const K width_m1 = (K)(((K)1 << s.shift) - 1);
-        bhi = (key_max<K>() - blo < width_m1) ? key_max<K>() : (K)(blo + width_m1);
-      }
+      const K blo = s.lo + ((K)b << s.shift);
+      const K width_m1 = (K)(((K)1 << s.shift) - 1);
+      K bhi = (key_max<K>() - blo < width_m1) ? key_max<K>() : (K)(blo + width_m1);
       if (bhi > s.hi) bhi = s.hi;
       if (blo == bhi) {
         uint32_t pid = atomicAdd(&C->npoints, 1u);
@@ -2433,18 +2265,6 @@ __device__ __forceinline__ void children_body(uint32_t* rows, const uint32_t* af
   }
 }
 
-template <typename K, int NT, bool Q = false>
-__global__ __launch_bounds__(NT) void lvl_children(uint32_t* rows, const uint32_t* __restrict__ aflag,
-                                                  const Seg<K>* __restrict__ segs, Counters* C, int p,
-                                                  Seg<K>* segs_q, uint32_t* cursor_q, TileRef* tiles_q,
-                                                  K* points, uint32_t* khead_q, uint32_t* smalls,
-                                                  uint32_t* tinies, const uint32_t* __restrict__ bigs,
-                                                  uint32_t* bigs_q, Caps caps, const K* __restrict__ qtab) {
-  pdl_entry();
-  children_body<K, NT, Q>(rows, aflag, segs, C, p, segs_q, cursor_q, tiles_q, points, khead_q, smalls, tinies,
-                          bigs, bigs_q, caps, qtab, blockIdx.x, gridDim.x);
-}
-
 // Copies each key whose bin became a child segment into that child's region.
 // Tiles go to CTAs grid-stride, so the CTAs running at one time fill the same
 // children side by side and L2 merges their partial sectors (contiguous tile
@@ -2452,22 +2272,16 @@ __global__ __launch_bounds__(NT) void lvl_children(uint32_t* rows, const uint32_
 // A tile's hits (3 % of its keys in a typical level) go through a per-warp
 // queue and are written 32 at a time, one per lane: the cursor reservations of
 // 32 hits are then one round trip to L2, where reserving each hit as it was
-// found paid a trip per hit.  (The batched level 0, where 12 % are hits, has
-// enough of them in flight without the queue: 13.9 ms with it, 13.2 without.)
+// found paid a trip per hit.
 // cm: NBIN words of shared memory, then the queues (COMPACT_SMEM bytes in all).
 template <typename K, int NT>
 constexpr size_t COMPACT_SMEM = 4u * NBIN + (NT / 32) * WQ_DEPTH * (sizeof(K) + 4u);
 
-template <typename InT, int NT, bool Q = false>
-__device__ __forceinline__ void compact_body(const InT* src, const Seg<typename KeyOf<InT>::K>* segs,
-                                             const TileRef* tiles, const Counters* C, int p, const uint32_t* rows,
-                                             const Seg<typename KeyOf<InT>::K>* segs_q, uint32_t* cursor_q,
-                                             typename KeyOf<InT>::K* dst, const Caps& caps,
-                                             const typename KeyOf<InT>::K* qtab, const uint16_t* qdir,
-                                             uint32_t* cm, uint32_t cta, uint32_t ncta) {
-  using K = typename KeyOf<InT>::K;
-  __shared__ __align__(16) K qb[Q ? QB : 1];
-  __shared__ __align__(16) uint16_t qd[Q ? QDS : 8];
+template <typename K, int NT>
+__device__ __forceinline__ void compact_body(const K* src, const Seg<K>* segs, const TileRef* tiles,
+                                             const Counters* C, int p, const uint32_t* rows, const Seg<K>* segs_q,
+                                             uint32_t* cursor_q, K* dst, const Caps& caps, uint32_t* cm, uint32_t cta,
+                                             uint32_t ncta) {
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lt = lanemask_lt();
   K* qk = reinterpret_cast<K*>(cm + NBIN) + warp * WQ_DEPTH;
   uint32_t* qc = reinterpret_cast<uint32_t*>(reinterpret_cast<K*>(cm + NBIN) + (NT / 32) * WQ_DEPTH) + warp * WQ_DEPTH;
@@ -2487,9 +2301,7 @@ __device__ __forceinline__ void compact_body(const InT* src, const Seg<typename 
   };
   const uint32_t nt = min(C->ntiles[p], caps.tiles);
   const uint32_t ns = min(C->nsegs[p], caps.segs);
-  if (Q && nt && cta == 0 && threadIdx.x == 0)  // level 0 reads the input
-    atomicAdd(&const_cast<Counters*>(C)->passes, 1u);
-  uint32_t loaded = 0xFFFFFFFFu;  // segment whose child map (and table) is in shared memory
+  uint32_t loaded = 0xFFFFFFFFu;  // segment whose child map is in shared memory
   for (uint32_t t = cta; t < nt; t += ncta) {
     const TileRef tr = tiles[t];
     if (tr.seg >= ns) continue;  // only after a capacity error (status already set)
@@ -2497,113 +2309,54 @@ __device__ __forceinline__ void compact_body(const InT* src, const Seg<typename 
     if (tr.seg != loaded) {  // the previous tile ended with a barrier
       const uint32_t* row = rows + (size_t)s.row * NBIN;
       for (uint32_t i = threadIdx.x; i < NBIN; i += NT) cm[i] = row[i];
-      if (Q) qtab_to_smem<K>(qtab, qdir, s.pad, qb, qd);
       loaded = tr.seg;
     }
     __syncthreads();
     const uint64_t beg = s.off + (uint64_t)tr.no * TILE;
     const uint64_t end = min(beg + TILE, s.off + s.cnt);
-    if constexpr (Q) {
-      constexpr int U = 4;  // loads in flight per thread before the warp-synchronous part
-      const uint64_t span = ((end - beg + NT * U - 1) / (NT * U)) * (NT * U);
-      for (uint64_t o = threadIdx.x; o < span; o += NT * U) {
-        K kk[U];
+    tile_stream<K, NT>(src, beg, end, [&](const K* k, uint32_t mask) {
+      constexpr int N = 16 / (int)sizeof(K);
+      uint32_t cc[N];
+      bool any = false;
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const uint64_t i = beg + o + (uint64_t)u * NT;
-          kk[u] = i < end ? KeyOf<InT>::to(src[i]) : (K)0;
+      for (int t = 0; t < N; ++t) {
+        cc[t] = cm[min((uint32_t)((K)(k[t] - s.lo) >> s.shift), (uint32_t)NBIN - 1u)];
+        if (!((mask >> t) & 1u)) cc[t] = CM_NONE;
+        any = any || cc[t] < CM_POINT;
+      }
+      if (!__any_sync(FULL, any)) return;
+#pragma unroll
+      for (int t = 0; t < N; ++t) {
+        const bool hit = cc[t] < CM_POINT;
+        const uint32_t hm = __ballot_sync(FULL, hit);
+        if (hit) {
+          const uint32_t at = qn + __popc(hm & lt);
+          qk[at] = k[t];
+          qc[at] = cc[t];
         }
-        // each key's child (CM_NONE when its bin is not copied)
-        uint32_t cc[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-          cc[u] = beg + o + (uint64_t)u * NT < end ? cm[qbin<K>(kk[u], s.lo, s.shift, qb, qd)] : CM_NONE;
-        // one cursor reservation per group of lanes with the same child, for
-        // all U keys before any result is used
-        uint32_t peers[U], base[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const bool hit = cc[u] < CM_POINT;
-          const uint32_t hm = __ballot_sync(FULL, hit);
-          peers[u] = 0u;
-          base[u] = 0u;
-          if (hit) {
-            peers[u] = __match_any_sync(hm, cc[u]);
-            if ((int)lane == __ffs(peers[u]) - 1) base[u] = atomicAdd(&cursor_q[cc[u]], (uint32_t)__popc(peers[u]));
+        qn += __popc(hm);
+        if (qn >= 32u) {
+          __syncwarp();
+          const K k0 = qk[lane];
+          const uint32_t c0 = qc[lane];
+          const bool more = lane + 32u < qn;
+          const K k1 = more ? qk[lane + 32u] : (K)0;
+          const uint32_t c1 = more ? qc[lane + 32u] : 0u;
+          __syncwarp();
+          if (more) {
+            qk[lane] = k1;
+            qc[lane] = c1;
           }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          if (peers[u]) {
-            const uint32_t b0 = __shfl_sync(peers[u], base[u], __ffs(peers[u]) - 1);
-            const uint32_t slot = b0 + __popc(peers[u] & lt);
-            const Seg<K>& sg = segs_q[cc[u]];
-            if (slot < sg.cnt) dst[sg.off + slot] = kk[u];
-            else set_status(const_cast<Counters*>(C), GGMS_E_INTERNAL);
-          }
+          qn -= 32u;
+          __syncwarp();
+          emit(FULL, k0, c0);
         }
       }
-    } else {
-      tile_stream<K, NT>(src, beg, end, [&](const K* k, uint32_t mask) {
-        constexpr int N = 16 / (int)sizeof(K);
-        uint32_t cc[N];
-        bool any = false;
-#pragma unroll
-        for (int t = 0; t < N; ++t) {
-          cc[t] = cm[min((uint32_t)((K)(k[t] - s.lo) >> s.shift), (uint32_t)NBIN - 1u)];
-          if (!((mask >> t) & 1u)) cc[t] = CM_NONE;
-          any = any || cc[t] < CM_POINT;
-        }
-        if (!__any_sync(FULL, any)) return;
-#pragma unroll
-        for (int t = 0; t < N; ++t) {
-          const bool hit = cc[t] < CM_POINT;
-          const uint32_t hm = __ballot_sync(FULL, hit);
-          if (hit) {
-            const uint32_t at = qn + __popc(hm & lt);
-            qk[at] = k[t];
-            qc[at] = cc[t];
-          }
-          qn += __popc(hm);
-          if (qn >= 32u) {
-            __syncwarp();
-            const K k0 = qk[lane];
-            const uint32_t c0 = qc[lane];
-            const bool more = lane + 32u < qn;
-            const K k1 = more ? qk[lane + 32u] : (K)0;
-            const uint32_t c1 = more ? qc[lane + 32u] : 0u;
-            __syncwarp();
-            if (more) {
-              qk[lane] = k1;
-              qc[lane] = c1;
-            }
-            qn -= 32u;
-            __syncwarp();
-            emit(FULL, k0, c0);
-          }
-        }
-      });
-    }
+    });
     __syncthreads();
   }
   __syncwarp();
   if (lane < qn) emit((1u << qn) - 1u, qk[lane], qc[lane]);  // qn < 32
-}
-
-template <typename InT, int NT, bool Q = false>
-__global__ __launch_bounds__(NT) void lvl_compact(const InT* __restrict__ src,
-                                                 const Seg<typename KeyOf<InT>::K>* __restrict__ segs,
-                                                 const TileRef* __restrict__ tiles,
-                                                 const Counters* __restrict__ C, int p,
-                                                 const uint32_t* __restrict__ rows,
-                                                 const Seg<typename KeyOf<InT>::K>* __restrict__ segs_q,
-                                                 uint32_t* cursor_q, typename KeyOf<InT>::K* dst,
-                                                 Caps caps, const typename KeyOf<InT>::K* __restrict__ qtab,
-                                                 const uint16_t* __restrict__ qdir) {
-  pdl_entry();
-  __shared__ __align__(16) uint32_t cm[Q ? NBIN : COMPACT_SMEM<typename KeyOf<InT>::K, NT> / 4];
-  compact_body<InT, NT, Q>(src, segs, tiles, C, p, rows, segs_q, cursor_q, dst, caps, qtab, qdir, cm, blockIdx.x,
-                           gridDim.x);
 }
 
 // ------------------------------------------------------------------ small segments
@@ -2623,15 +2376,14 @@ constexpr size_t SMALL_SELECT_SMEM = SMALL_SMEM + (size_t)SS_GROUP * 256 * 4;
 template <typename InT, int NT>
 __device__ __forceinline__ void small_select_body(const InT* src, const Seg<typename KeyOf<InT>::K>* segs_q,
                                                   const uint32_t* smalls, Counters* C, const uint32_t* khead_q,
-                                                  const uint32_t* knext, const int64_t* k_off,
-                                                  const uint32_t* k_rank, uint32_t* k_seg,
+                                                  const uint32_t* knext, const uint32_t* k_rank, uint32_t* k_seg,
                                                   typename KeyOf<InT>::K* k_key, uint32_t small_keys,
                                                   const Caps& caps, uint8_t* smem, uint32_t cta, uint32_t ncta) {
   using K = typename KeyOf<InT>::K;
   K* vals = (K*)smem;
   uint32_t* hist = (uint32_t*)(smem + SMALL_SMEM);           // [SS_GROUP][256]
   __shared__ uint32_t kid[SS_MAXK];
-  __shared__ uint32_t nk_s, next_s, kend_s;
+  __shared__ uint32_t nk_s, next_s;
   __shared__ uint32_t rk[SS_GROUP];
   __shared__ K pk[SS_GROUP];
   __shared__ K upk[SS_GROUP];       // distinct prefixes of the current round
@@ -2685,27 +2437,11 @@ __device__ __forceinline__ void small_select_body(const InT* src, const Seg<type
     for (uint32_t i = tid; i < cnt; i += NT) vals[i] = (K)(vals[i] - mn);
     const int bits = bitlen((K)(mx - mn));
     bool sorted_seg = false;
-    if (tid == 0) {  // the ks: the segment's list, or (k_off: a caller segment) its k range
-      if (k_off) {
-        const uint32_t k0 = (uint32_t)k_off[id], k1 = (uint32_t)k_off[id + 1];
-        next_s = k0 < k1 ? k0 : K_NIL;
-        kend_s = k1;
-      } else {
-        next_s = khead_q[id];
-      }
-    }
+    if (tid == 0) next_s = khead_q[id];  // the ks: the segment's list
     __syncthreads();
     while (next_s != K_NIL) {
       __syncthreads();
-      if (k_off) {  // the next up to SS_MAXK ks of the range
-        const uint32_t k0 = next_s, m = min((uint32_t)SS_MAXK, kend_s - k0);
-        for (uint32_t j = tid; j < m; j += NT) kid[j] = k0 + j;
-        __syncthreads();
-        if (tid == 0) {
-          nk_s = m;
-          next_s = (k0 + m < kend_s) ? k0 + m : K_NIL;
-        }
-      } else if (tid == 0) {  // collect up to SS_MAXK ks from the list
+      if (tid == 0) {  // collect up to SS_MAXK ks from the list
         uint32_t k = next_s, m = 0;
         while (k != K_NIL && m < (uint32_t)SS_MAXK) { kid[m++] = k; k = knext[k]; }
         nk_s = m;
@@ -2833,23 +2569,20 @@ __global__ __launch_bounds__(NT) void small_select(const InT* __restrict__ src,
                                                   const Counters* __restrict__ C_,
                                                   const uint32_t* __restrict__ khead_q,
                                                   const uint32_t* __restrict__ knext,
-                                                  const int64_t* __restrict__ k_off,
                                                   const uint32_t* __restrict__ k_rank, uint32_t* k_seg,
                                                   typename KeyOf<InT>::K* k_key, uint32_t small_keys,
                                                   Caps caps) {
   pdl_entry();
   extern __shared__ __align__(128) uint8_t smem[];
-  small_select_body<InT, NT>(src, segs_q, smalls, const_cast<Counters*>(C_), khead_q, knext, k_off, k_rank, k_seg,
+  small_select_body<InT, NT>(src, segs_q, smalls, const_cast<Counters*>(C_), khead_q, knext, k_rank, k_seg,
                              k_key, small_keys, caps, smem, blockIdx.x, gridDim.x);
 }
 
-// One warp finishes a whole tiny segment (at most tiny_keys<K>() keys, as
-// offsets from its lo, in the warp's slice of shared memory).  With few ks: per
-// k, a radix select with 8-bit digits from the top of the segment's range (one
-// warp-private 256-bin histogram per digit).  With more than TS_SORT_ABOVE ks
-// (caller segments of the batched path): the slice is bitonic-sorted once and
-// the lanes read their ks' answers from it.  The ks come from the segment's
-// list, or (k_off given: the segments are the caller's) from its k range.
+// One warp finishes a whole tiny segment (at most TK keys, as offsets from its
+// lo, in the warp's slice of shared memory).  Up to 64 keys: every key's rank by
+// comparison.  Else per k a radix select with 8-bit digits from the top of the
+// segment's range (one warp-private 256-bin histogram per digit), or, with more
+// than TS_SORT_ABOVE ks, one bitonic sort.  The ks come from the segment's list.
 constexpr int TS_NT = 128;
 
 template <typename K>
@@ -2911,8 +2644,7 @@ __device__ __forceinline__ K warp_radix_select(const K* v, uint32_t cnt, int bit
 template <typename InT, int NW, uint32_t TK>
 __device__ __forceinline__ void tiny_select_body(const InT* src, const Seg<typename KeyOf<InT>::K>* segs_q,
                                                  const uint32_t* tinies, Counters* C, const uint32_t* khead_q,
-                                                 const uint32_t* knext, const int64_t* k_off,
-                                                 const uint32_t* k_rank, uint32_t* k_seg,
+                                                 const uint32_t* knext, const uint32_t* k_rank, uint32_t* k_seg,
                                                  typename KeyOf<InT>::K* k_key, const Caps& caps,
                                                  typename KeyOf<InT>::K* buf, uint32_t* hist, uint32_t cta,
                                                  uint32_t ncta) {
@@ -2953,7 +2685,7 @@ __device__ __forceinline__ void tiny_select_body(const InT* src, const Seg<typen
     if (lane < batch && tj < nt) {
       pid = tinies[tj];
       ps = segs_q[pid];
-      if (!k_off) pkh = khead_q[pid];
+      pkh = khead_q[pid];
     }
     const uint32_t nb = min(batch, nt - t0);
     for (uint32_t j = 0; j < nb; ++j) {
@@ -3010,55 +2742,20 @@ __device__ __forceinline__ void tiny_select_body(const InT* src, const Seg<typen
         const K xb = __shfl_sync(FULL, kb, mb ? __ffs(mb) - 1 : 0);
         return ma ? xa : xb;
       };
-      if (k_off && by_rank) {
-        const int64_t k0 = k_off[id], k1 = k_off[id + 1];
-        for (int64_t k = k0; k < k1; ++k) {
-          if (k_seg[k] == K_DONE) continue;  // warp-uniform
-          bool ok = false;
-          const K pre = rank_pick(k_rank[k], &ok);
-          if (lane == 0) {
-            if (ok) k_key[k] = (K)(s.lo + pre); else set_status(C, GGMS_E_INTERNAL);
-            k_seg[k] = K_DONE;
-          }
-        }
-      } else if (k_off) {
-        const int64_t k0 = k_off[id], k1 = k_off[id + 1];
-        if ((uint64_t)(k1 - k0) > TS_SORT_ABOVE) {
-          sort_slice(cnt);
-          for (int64_t k = k0 + lane; k < k1; k += 32) {
-            if (k_seg[k] == K_DONE) continue;  // an invalid k (status already set)
-            const uint32_t r = k_rank[k];
-            if (r < cnt) k_key[k] = (K)(s.lo + v[r]); else set_status(C, GGMS_E_INTERNAL);
-            k_seg[k] = K_DONE;
-          }
-        } else {
-          for (int64_t k = k0; k < k1; ++k) {
-            if (k_seg[k] == K_DONE) continue;  // warp-uniform
-            bool ok = false;
-            const uint32_t r = k_rank[k];
-            const K pre = r < cnt ? warp_radix_select<K>(v, cnt, bits, r, h, lane, &ok) : (K)0;
-            if (lane == 0) {
-              if (ok) k_key[k] = (K)(s.lo + pre); else set_status(C, GGMS_E_INTERNAL);
-              k_seg[k] = K_DONE;
-            }
-          }
-        }
-      } else {
-        uint32_t some = 0;  // ks, up to TS_SORT_ABOVE + 1 of them
-        if (!by_rank)
-          for (uint32_t k = khead; k != K_NIL && some <= TS_SORT_ABOVE; k = knext[k]) ++some;
-        const bool sorted = some > TS_SORT_ABOVE;
-        if (sorted) sort_slice(cnt);
-        for (uint32_t k = khead; k != K_NIL; k = knext[k]) {
-          bool ok = false;
-          const uint32_t r = k_rank[k];
-          K pre = 0;
-          if (by_rank) pre = rank_pick(r, &ok);
-          else if ((ok = r < cnt)) pre = sorted ? v[r] : warp_radix_select<K>(v, cnt, bits, r, h, lane, &ok);
-          if (lane == 0) {
-            if (ok) k_key[k] = (K)(s.lo + pre); else set_status(C, GGMS_E_INTERNAL);
-            k_seg[k] = K_DONE;
-          }
+      uint32_t some = 0;  // ks, up to TS_SORT_ABOVE + 1 of them
+      if (!by_rank)
+        for (uint32_t k = khead; k != K_NIL && some <= TS_SORT_ABOVE; k = knext[k]) ++some;
+      const bool sorted = some > TS_SORT_ABOVE;
+      if (sorted) sort_slice(cnt);
+      for (uint32_t k = khead; k != K_NIL; k = knext[k]) {
+        bool ok = false;
+        const uint32_t r = k_rank[k];
+        K pre = 0;
+        if (by_rank) pre = rank_pick(r, &ok);
+        else if ((ok = r < cnt)) pre = sorted ? v[r] : warp_radix_select<K>(v, cnt, bits, r, h, lane, &ok);
+        if (lane == 0) {
+          if (ok) k_key[k] = (K)(s.lo + pre); else set_status(C, GGMS_E_INTERNAL);
+          k_seg[k] = K_DONE;
         }
       }
       __syncwarp();  // the slice is reloaded by the warp's next segment
@@ -3076,7 +2773,6 @@ __global__ __launch_bounds__(NT) void tiny_select(const InT* __restrict__ src,
                                                  const Counters* __restrict__ C,
                                                  const uint32_t* __restrict__ khead_q,
                                                  const uint32_t* __restrict__ knext,
-                                                 const int64_t* __restrict__ k_off,
                                                  const uint32_t* __restrict__ k_rank, uint32_t* k_seg,
                                                  typename KeyOf<InT>::K* k_key, Caps caps) {
   // Launched right after small_select, whose output it does not read: it lets
@@ -3086,92 +2782,9 @@ __global__ __launch_bounds__(NT) void tiny_select(const InT* __restrict__ src,
   using K = typename KeyOf<InT>::K;
   __shared__ K buf[NT / 32 * tiny_keys<K>()];
   __shared__ uint32_t hist[NT / 32 * 256];
-  tiny_select_body<InT, NT / 32, tiny_keys<K>()>(src, segs_q, tinies, const_cast<Counters*>(C), khead_q, knext, k_off,
+  tiny_select_body<InT, NT / 32, tiny_keys<K>()>(src, segs_q, tinies, const_cast<Counters*>(C), khead_q, knext,
                                                  k_rank, k_seg, k_key, caps, buf, hist, blockIdx.x, gridDim.x);
   pdl_wait();
-}
-
-// ------------------------------------------------------------------ batched segments
-// Level 0 of the batched mode.  A caller segment that holds a k is finished
-// directly from the input when it is small (tiny_select for tiny ones,
-// small_select below QSAMP keys); a larger one gets quantile bins (seg_sample
-// fills its table) and tiles for the level-0 count -- its children then hold
-// about 1/QB of it, mostly a single k each.
-template <typename K>
-__global__ void seg_init(const int64_t* __restrict__ seg_off, uint32_t nseg,
-                         const int64_t* __restrict__ k_off, Seg<K>* segs0, TileRef* tiles0,
-                         uint32_t* khead0, uint32_t* smalls, uint32_t* tinies, uint32_t* bigs0,
-                         uint32_t cap_q, Counters* C, Caps caps) {
-  pdl_entry();
-  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nseg) return;
-  const int64_t a = seg_off[s], b = seg_off[s + 1];
-  Seg<K> d;
-  d.off = (uint64_t)a;
-  d.cnt = (b > a) ? (uint32_t)(b - a) : 0u;
-  d.lo = 0;
-  d.hi = key_max<K>();
-  d.shift = 0u;
-  d.row = SEG_SMALL;
-  d.pad = 0u;
-  khead0[s] = K_NIL;
-  if (b < a) set_status(C, GGMS_E_INVALID_ARG);
-  if (k_off[s + 1] == k_off[s] || d.cnt == 0) {  // nothing to select here: no row, no tiles
-    segs0[s] = d;
-    return;
-  }
-  if (d.cnt <= caps.tiny_keys || d.cnt < QSAMP) {
-    segs0[s] = d;
-    const bool tiny = d.cnt <= caps.tiny_keys;
-    const uint32_t si = atomicAdd(tiny ? &C->ntiny : &C->nsmall, 1u);
-    if (si < caps.segs) (tiny ? tinies : smalls)[si] = s; else set_status(C, GGMS_E_INTERNAL);
-    return;
-  }
-  const uint32_t q = atomicAdd(&C->nbig[0], 1u);  // its quantile table: q
-  if (q >= cap_q) {  // cannot happen: cap_q (<= caps.rows) bounds the segments of QSAMP keys or more
-    set_status(C, GGMS_E_INTERNAL);
-    segs0[s] = d;
-    return;
-  }
-  bigs0[q] = s;
-  d.row = q;
-  d.pad = q;
-  segs0[s] = d;
-  const uint32_t nt = (d.cnt + TILE - 1) / TILE;
-  const uint32_t t0 = atomicAdd(&C->ntiles[0], nt);
-  if (t0 + nt > caps.tiles) { set_status(C, GGMS_E_INTERNAL); return; }
-  for (uint32_t t = 0; t < nt; ++t) tiles0[t0 + t] = TileRef{s, t};
-}
-
-__global__ void seg_set_count(Counters* C, uint32_t nseg) {
-  pdl_entry(); C->nsegs[0] = nseg; }
-
-// k i belongs to the segment s with k_off[s] <= i < k_off[s+1]; the ks of a
-// segment that is finished directly go on its list.
-template <typename K>
-__global__ void k_init_seg(const uint32_t* __restrict__ ks, uint32_t nk,
-                           const int64_t* __restrict__ seg_off, const int64_t* __restrict__ k_off,
-                           uint32_t nseg, const Seg<K>* __restrict__ segs0, uint32_t* khead0,
-                           uint32_t* knext, uint32_t* k_rank, uint32_t* k_seg, Counters* C) {
-  pdl_entry();
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nk) return;
-  uint32_t lo = 0, hi = nseg - 1;  // largest s with k_off[s] <= i
-  while (lo < hi) {
-    uint32_t m = (lo + hi + 1) >> 1;
-    if (k_off[m] <= (int64_t)i) lo = m; else hi = m - 1;
-  }
-  const uint64_t len = (uint64_t)(seg_off[lo + 1] - seg_off[lo]);
-  const uint32_t k = ks[i];
-  if (k < 1u || (uint64_t)k > len) {
-    set_status(C, GGMS_E_INVALID_ARG);
-    k_seg[i] = K_DONE;
-    k_rank[i] = 0;
-    return;
-  }
-  k_rank[i] = (uint32_t)(len - k);
-  k_seg[i] = lo;
-  if (segs0[lo].row == SEG_SMALL) knext[i] = atomicExch(&khead0[lo], i);  // lock-free push
 }
 
 GGMS_END

@@ -48,19 +48,19 @@ int launch_refine(Context* ctx, const RefineArgs<T>& a, cudaStream_t s);
 
 GGMS_BEGIN
 
-// Barrier over the ncta CTAs of a cooperative launch (all resident at once).
-// CTA 0 adds 2^31 - (ncta - 1), the others 1: when all have arrived the top bit
+// Barrier over ncta CTAs of a cooperative launch (all resident at once), one of
+// them the leader.  It adds 2^31 - (ncta - 1), the others 1: when all have arrived the top bit
 // has flipped and the low bits are back where they were, so the word needs no
 // reset between barriers or launches.  In two halves: what the CTA did before
 // arrive() is visible to a CTA after its wait().  The wait is bounded (about
 // two seconds): false for the whole CTA, with the status set, when it ran out.
 struct GridBarrier {
   uint32_t old;  // thread 0's
-  __device__ __forceinline__ void arrive(uint32_t* bar, uint32_t ncta) {
+  __device__ __forceinline__ void arrive(uint32_t* bar, uint32_t ncta, bool leader) {
     __syncthreads();
     if (threadIdx.x == 0 && ncta > 1u) {
       __threadfence();
-      old = atomicAdd(bar, blockIdx.x == 0 ? 0x80000000u - (ncta - 1u) : 1u);
+      old = atomicAdd(bar, leader ? 0x80000000u - (ncta - 1u) : 1u);
     }
   }
   __device__ __forceinline__ bool wait(uint32_t* bar, uint32_t ncta, Counters* C) {
@@ -83,9 +83,9 @@ struct GridBarrier {
   }
 };
 
-__device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t ncta, Counters* C) {
+__device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t ncta, bool leader, Counters* C) {
   GridBarrier b;
-  b.arrive(bar, ncta);
+  b.arrive(bar, ncta, leader);
   return b.wait(bar, ncta, C);
 }
 
@@ -138,18 +138,18 @@ __device__ __forceinline__ bool refine_body(const RefineArgs<T>& a, uint8_t* sme
     const K* src = a.cand[(l - 1) & 1];
     K* dst = a.cand[l & 1];
     prep_body(a.rows[p], a.aflag[p], C, p, a.caps, cta, ncta);
-    if (!grid_barrier(a.bar, ncta, C)) return false;
-    count_body<K, NT>(src, a.segs[p], a.tiles[p], C, p, a.rows[p], a.caps, nullptr, nullptr, bins, cta, ncta);
-    if (!grid_barrier(a.bar, ncta, C)) return false;
+    if (!grid_barrier(a.bar, ncta, cta == 0u, C)) return false;
+    count_body<K, NT>(src, a.segs[p], a.tiles[p], C, p, a.rows[p], a.caps, bins, cta, ncta);
+    if (!grid_barrier(a.bar, ncta, cta == 0u, C)) return false;
     scan_body<NT>(a.rows[p], C, p, a.caps, red, cta, ncta);
-    if (!grid_barrier(a.bar, ncta, C)) return false;
+    if (!grid_barrier(a.bar, ncta, cta == 0u, C)) return false;
     for (uint32_t i = cta * NT + threadIdx.x; i < a.nk; i += ncta * NT)
       locate_in_row(i, a.rows[p], NBIN, a.krank, a.kseg, &a.segs[p]->row, sizeof(Seg<K>) / 4, a.kbin, a.aflag[p],
                     NBIN_WORDS, C, nullptr);
-    if (!grid_barrier(a.bar, ncta, C)) return false;
+    if (!grid_barrier(a.bar, ncta, cta == 0u, C)) return false;
     children_body<K, NT>(a.rows[p], a.aflag[p], a.segs[p], C, p, a.segs[q], a.cursor[q], a.tiles[q], a.points,
-                         a.khead[q], a.smalls, a.tinies, a.bigs[p], a.bigs[q], a.caps, nullptr, cta, ncta);
-    if (!grid_barrier(a.bar, ncta, C)) return false;
+                         a.khead[q], a.smalls, a.tinies, a.bigs[p], a.bigs[q], a.caps, cta, ncta);
+    if (!grid_barrier(a.bar, ncta, cta == 0u, C)) return false;
     for (uint32_t i = cta * NT + threadIdx.x; i < a.nk; i += ncta * NT) {
       const uint32_t s = a.kseg[i];
       if (s != K_DONE)
@@ -157,9 +157,9 @@ __device__ __forceinline__ bool refine_body(const RefineArgs<T>& a, uint8_t* sme
                        a.khead[q], a.knext);
     }
     if (l < MAXLEV)
-      compact_body<K, NT>(src, a.segs[p], a.tiles[p], C, p, a.rows[p], a.segs[q], a.cursor[q], dst, a.caps, nullptr,
-                          nullptr, bins, cta, ncta);
-    if (!grid_barrier(a.bar, ncta, C)) return false;
+      compact_body<K, NT>(src, a.segs[p], a.tiles[p], C, p, a.rows[p], a.segs[q], a.cursor[q], dst, a.caps, bins,
+                          cta, ncta);
+    if (!grid_barrier(a.bar, ncta, cta == 0u, C)) return false;
     if (l < MAXLEV) {
       // children of up to RF_TINY bytes: a warp each, in the space of the CTA
       // finisher (2^28 keys, 2^14 ks: 16 K children of ~500 keys, 260 us at a
@@ -167,13 +167,13 @@ __device__ __forceinline__ bool refine_body(const RefineArgs<T>& a, uint8_t* sme
       constexpr uint32_t TK = RF_TINY / sizeof(K);
       K* slices = reinterpret_cast<K*>(smem);
       if (threadIdx.x < RF_WARPS * 32)
-        tiny_select_body<K, RF_WARPS, TK>(dst, a.segs[q], a.tinies, C, a.khead[q], a.knext, nullptr, a.krank, a.kseg,
+        tiny_select_body<K, RF_WARPS, TK>(dst, a.segs[q], a.tinies, C, a.khead[q], a.knext, a.krank, a.kseg,
                                         a.kkey, a.caps, slices,
                                         reinterpret_cast<uint32_t*>(slices + RF_WARPS * TK), cta, ncta);
       __syncthreads();
-      small_select_body<K, NT>(dst, a.segs[q], a.smalls, C, a.khead[q], a.knext, nullptr, a.krank, a.kseg, a.kkey,
+      small_select_body<K, NT>(dst, a.segs[q], a.smalls, C, a.khead[q], a.knext, a.krank, a.kseg, a.kkey,
                                a.caps.small_keys, a.caps, smem, cta, ncta);
-      if (!grid_barrier(a.bar, ncta, C)) return false;
+      if (!grid_barrier(a.bar, ncta, cta == 0u, C)) return false;
     }
   }
   return true;
