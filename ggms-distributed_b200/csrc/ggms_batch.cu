@@ -41,7 +41,6 @@ int launch_batch(Context* ctx, const BatchArgs<T>& a, cudaStream_t s) {
       a, (uint32_t)ctx->sms);
   if (const int r = launch_rows<T, BT_ROW0>(ctx, a, s)) return r;
   if (const int r = launch_rows<T, BT_ROW0 * 2>(ctx, a, s)) return r;
-  if (const int r = launch_rows<T, BT_ROW0 * 4>(ctx, a, s)) return r;
   batch_sorts<T><<<(unsigned)ctx->sms, DR_NT, sort_smem, s>>>(a);
   GGMS_CU(launch_coop(batch_teams<T>, (unsigned)ctx->sms, DR_NT, team_smem<T>(), s, a));
   // a single's segment has more than direct_cap keys

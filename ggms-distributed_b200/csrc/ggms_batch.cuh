@@ -11,7 +11,7 @@
 //            barriers are CTA barriers), taken from a shared list, longer ones
 //            first, so that the CTAs end together;
 //   sorts    a segment of up to 32 KB: one CTA sorts it;
-//   rows     up to 16 KB: one warp each.
+//   rows     up to 8 KB: one warp each.
 //
 // Children that are still large go to the refinement levels, which write the
 // answers.
@@ -26,9 +26,13 @@
 
 namespace ggms {
 
-// Keys of a segment that one warp finishes (32-bit keys): three classes, whose
-// warps hold 1024, 2048 and 4096 keys.
-constexpr uint32_t BT_ROW0 = 1024;
+// Keys of a segment that one warp finishes (32-bit keys): two classes, whose
+// warps hold 1024 and 2048 keys.  A warp takes 10 to 50 us for such a row and
+// an SM holds 20 or 10 of them; a CTA sort takes 5 to 10 us and has the SM to
+// itself.  So a warp is the better for many rows, and with fewer than
+// BT_FEW rows per SM only for the shortest (126 rows of 900 fp32 keys: 52 us by
+// warps, 8 by CTAs).
+constexpr uint32_t BT_ROW0 = 1024, BT_ROW_FEW = 256, BT_FEW = 4;
 
 template <typename T>
 struct BatchArgs {
@@ -105,8 +109,8 @@ __global__ void batch_init(const __grid_constant__ BatchArgs<T> a, uint32_t ncta
       if (bad) set_status(C, GGMS_E_INVALID_ARG);
       if (g.nk) {
         constexpr uint32_t CAP = direct_cap<typename KeyOf<T>::K>();
-        if (g.cnt <= BT_ROW0 << 2) {
-          cls = BT_WARP + (g.cnt > BT_ROW0) + (g.cnt > BT_ROW0 << 1);
+        if (g.cnt <= (a.nseg < BT_FEW * ncta ? BT_ROW_FEW : BT_ROW0 << 1)) {
+          cls = BT_WARP + (g.cnt > BT_ROW0 ? 1u : 0u);
         } else if (g.cnt <= CAP) {
           cls = BT_SORT;
         } else {
@@ -175,7 +179,7 @@ template <typename T>
 __device__ __noinline__ bool team_vector() {
   extern __shared__ __align__(128) uint8_t smem[];
   const TeamShared<T>& b = *reinterpret_cast<const TeamShared<T>*>(smem + direct_smem<typename KeyOf<T>::K>());
-  return direct_body<T, false>(b.task, b.r, smem);
+  return direct_body<T, false, 2>(b.task, b.r, smem);
 }
 
 // Segments of teams: a cooperative launch of gridDim.x CTAs.  Level l has 2^l
@@ -235,7 +239,7 @@ __global__ __launch_bounds__(DR_NT, 1) void batch_singles(const __grid_constant_
   if (cls == BT_SORT) return;
   if (threadIdx.x == 0) batch_task<T>(a, a.lists[(size_t)cls * a.nseg + j], 0u, 0u, 1u, a.r.bar, task);
   __syncthreads();
-  direct_body<T, true>(task, a.r, smem);
+  direct_body<T, true, 4>(task, a.r, smem);
 }
 
 // Segments of one CTA's sort.
@@ -268,9 +272,10 @@ __global__ __launch_bounds__(DR_NT, 1) void batch_sorts(const __grid_constant__ 
 // by one lane; every k then reads its rank.  The cost does not depend on the
 // number of ks, where a radix select pays four rounds per k (rows of 600 keys
 // with 4-5 ks: 386 us for 12 M keys).  Up to 64 keys: every key's rank by
-// comparison.  A bin that holds many different keys falls back to a bitonic
-// sort of the row.
-constexpr int RW_NT = 160;  // 5 warps: 4, 2 and 1 CTAs per SM by shared memory
+// comparison.
+constexpr int RW_NT = 160;  // 5 warps: 4 and 2 CTAs per SM by shared memory
+constexpr int RW_U = 4;     // keys in flight per lane (a lane's accesses are one long chain otherwise)
+constexpr uint32_t RW_LANE = 24;
 template <typename K, uint32_t ROW>
 struct RowSmem {
   K v[ROW], w[ROW];
@@ -282,7 +287,7 @@ __global__ __launch_bounds__(RW_NT) void rows_select(const __grid_constant__ Bat
   pdl_entry();
   using K = typename KeyOf<T>::K;
   constexpr uint32_t RW_BINS = ROW / 2;
-  constexpr int RW_BITS = ROW == BT_ROW0 ? 9 : ROW == BT_ROW0 << 1 ? 10 : 11;
+  constexpr int RW_BITS = ROW == BT_ROW0 ? 9 : 10;
   constexpr uint32_t CLS = BT_WARP + RW_BITS - 9;
   constexpr bool FP = std::is_floating_point<T>::value;
   constexpr K MID = (K)((K)1 << (sizeof(K) * 8 - 1));
@@ -349,55 +354,73 @@ __global__ __launch_bounds__(RW_NT) void rows_select(const __grid_constant__ Bat
         auto bin = [&](K k) -> uint32_t {
           return FP ? (uint32_t)((K)((min(k, hn) - lo) + (max(k, lp) - lp)) >> sh) : (uint32_t)((K)(k - lo) >> sh);
         };
-        for (uint32_t i = lane; i < cnt; i += 32u) atomicAdd(&sm.h[bin(sm.v[i])], 1u);
+        for (uint32_t i0 = lane; i0 < cnt; i0 += 32u * RW_U) {
+          uint32_t b[RW_U];
+#pragma unroll
+          for (int q = 0; q < RW_U; ++q) b[q] = bin(i0 + q * 32u < cnt ? sm.v[i0 + q * 32u] : lo);
+#pragma unroll
+          for (int q = 0; q < RW_U; ++q)
+            if (i0 + q * 32u < cnt) atomicAdd(&sm.h[b[q]], 1u);
+        }
         __syncwarp();
-        uint32_t run = 0, mx = 0;
+        uint32_t run = 0;
         for (uint32_t b0 = 0; b0 < RW_BINS; b0 += 32u) {
           const uint32_t x = sm.h[b0 + lane];
-          mx = max(mx, x);
           const uint32_t inc = warp_incl_scan_u32(x, lane);
           sm.h[b0 + lane] = run + inc - x;
           run += __shfl_sync(FULL, inc, 31);
         }
         __syncwarp();
-        for (uint32_t i = lane; i < cnt; i += 32u) {
-          const K k = sm.v[i];
-          sm.w[atomicAdd(&sm.h[bin(k)], 1u)] = k;
+        for (uint32_t i0 = lane; i0 < cnt; i0 += 32u * RW_U) {
+          K k[RW_U];
+          uint32_t at[RW_U];
+#pragma unroll
+          for (int q = 0; q < RW_U; ++q) k[q] = i0 + q * 32u < cnt ? sm.v[i0 + q * 32u] : lo;
+#pragma unroll
+          for (int q = 0; q < RW_U; ++q) at[q] = i0 + q * 32u < cnt ? atomicAdd(&sm.h[bin(k[q])], 1u) : 0u;
+#pragma unroll
+          for (int q = 0; q < RW_U; ++q)
+            if (i0 + q * 32u < cnt) sm.w[at[q]] = k[q];
         }
         __syncwarp();
-        // h[b] is now the end of bin b.  One lane per bin: insertion sort; a
-        // bin of over 32 keys is fine when they are all equal
-        bool unsorted = false;
-        for (uint32_t b = lane; b < RW_BINS; b += 32u) {
-          const uint32_t e = sm.h[b], s0 = b ? sm.h[b - 1u] : 0u;
-          if (e - s0 > 32u) {
-            const K x = sm.w[s0];
-            for (uint32_t i = s0 + 1u; i < e && !unsorted; ++i) unsorted = sm.w[i] != x;
-            continue;
-          }
-          for (uint32_t i = s0 + 1u; i < e; ++i) {
-            const K x = sm.w[i];
-            uint32_t p = i;
-            for (; p > s0 && sm.w[p - 1u] > x; --p) sm.w[p] = sm.w[p - 1u];
-            sm.w[p] = x;
-          }
-        }
-        __syncwarp();
-        if (__any_sync(FULL, unsorted)) {
-          uint32_t N = 64;
-          while (N < cnt) N <<= 1;
-          for (uint32_t i = cnt + lane; i < N; i += 32u) sm.w[i] = key_max<K>();
-          __syncwarp();
-          for (uint32_t kk = 2; kk <= N; kk <<= 1)
-            for (uint32_t jj = kk >> 1; jj > 0; jj >>= 1) {
-              for (uint32_t t = lane; t < N / 2; t += 32u) {  // pair t: i has bit jj clear
-                const uint32_t i = ((t & ~(jj - 1u)) << 1) | (t & (jj - 1u));
-                const K x = sm.w[i], y = sm.w[i | jj];
-                if ((x > y) == ((i & kk) == 0)) { sm.w[i] = y; sm.w[i | jj] = x; }
-              }
-              __syncwarp();
+        // h[b] is now the end of bin b.  Bins of up to RW_LANE keys: one lane
+        // each, insertion sort.  Larger ones (a dense spot of the keys): the
+        // warp, one by one, unless all their keys are equal
+        for (uint32_t b0 = 0; b0 < RW_BINS; b0 += 32u) {
+          const uint32_t b = b0 + lane, e = sm.h[b], s0 = b ? sm.h[b - 1u] : 0u;
+          const uint32_t large = __ballot_sync(FULL, e - s0 > RW_LANE);
+          if (e - s0 <= RW_LANE)
+            for (uint32_t i = s0 + 1u; i < e; ++i) {
+              const K x = sm.w[i];
+              uint32_t p = i;
+              for (; p > s0 && sm.w[p - 1u] > x; --p) sm.w[p] = sm.w[p - 1u];
+              sm.w[p] = x;
             }
+          for (uint32_t todo = large; todo; todo &= todo - 1u) {
+            const int src = __ffs(todo) - 1;
+            const uint32_t c0 = __shfl_sync(FULL, s0, src), c1 = __shfl_sync(FULL, e, src), len = c1 - c0;
+            const K x0 = sm.w[c0];
+            bool equal = true;
+            for (uint32_t i = lane; i < len; i += 32u) equal = equal && sm.w[c0 + i] == x0;
+            if (__all_sync(FULL, equal)) continue;
+            uint32_t N = 64;  // bitonic sort in v (the row's copy is no longer needed)
+            while (N < len) N <<= 1;
+            for (uint32_t i = lane; i < N; i += 32u) sm.v[i] = i < len ? sm.w[c0 + i] : key_max<K>();
+            __syncwarp();
+            for (uint32_t kk = 2; kk <= N; kk <<= 1)
+              for (uint32_t jj = kk >> 1; jj > 0; jj >>= 1) {
+                for (uint32_t t = lane; t < N / 2; t += 32u) {  // pair t: i has bit jj clear
+                  const uint32_t i = ((t & ~(jj - 1u)) << 1) | (t & (jj - 1u));
+                  const K x = sm.v[i], y = sm.v[i | jj];
+                  if ((x > y) == ((i & kk) == 0)) { sm.v[i] = y; sm.v[i | jj] = x; }
+                }
+                __syncwarp();
+              }
+            for (uint32_t i = lane; i < len; i += 32u) sm.w[c0 + i] = sm.v[i];
+            __syncwarp();
+          }
         }
+        __syncwarp();
       }
       for (uint32_t i = lane; i < nk; i += 32u) {
         const uint32_t k = a.ks[k0 + i];

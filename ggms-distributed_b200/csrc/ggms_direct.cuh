@@ -43,7 +43,17 @@ constexpr uint32_t DIRECT_MAX_B = 16384;  // buckets
 constexpr uint32_t DIRECT_SAMPLE = 4096;  // sampled keys
 constexpr uint32_t DIRECT_CELLS = 2048;   // cells of the map
 constexpr uint32_t DIRECT_EXT = 16;       // ... of them beyond each extreme of the sample
-constexpr uint32_t DIRECT_WT = 8;         // weight of a sampled key; of a cell beyond the extremes: 1
+constexpr uint32_t DIRECT_GAP = 128;      // ... and on each side of the gap around zero (DirectMap)
+// A cell's weight: WT per sampled key, WT more for its sampled keys or for the
+// mean of its and its four neighbours', whichever is larger, and CELL_WT for
+// having keys at all.  Cells hold a sampled key or six: one that drew none by
+// chance would be a single bucket of 26,000 keys of 2^23, and a set of 300 ks
+// met such a bucket every other time (50 us of levels).  Keys in buckets of
+// more than 8192, 2^24 to 2^25 keys, 16384 buckets: normal 0.08 to 0.7 %
+// without the neighbours, none with them; Cauchy 0.4 to 1.3 %, 0 to 0.04 %;
+// narrow modes keep their buckets, which they lose to a plain smoothing (1.4 %
+// to 15 % of a mixture of eight; 0.9 % with the larger of the two).
+constexpr uint32_t DIRECT_WT = 4, DIRECT_CELL_WT = 4;
 
 template <typename T>
 struct DirectArgs {
@@ -313,9 +323,9 @@ __device__ K* cta_radix(SortSmem<K>& sm, K* A, K* Bf, uint32_t m, int sh0, int s
 // f(key) for every key of CTA cta's share of the input, called by all threads
 // of the CTA.  The 16-byte vectors of the body are split into equal contiguous
 // ranges; CTA 0 also takes the unaligned head and the tail.
-template <typename T, typename F>
+template <typename T, int U, typename F>
 __device__ __forceinline__ void direct_stream(const T* in, uint64_t n, uint32_t cta, uint32_t ncta, F&& f) {
-  constexpr int EPV = Vec16<T>::N, U = 2;
+  constexpr int EPV = Vec16<T>::N;
   const uint32_t tid = threadIdx.x;
   uint64_t head = ((16u - (uint32_t)((uintptr_t)in & 15u)) & 15u) / sizeof(T);
   if (head > n) head = n;
@@ -476,8 +486,8 @@ struct DirectTask {
 // Steps 1 to 5 for one vector.  On return its ks are resolved but for those in
 // large children, which are in pool 1 for the refinement levels, with their
 // true key ranges.  False after a barrier that ran out.  ONE: a single CTA's
-// vector (a.cta == 0, a.ncta == 1).
-template <typename T, bool ONE>
+// vector (a.cta == 0, a.ncta == 1).  U: vectors in flight per thread, twice.
+template <typename T, bool ONE, int U>
 __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const RefineArgs<T>& r, uint8_t* smem) {
   using K = typename KeyOf<T>::K;
   constexpr bool FP = std::is_floating_point<T>::value, K64 = sizeof(K) == 8;
@@ -575,27 +585,47 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
   const K range = (K)((map.hn - map.lo) + (map.hi - map.lp));
   map.csh = (uint32_t)max(0, bitlen(range) - 11);
   static_assert(DIRECT_CELLS == 1u << 11, "cells of 11 bits");
-  if ((range >> map.csh) >= (K)(DIRECT_CELLS - 2 * DIRECT_EXT)) ++map.csh;
+  if ((range >> map.csh) >= (K)(DIRECT_CELLS - 2 * DIRECT_EXT - (two ? 2 * DIRECT_GAP : 0u))) ++map.csh;
   const K ext = a.n > S ? (K)((K)DIRECT_EXT << map.csh) : (K)0;
   map.lo = (K)(map.lo - min(map.lo, ext));
   map.hi = (K)(map.hi + min((K)(dmax - map.hi), ext));
-  if (!two) map.hn = map.lp = map.hi;
+  // ... and likewise for the gap: two sampled keys' worth of values lie in it,
+  // which as one bucket would be a large child (90 us of levels at 2^24 fp32)
+  if (two) {
+    const K half = (K)((map.lp - map.hn) >> 1), g = min((K)((K)DIRECT_GAP << map.csh), half ? (K)(half - 1u) : (K)0);
+    map.hn = (K)(map.hn + (a.n > S ? g : (K)0));
+    map.lp = (K)(map.lp - (a.n > S ? g : (K)0));
+  } else {
+    map.hn = map.lp = map.hi;
+  }
   map.tab = sm.tab;
   auto cell = [&](K k) { return (uint32_t)((K)((min(max(k, map.lo), map.hn) - map.lo) +
                                                (min(max(k, map.lp), map.hi) - map.lp)) >> map.csh); };
-  const uint32_t c_lo = cell(dom(lo)), c_hi = cell(dom(hi)), c_end = cell(map.hi);
+  const uint32_t c_end = cell(map.hi);
 #pragma unroll
   for (int j = 0; j < (int)(DIRECT_SAMPLE / DR_NT); ++j)
-    if (tid + j * DR_NT < S) atomicAdd(&sm.I[cell(dom(sv[j]))], DIRECT_WT);
-  // the cells beyond the extremes weigh a sampled key or two at each end
-  for (uint32_t c = tid; c < c_lo; c += DR_NT) atomicAdd(&sm.I[c], 1u);
-  for (uint32_t c = c_hi + 1u + tid; c <= c_end; c += DR_NT) atomicAdd(&sm.I[c], 1u);
+    if (tid + j * DR_NT < S) atomicAdd(&sm.I[cell(dom(sv[j]))], 1u);
   __syncthreads();
   static_assert(DIRECT_CELLS == 2 * DR_NT, "two cells per thread");
-  uint32_t w2[2] = {sm.I[2 * tid], sm.I[2 * tid + 1]};
+  uint32_t w2[2], raw[2];  // this thread's cells: weights, sampled keys
+  {
+    uint32_t near[6];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+      const uint32_t c = 2 * tid + i - 2u;  // (wraps below 0)
+      near[i] = c < DIRECT_CELLS ? sm.I[c] : 0u;
+    }
+    raw[0] = near[2];
+    raw[1] = near[3];
+    const uint32_t mid = near[1] + near[2] + near[3] + near[4];
+    w2[0] = DIRECT_WT * (raw[0] + max(raw[0], (mid + near[0]) / 5u)) + DIRECT_CELL_WT;
+    w2[1] = DIRECT_WT * (raw[1] + max(raw[1], (mid + near[5]) / 5u)) + DIRECT_CELL_WT;
+    if (2 * tid > c_end) w2[0] = 0u;
+    if (2 * tid + 1 > c_end) w2[1] = 0u;
+  }
   const uint32_t own0 = w2[0], own1 = w2[1];
   block_scan_regs<2>(w2, red);
-  uint32_t W = 0, hot = 0;  // all weights, about DIRECT_WT * S; of the cells that can hold a k (0: no focus)
+  uint32_t hot = 0;  // the weight of the cells that can hold a k (0: no focus)
   uint32_t nfirst = w2[0] - own0;  // packed prefix before this thread's cells: hot | other << 16
   bool focus = false;
   if (a.focus) {
@@ -607,14 +637,14 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
       if (rank != NONE) occ |= 1ull << (uint32_t)(((uint64_t)rank * 64u) / a.n);
     }
     const uint32_t o0 = __reduce_or_sync(FULL, (uint32_t)occ), o1 = __reduce_or_sync(FULL, (uint32_t)(occ >> 32));
-    sm.I[2 * tid] = w2[0];
-    sm.I[2 * tid + 1] = w2[1];
+    block_scan_regs<2>(raw, red);  // I: inclusive counts of the sampled keys
+    sm.I[2 * tid] = raw[0];
+    sm.I[2 * tid + 1] = raw[1];
     if (lane == 0) {
       red[warp] = o0;
       red[32 + warp] = o1;
     }
     __syncthreads();
-    W = sm.I[DIRECT_CELLS - 1u];
     focus = __popc(__reduce_or_sync(FULL, red[lane])) + __popc(__reduce_or_sync(FULL, red[32 + lane])) <= 16;
     __syncthreads();
   }
@@ -628,17 +658,16 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
       const float q = ((float)rank + 0.5f) / (float)a.n;
       const float pos = q * (float)S, m = 6.0f * sqrtf((float)S * q * fmaxf(1.0f - q, 0.0f)) + 8.0f;
       const uint32_t p0 = min((uint32_t)fmaxf(pos - m, 0.0f), S - 1u), p1 = (uint32_t)(pos + m) + 1u;
-      auto cell_of = [&](uint32_t w) {  // the cell that holds the w-th part of the weight
-        uint32_t l = 0, h = DIRECT_CELLS - 1u;
+      auto cell_of = [&](uint32_t p) {  // the cell of the p-th sampled key
+        uint32_t l = 0, h = c_end;
         while (l < h) {
           const uint32_t mid = (l + h) >> 1;
-          if (sm.I[mid] > w) h = mid; else l = mid + 1u;
+          if (sm.I[mid] > p) h = mid; else l = mid + 1u;
         }
         return l;
       };
-      // (the low end's extra cells shift the weights by c_lo)
-      const uint32_t c0 = p0 ? cell_of(min(p0 * DIRECT_WT + c_lo, W - 1u)) : 0u;
-      const uint32_t c1 = p1 < S ? cell_of(min(p1 * DIRECT_WT + c_lo, W - 1u)) : c_end;
+      const uint32_t c0 = p0 ? cell_of(p0) : 0u;
+      const uint32_t c1 = p1 < S ? cell_of(p1) : c_end;
       atomicAdd(&sm.hist[c0], 1u);
       if (c1 + 1u < DIRECT_CELLS) atomicAdd(&sm.hist[c1 + 1u], NONE);
     }
@@ -648,7 +677,7 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
     sm.hist[2 * tid] = 0u;
     sm.hist[2 * tid + 1] = 0u;
     // the weight of hot cells in the low half, of the others in the high half
-    static_assert(DIRECT_WT * DIRECT_SAMPLE + 2 * DIRECT_EXT < 65536u, "weights of 16 bits");
+    static_assert(3 * DIRECT_WT * DIRECT_SAMPLE + DIRECT_CELL_WT * DIRECT_CELLS < 65536u, "weights of 16 bits");
     w2[0] = own0 << (d2[0] ? 0 : 16);
     w2[1] = own1 << (d2[1] ? 0 : 16);
     nfirst = w2[0];
@@ -657,7 +686,7 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
   }
   if (tid == DR_NT - 1) red[70] = w2[1];
   __syncthreads();
-  W = (red[70] & 0xFFFFu) + (red[70] >> 16);
+  const uint32_t W = (red[70] & 0xFFFFu) + (red[70] >> 16);
   if (focus) hot = red[70] & 0xFFFFu;
   // first bucket of a cell with (packed) weight prefix p: 7/8 of the buckets
   // over the hot cells and 1/8 over the others, or all evenly
@@ -694,7 +723,7 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
   GGMS_TRACE(1);
   // ---- count
   with_map([&](const auto& m) {
-    direct_stream<T>(a.in, a.n, cta, ncta, [&](K key) { atomicAdd(&sm.hist[m(key)], 1u); });
+    direct_stream<T, U>(a.in, a.n, cta, ncta, [&](K key) { atomicAdd(&sm.hist[m(key)], 1u); });
   });
   GGMS_TRACE(2);
   if (a.focus) __syncthreads();
@@ -802,7 +831,7 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
   // ---- copy
   with_map([&](const auto& m) {
     K* cand = r.cand[0] + a.off;
-    direct_stream<T>(a.in, a.n, cta, ncta, [&](K key) {
+    direct_stream<T, U>(a.in, a.n, cta, ncta, [&](K key) {
       const uint32_t b = m(key);
       if (active(b)) cand[atomicAdd(&sm.hist[b], 1u)] = key;
     });
@@ -949,7 +978,7 @@ __global__ __launch_bounds__(DR_NT, 1) void direct_select(const __grid_constant_
   t.ncta = ncta;
   t.off = 0;
   t.k0 = 0;
-  if (!direct_body<T, false>(t, r, smem)) return;
+  if (!direct_body<T, false, 4>(t, r, smem)) return;
   if (__ldcg(&C->nbig[1]) && (!refine_body<T, DR_NT>(r, smem) || !grid_barrier(r.bar, ncta, cta == 0u, C))) return;
   write_out_body<T>(r.kkey, r.kseg, r.nk, r.out, C, cta, ncta);
   report_body(C, r.report, ncta);

@@ -385,13 +385,19 @@ static int sort_cluster_ctas(uint32_t S) {
 
 // The one-launch path (ggms_direct.cuh) takes calls that leave everything to
 // the library: AUTO with no tuning field set, no statistics and no profiling
-// (those describe the two-pass pipeline), on a vector of up to
-// DIRECT_MAX_BYTES.  The lines below, and where they lie (us per call, one
-// launch / pipeline, B200, device ks and answers, normal values):
-//   bytes: the second read has to come from L2 (126 MB).  2^24 fp32: 90 / 189
-//     for 5 random ks, 154 / 260 for 1000, 132 / 164 for 1000 in the top 1 %;
-//     2^24 fp64 (128 MB): 175 / 285, 231 / 396, 190 / 244; 2^26 fp32 (256 MB):
-//     229 / 335, 401 / 472, but 295 / 238 and 1895 / 1230 for 2^14 random ks.
+// (those describe the two-pass pipeline).  The lines below, and where they lie
+// (us per call, one launch / pipeline, B200, device ks and answers):
+//   bytes: the second read comes from L2 (126 MB) up to 2^24 fp32: 80 / 189
+//     for 5 random ks, 86 / 165 for 1000 in the top 1 %.  At 128 MB fp32 it is
+//     138 / 241 for 8 random ks, at 160 MB 164 / 265, at 280 MB 331 / 360, and
+//     242 / 233 for 300 in the top 1 %.
+//   keys: what the buckets of the ks hold is copied and sorted whole, and
+//     16384 buckets over more keys hold more each, where the pipeline has a
+//     bucket per k or more.  The mixture of eight narrow modes is the worst:
+//     300 ks 343 / 349 at 40 M keys; 1000 ks 262 / 287 at 16 M, 334 / 312 at
+//     24 M; 4000 ks 261 / 389 at 8 M, 378 / 457 at 16 M fp32 but 733 / 651
+//     fp64.  Top-k, one cluster of ks, has no such limit: 146 / 224 for 2^13
+//     of 2^25.
 //   ks: every k costs each CTA a search up to DIRECT_SLICE_KS; beyond, each CTA
 //     searches its own (one more barrier): 2^14 ks took 50 us of searching
 //     without it, 10 with it.  DIRECT_MAX_KS is the largest count measured.
@@ -401,6 +407,8 @@ static int sort_cluster_ctas(uint32_t S) {
 //   focus (most buckets to clustered ks): costs 3 us of the map, saves 25 of
 //     the copy and sort at 2^22 and 100 at 2^24 with 1000 ks in the top 1 %.
 constexpr uint64_t DIRECT_MAX_BYTES = 160ull << 20;
+constexpr uint64_t DIRECT_SOME_KS = 512, DIRECT_MANY_KS = 2048;  // more than so many ks: up to ..
+constexpr uint64_t DIRECT_SOME_N = 20u << 20, DIRECT_MANY_N = 12u << 20;  // .. so many keys
 constexpr uint32_t DIRECT_MAX_KS = 65536;
 constexpr uint64_t DIRECT_CTA_KEYS = 1024;    // keys that repay another CTA
 constexpr uint64_t DIRECT_BUCKET_KEYS = 8;
@@ -409,8 +417,9 @@ constexpr uint64_t DIRECT_FOCUS_N = 1u << 18;
 constexpr uint32_t DIRECT_FOCUS_KS = 16;
 constexpr uint32_t DIRECT_SLICE_KS = 2048;
 
-static bool direct_ok(const Context* ctx, const ggms_opts& o, uint64_t n, uint64_t nk, size_t elem) {
-  return n * elem <= DIRECT_MAX_BYTES && nk <= DIRECT_MAX_KS && !ctx->profile && !o.stats && !o.autotune &&
+static bool direct_ok(const Context* ctx, const ggms_opts& o, uint64_t n, uint64_t nk, size_t elem, bool topk) {
+  const uint64_t max_n = nk > DIRECT_MANY_KS ? DIRECT_MANY_N : nk > DIRECT_SOME_KS ? DIRECT_SOME_N : ~0ull;
+  return n * elem <= DIRECT_MAX_BYTES && (topk || n <= max_n) && nk <= DIRECT_MAX_KS && !ctx->profile && !o.stats && !o.autotune &&
          o.assigner == GGMS_ASSIGNER_AUTO && !o.num_buckets && !o.sample_size && o.train_steps <= 0 &&
          !o.pass_threads && !o.pass_unroll && o.window_z == 0.0f && !o.pl_knots;
 }
@@ -495,7 +504,7 @@ static int run_single(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
     for (uint32_t i = 0; i < nk; ++i)
       if (ks[i] < 1u || (uint64_t)ks[i] > n) return GGMS_E_INVALID_ARG;
   }
-  if (direct_ok(ctx, o, n, nk, sizeof(T))) return run_direct<T>(ctx, d_in, n, ks, nk, out, o, st, topk);
+  if (direct_ok(ctx, o, n, nk, sizeof(T), topk)) return run_direct<T>(ctx, d_in, n, ks, nk, out, o, st, topk);
   Plan p;
   int rc = make_plan(&p, n, nk, o);
   if (rc) return rc;
