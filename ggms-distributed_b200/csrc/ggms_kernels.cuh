@@ -11,9 +11,10 @@
 //                 become refinement segments
 //   l0_relabel    ks follow their bucket
 //   l0_compact    PASS 2 over the input: copy the keys of refinement segments
-//   lvl_* (x L)   the same steps over candidates only, with radix bins of
-//                 11 key bits, until every k sits in a single-key bin
-//   write_out     answers (as the caller's type) in the caller's k order
+//   refine_levels the same steps over candidates only (the *_body functions
+//                 below, in one cooperative launch: ggms_refine.cuh), with
+//                 radix bins of 11 key bits, until every k sits in a single-key
+//                 bin; then the answers in the caller's k order
 //
 // Reference steps these replace (DistributedSMOS/bucketMultiselect.cu):
 //   minmax (:543-547) -- not needed: the assigner has open tail buckets;
@@ -22,7 +23,7 @@
 //   sumCounts (:219-226) -> l0_scan;  findKBuckets (:92-116, host) -> l0_locate;
 //   unique buckets + reindexCounts (:726-768, host + kernel) -> l0_children;
 //   copyElements (:254-313) -> l0_compact;  thrust::sort + copyValuesInChunk
-//   (:814-833) -> the refinement levels + write_out.
+//   (:814-833) -> refine_levels.
 // IterativeSMOS (DistributedSMOS/iterativeSMOS.cu:1348-1531) repeats
 // bucketing over the survivors with re-fitted pivots; here the survivors are
 // refined with exact radix bins of the known key range, which ends in a bounded
@@ -1529,7 +1530,7 @@ __global__ void l0_bases(uint32_t* crow, uint32_t B, uint32_t ncta, const Seg<K>
   bases_body<K>(crow, B, ncta, segs1, C, caps);
 }
 
-// After l0_children: the ks follow their level-0 child (lvl_relabel) and the
+// After l0_children: the ks follow their level-0 child (relabel_one) and the
 // per-CTA write cursors of PASS 2 are formed (l0_bases), in one launch --
 // threads [0, nk) relabel, all warps then take children for the cursors.
 template <typename K>
@@ -2148,7 +2149,8 @@ __device__ __forceinline__ void count_body(const K* src, const Seg<K>* segs, con
   uint32_t open = 0xFFFFFFFFu;  // segment whose counts the shared histogram holds
   uint32_t open_row = 0;
   unsigned long long open_keys = 0;
-  auto flush = [&]() {  // all threads, after a barrier
+  auto flush = [&]() {  // all threads
+    __syncthreads();
     uint32_t* row = rows + (size_t)open_row * NBIN;
     for (uint32_t i = threadIdx.x; i < NBIN; i += NT) {
       const uint32_t v = h[i];
@@ -2160,7 +2162,7 @@ __device__ __forceinline__ void count_body(const K* src, const Seg<K>* segs, con
     const TileRef tr = tiles[t];
     if (tr.seg >= ns) continue;  // only after a capacity error (status already set)
     const Seg<K> s = segs[tr.seg];
-    if (tr.seg != open) {  // the previous tile ended with a barrier
+    if (tr.seg != open) {  // (no barrier between a segment's tiles: the warps run on into the next one's loads)
       if (open != 0xFFFFFFFFu) {
         flush();
         __syncthreads();
@@ -2180,9 +2182,8 @@ __device__ __forceinline__ void count_body(const K* src, const Seg<K>* segs, con
           atomicAdd(&h[min((uint32_t)((K)(k[t] - s.lo) >> s.shift), (uint32_t)NBIN - 1u)], 1u);
     });
     open_keys += end - beg;
-    __syncthreads();
   }
-  if (open != 0xFFFFFFFFu) flush();  // the last tile ended with a barrier
+  if (open != 0xFFFFFFFFu) flush();
 }
 
 // w: 72 words of shared memory
@@ -2306,12 +2307,13 @@ __device__ __forceinline__ void compact_body(const K* src, const Seg<K>* segs, c
     const TileRef tr = tiles[t];
     if (tr.seg >= ns) continue;  // only after a capacity error (status already set)
     const Seg<K> s = segs[tr.seg];
-    if (tr.seg != loaded) {  // the previous tile ended with a barrier
+    if (tr.seg != loaded) {
       const uint32_t* row = rows + (size_t)s.row * NBIN;
+      __syncthreads();
       for (uint32_t i = threadIdx.x; i < NBIN; i += NT) cm[i] = row[i];
       loaded = tr.seg;
+      __syncthreads();
     }
-    __syncthreads();
     const uint64_t beg = s.off + (uint64_t)tr.no * TILE;
     const uint64_t end = min(beg + TILE, s.off + s.cnt);
     tile_stream<K, NT>(src, beg, end, [&](const K* k, uint32_t mask) {
@@ -2353,7 +2355,6 @@ __device__ __forceinline__ void compact_body(const K* src, const Seg<K>* segs, c
         }
       }
     });
-    __syncthreads();
   }
   __syncwarp();
   if (lane < qn) emit((1u << qn) - 1u, qk[lane], qc[lane]);  // qn < 32

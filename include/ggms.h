@@ -49,7 +49,8 @@ enum {
 
 /* ---- level-0 bucket assigners ---- */
 enum {
-  GGMS_ASSIGNER_AUTO = 0,        /* learned PL-CDF, sampled pivots if its imbalance is over the bound */
+  GGMS_ASSIGNER_AUTO = 0,        /* learned PL-CDF, sampled pivots if its imbalance is over the bound; vectors
+                                    of up to 160 MB with no other field set: one launch, sampled cells */
   GGMS_ASSIGNER_SAMPLED = 1,     /* sampled pivots + per-segment slopes (the reference's method) */
   GGMS_ASSIGNER_LEARNED_PL = 2,  /* monotone piecewise-linear CDF, trained on the GPU */
   GGMS_ASSIGNER_LEARNED_MLP = 3  /* monotone 1-32-32-1 MLP CDF, trained on the GPU */
@@ -60,8 +61,9 @@ typedef struct ggms_stats {
   int32_t assigner_used;        /* GGMS_ASSIGNER_* that produced the level-0 buckets */
   int32_t num_buckets;          /* level-0 buckets */
   int32_t full_passes;          /* launches that read the whole input, counted by those kernels on the
-                                   device: 2 on the single-vector path (PASS 1 and PASS 2); on the
-                                   batched path the level-0 count and copy when a segment needs them */
+                                   device: 2 on the single-vector path (PASS 1 and PASS 2; a request for
+                                   statistics takes that path); on the batched path 2 (the count and the
+                                   copy) when a segment is longer than one CTA's sort */
   int32_t levels;               /* refinement levels that ran over candidates */
   int64_t candidates;           /* elements the level-0 compaction copied */
   int64_t refine_elements;      /* elements read by all refinement levels together */
@@ -98,7 +100,7 @@ typedef struct ggms_opts {
                                    binomial standard deviations; 0 = 6; < 0 = no windows */
   int32_t autotune;             /* 1: when num_buckets and the pass shape are left at 0, the first call of a
                                    shape class times the candidates on the caller's data and the context
-                                   keeps the fastest (the batched path tunes its level kernels' CTAs) */
+                                   keeps the fastest (the batched path has nothing to tune) */
   ggms_stats* stats;            /* optional host pointer */
   int32_t pl_knots;             /* segments of the learned piecewise-linear CDF model: 16..1024;
                                    0 = auto (PL: min(512, num_buckets / 4); MLP: min(1024,
