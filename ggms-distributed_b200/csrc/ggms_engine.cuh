@@ -26,7 +26,6 @@ GGMS_BEGIN
 template <typename K>
 struct Workspace {
   Counters* C;
-  uint32_t* kin;
   uint32_t* krank;
   uint32_t* kseg;
   uint32_t* kbin;
@@ -69,7 +68,6 @@ static Workspace<K> layout(const Plan& p, uint8_t* base) {
   static_assert(sizeof(Counters) <= ARENA_BAR, "the barrier word follows the counters");
   size_t o_C = b.take(sizeof(Counters));
   b.take(ARENA_BAR_BYTES);
-  size_t o_kin = b.take(4ull * p.nk);
   size_t o_krank = b.take(4ull * p.nk);
   size_t o_kseg = b.take(4ull * p.nk);
   size_t o_kbin = b.take(4ull * p.nk);
@@ -107,7 +105,6 @@ static Workspace<K> layout(const Plan& p, uint8_t* base) {
   w.bytes = b.take(0) + 256;
   if (!base) return w;
   w.C = (Counters*)(base + o_C);
-  w.kin = (uint32_t*)(base + o_kin);
   w.krank = (uint32_t*)(base + o_krank);
   w.kseg = (uint32_t*)(base + o_kseg);
   w.kbin = (uint32_t*)(base + o_kbin);
