@@ -260,6 +260,16 @@ int64_t ggms_context_graph_launches(ggms_context* ctx) {
   return c->graph_launches;
 }
 
+int ggms_diag_pinned_layout(int64_t nk, int elem, int host_k, int host_out, int64_t* out) {
+  if (nk < 0 || elem <= 0 || !out) return GGMS_E_INVALID_ARG;
+  const PinLayout l = pin_layout((uint64_t)nk, (size_t)elem, host_k != 0, host_out != 0);
+  out[0] = (int64_t)sizeof(Counters);
+  out[1] = (int64_t)l.ks;
+  out[2] = (int64_t)l.out;
+  out[3] = (int64_t)l.bytes;
+  return GGMS_OK;
+}
+
 int ggms_diag_pl_gradient(const uint32_t* keys, int S, const float* theta, float* loss, float* grad,
                           uint32_t* knots, int* M) {
   return diag::pl_gradient(keys, S, theta, loss, grad, knots, M);

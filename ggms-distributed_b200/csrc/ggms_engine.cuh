@@ -437,12 +437,12 @@ static int run_direct(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
   if (rc) return rc;
   const Workspace<K> w = layout<K>(p, ctx->arena);
   const bool host_k = !o.ks_on_device && !topk, host_out = !o.out_on_device;
-  const size_t k_bytes = host_k ? ((4ull * nk + 63) & ~(size_t)63) : 0;
-  rc = ensure_pinned(ctx, sizeof(Counters) + 64 + k_bytes + (host_out ? sizeof(T) * nk : 0) + 64);
+  const PinLayout pl = pin_layout(nk, sizeof(T), host_k, host_out);
+  rc = ensure_pinned(ctx, pl.bytes);
   if (rc) return rc;
   Counters* pin_C = (Counters*)ctx->pinned;
-  uint8_t* pin_k = ctx->pinned + ((sizeof(Counters) + 63) & ~(size_t)63);
-  T* pin_out = (T*)(pin_k + k_bytes);
+  uint8_t* pin_k = ctx->pinned + pl.ks;
+  T* pin_out = (T*)(ctx->pinned + pl.out);
   if (host_k) {
     if (ctx->pin_busy) GGMS_CU(cudaEventSynchronize(ctx->pin_busy));
     memcpy(pin_k, ks, 4ull * nk);
@@ -517,13 +517,12 @@ static int run_single(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
   if (rc) return rc;
   Workspace<K> w = layout<K>(p, ctx->arena);
   const bool host_k = !o.ks_on_device && !topk, host_out = !o.out_on_device;
-  const size_t pin_bytes = (host_k ? 4ull * nk : 0) + (host_out ? sizeof(T) * nk : 0) + sizeof(Counters) + 64;
-  rc = ensure_pinned(ctx, pin_bytes);
+  const PinLayout pl = pin_layout(nk, sizeof(T), host_k, host_out);
+  rc = ensure_pinned(ctx, pl.bytes);
   if (rc) return rc;
-  uint8_t* pin = ctx->pinned;
-  Counters* pin_C = (Counters*)pin;
-  uint8_t* pin_k = pin + ((sizeof(Counters) + 63) & ~(size_t)63);
-  uint8_t* pin_out = pin_k + (host_k ? ((4ull * nk + 63) & ~(size_t)63) : 0);
+  Counters* pin_C = (Counters*)ctx->pinned;
+  uint8_t* pin_k = ctx->pinned + pl.ks;
+  uint8_t* pin_out = ctx->pinned + pl.out;
 
   const Caps caps{p.cap_seg, p.cap_tiles, p.nk, (uint32_t)(SMALL_SMEM / sizeof(K)), 0u, p.cap_rows};
   if (host_k && !topk) {

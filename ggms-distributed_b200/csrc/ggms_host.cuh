@@ -117,6 +117,22 @@ static int ensure_pinned(Context* c, size_t bytes) {
   return GGMS_OK;
 }
 
+// The pinned buffer of one call: the counters, the ks and the answers, each
+// from a 64-byte boundary.  The kernels read the ks and store the answers
+// there, so `bytes` is what ensure_pinned has to be asked for.
+struct PinLayout {
+  size_t ks, out, bytes;
+};
+
+static PinLayout pin_layout(uint64_t nk, size_t elem, bool host_k, bool host_out) {
+  auto up = [](size_t b) { return (b + 63) & ~(size_t)63; };
+  PinLayout l;
+  l.ks = up(sizeof(Counters));
+  l.out = l.ks + (host_k ? up(4ull * nk) : 0);
+  l.bytes = l.out + (host_out ? elem * nk : 0);
+  return l;
+}
+
 static int create_context(Context** out, int device) {
   Context* c = new (std::nothrow) Context();
   if (!c) return GGMS_E_OOM;

@@ -1,9 +1,10 @@
-/* ggms_diag.h -- diagnostic entry points of the learned bucket assigners.
+/* ggms_diag.h -- diagnostic entry points.
  *
- * No reference counterpart (the reference has no learned component).  They
- * expose the GPU forward/backward kernels of the two CDF models so that their
- * gradients can be checked against a CPU restatement; they allocate and free
- * their own device memory and synchronize.  Not for the hot path.
+ * No reference counterpart (the reference has no learned component and no
+ * workspace of its own).  Those of the learned bucket assigners expose the GPU
+ * forward/backward kernels of the two CDF models so that their gradients can
+ * be checked against a CPU restatement; they allocate and free their own
+ * device memory and synchronize.  Not for the hot path.
  */
 #ifndef GGMS_DIAG_H
 #define GGMS_DIAG_H
@@ -37,6 +38,12 @@ GGMS_API int ggms_diag_mlp_gradient(const float* x, const float* t, const float*
 GGMS_API int ggms_diag_fit(const uint32_t* sorted_keys, int S, int kind, int steps,
                            float* loss_before, float* loss_after, float* imbalance_model,
                            float* imbalance_sampled);
+
+/* Layout of the pinned buffer of a call with nk ks and answers of `elem`
+ * bytes, in bytes: out[0] the counters (from 0), out[1] where the host ks are
+ * copied, out[2] where the answers arrive, out[3] the buffer's size.  Host
+ * arithmetic only: no CUDA call. */
+GGMS_API int ggms_diag_pinned_layout(int64_t nk, int elem, int host_k, int host_out, int64_t* out);
 
 #ifdef __cplusplus
 }
