@@ -260,6 +260,14 @@ int64_t ggms_context_graph_launches(ggms_context* ctx) {
   return c->graph_launches;
 }
 
+int ggms_diag_barrier_limit(ggms_context* ctx, int64_t cycles) {
+  Context* c = (Context*)ctx;
+  if (!c) return GGMS_E_INVALID_ARG;
+  std::lock_guard<std::mutex> lk(c->mu);
+  c->barrier_limit = (long long)cycles;
+  return GGMS_OK;
+}
+
 int ggms_diag_pinned_layout(int64_t nk, int elem, int host_k, int host_out, int64_t* out) {
   if (nk < 0 || elem <= 0 || !out) return GGMS_E_INVALID_ARG;
   const PinLayout l = pin_layout((uint64_t)nk, (size_t)elem, host_k != 0, host_out != 0);

@@ -629,7 +629,7 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
   uint32_t nfirst = w2[0] - own0;  // packed prefix before this thread's cells: hot | other << 16
   bool focus = false;
   if (a.focus) {
-    if (!zeroed.wait(a.bar, ncta, r.C)) return false;
+    if (!zeroed.wait(a.bar, ncta, r.C, r.limit)) return false;
     // clustered ks: their ranks occupy at most a quarter of 64 equal ranges
     unsigned long long occ = 0;
     for (uint32_t i = tid; i < nk; i += DR_NT) {
@@ -727,13 +727,13 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
   });
   GGMS_TRACE(2);
   if (a.focus) __syncthreads();
-  else if (!zeroed.wait(a.bar, ncta, r.C)) return false;  // (a CTA barrier too)
+  else if (!zeroed.wait(a.bar, ncta, r.C, r.limit)) return false;  // (a CTA barrier too)
   if (ncta > 1u)
     for (uint32_t i = tid; i < B; i += DR_NT) {
       const uint32_t v = sm.hist[i];
       if (v) atomicAdd(&a.ghist[i], v);
     }
-  if (!grid_barrier(a.bar, ncta, cta == 0u, r.C)) return false;
+  if (!grid_barrier(a.bar, ncta, cta == 0u, r.C, r.limit)) return false;
 
   GGMS_TRACE(3);
   // ---- scan, locate
@@ -772,7 +772,7 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
       const uint32_t b = bucket_of(rank);
       atomicOr(&a.gact[b >> 5], 1u << (b & 31));
     }
-    if (!grid_barrier(a.bar, ncta, cta == 0u, r.C)) return false;
+    if (!grid_barrier(a.bar, ncta, cta == 0u, r.C, r.limit)) return false;
     for (uint32_t w = tid; w < B / 32; w += DR_NT) sm.act[w] = __ldcg(&a.gact[w]);
   }
   __syncthreads();
@@ -837,7 +837,7 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
     });
   });
   GGMS_TRACE(6);
-  if (!grid_barrier(a.bar, ncta, cta == 0u, r.C)) return false;
+  if (!grid_barrier(a.bar, ncta, cta == 0u, r.C, r.limit)) return false;
   GGMS_TRACE(7);
   GGMS_TRACE_CTA(0);
 
@@ -913,7 +913,7 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
   }
   GGMS_TRACE(8);
   GGMS_TRACE_CTA(1);
-  if (!grid_barrier(a.bar, ncta, cta == 0u, r.C)) return false;
+  if (!grid_barrier(a.bar, ncta, cta == 0u, r.C, r.limit)) return false;
   GGMS_TRACE(9);
   // ks of the sorted children (the barrier makes every child's order visible)
   for (uint32_t i = gt; i < nk; i += gs) {
@@ -945,7 +945,7 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
         key_atomic_max(&r.segs[1][id].hi, mx);
       }
     }
-  if (!grid_barrier(a.bar, ncta, cta == 0u, r.C)) return false;
+  if (!grid_barrier(a.bar, ncta, cta == 0u, r.C, r.limit)) return false;
   for (uint32_t j = first_big + gt; j < min(first_big + nbig, min(r.caps.rows, r.caps.segs)); j += gs) {
     Seg<K>& s = r.segs[1][j];
     s.shift = (uint32_t)max(0, bitlen((K)(__ldcg(&s.hi) - __ldcg(&s.lo))) - RADIX_BITS);
@@ -978,10 +978,11 @@ __global__ __launch_bounds__(DR_NT, 1) void direct_select(const __grid_constant_
   t.ncta = ncta;
   t.off = 0;
   t.k0 = 0;
-  if (!direct_body<T, false, 4>(t, r, smem)) return;
-  if (__ldcg(&C->nbig[1]) && (!refine_body<T, DR_NT>(r, smem) || !grid_barrier(r.bar, ncta, cta == 0u, C))) return;
-  write_out_body<T>(r.kkey, r.kseg, r.nk, r.out, C, cta, ncta);
-  report_body(C, r.report, ncta);
+  bool good = direct_body<T, false, 4>(t, r, smem);
+  if (good && __ldcg(&C->nbig[1]))
+    good = refine_body<T, DR_NT>(r, smem) && grid_barrier(r.bar, ncta, cta == 0u, C, r.limit);
+  if (good) write_out_body<T>(r.kkey, r.kseg, r.nk, r.out, C, cta, ncta);
+  leave_body(C, r.left, r.report, ncta);
   GGMS_TRACE(10);
 }
 

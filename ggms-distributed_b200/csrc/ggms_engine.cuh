@@ -150,6 +150,8 @@ static RefineArgs<T> refine_args(const Workspace<typename KeyOf<T>::K>& w, const
   RefineArgs<T> a;
   a.C = w.C;
   a.bar = (uint32_t*)(c->arena + ARENA_BAR);
+  a.left = a.bar + ARENA_BAR_BYTES / 4 - 1;
+  a.limit = barrier_limit(c);
   for (int i = 0; i < 2; ++i) {
     a.cand[i] = w.cand[i];
     a.segs[i] = w.segs[i];
@@ -468,7 +470,8 @@ static int run_direct(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
                               (std::is_floating_point<T>::value ? 32u : 0u),
                           (uint64_t)(uintptr_t)d_in, n, host_k ? 1ull : (uint64_t)(uintptr_t)ks, nk,
                           host_out ? 1ull : (uint64_t)(uintptr_t)out, p.seed, (uint64_t)(uintptr_t)ctx->arena,
-                          (uint64_t)(uintptr_t)ctx->pinned};
+                          (uint64_t)(uintptr_t)ctx->pinned, (uint64_t)barrier_limit(ctx)};
+  if (host_out) pin_C->status = GGMS_E_INTERNAL;  // until the launch reports
   rc = run_graphed(ctx, key, (int)(sizeof(key) / sizeof(key[0])), st, enqueue);
   if (rc) return rc;
   rc = mark_done(ctx, st);
@@ -481,7 +484,7 @@ static int run_direct(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
     return GGMS_OK;
   }
   GGMS_CU(cudaStreamSynchronize(st));
-  memcpy(out, pin_out, sizeof(T) * nk);
+  if (pin_C->status != GGMS_E_INTERNAL) memcpy(out, pin_out, sizeof(T) * nk);
   return (int)pin_C->status;
 }
 
@@ -659,6 +662,7 @@ static int run_single(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
     prof_rec(prof, 5, s);
     return GGMS_OK;
   };
+  if (host_out || o.stats) pin_C->status = GGMS_E_INTERNAL;  // until the last launch reports
   if (o.stats || prof) {
     rc = enqueue(st);
   } else {
@@ -670,7 +674,7 @@ static int run_single(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
                             p.seed, (uint64_t)(uint32_t)p.train_steps | ((uint64_t)pv->nt << 32),
                             (uint64_t)pv->unroll | ((uint64_t)float_bits(p.bound) << 8),
                             (uint64_t)float_bits(p.window_z), (uint64_t)(uintptr_t)ctx->arena,
-                            (uint64_t)(uintptr_t)ctx->pinned, (uint64_t)p.pl_knots};
+                            (uint64_t)(uintptr_t)ctx->pinned, (uint64_t)p.pl_knots, (uint64_t)barrier_limit(ctx)};
     rc = run_graphed(ctx, key, (int)(sizeof(key) / sizeof(key[0])), st, enqueue);
   }
   if (rc) return rc;
@@ -683,6 +687,7 @@ static int run_single(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
   const bool need_sync = host_out || o.stats;
   if (!need_sync) return GGMS_OK;
   GGMS_CU(cudaStreamSynchronize(st));
+  if (pin_C->status == GGMS_E_INTERNAL) return GGMS_E_INTERNAL;  // no answers, and no counters to report
   if (host_out) memcpy(out, pin_out, sizeof(T) * nk);
   if (o.stats) {
     ggms_stats* s = o.stats;
@@ -868,7 +873,7 @@ static int run_segmented(Context* ctx, const T* d_in, const int64_t* seg_off, in
     const uint64_t key[] = {0x5E6ull + sizeof(T), (uint64_t)(uintptr_t)d_in, (uint64_t)(uintptr_t)seg_off, nseg,
                             (uint64_t)(uintptr_t)ks, (uint64_t)(uintptr_t)k_off, (uint64_t)(uintptr_t)out, n,
                             nk, (uint64_t)(uintptr_t)ctx->arena, (uint64_t)std::is_signed<T>::value,
-                            (uint64_t)std::is_floating_point<T>::value, p.seed};
+                            (uint64_t)std::is_floating_point<T>::value, p.seed, (uint64_t)barrier_limit(ctx)};
     rc = run_graphed(ctx, key, (int)(sizeof(key) / sizeof(key[0])), st, enqueue);
   }
   if (rc) return rc;

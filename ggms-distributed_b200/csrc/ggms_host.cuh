@@ -59,6 +59,7 @@ struct Context {
   cudaEvent_t pin_busy = nullptr;  // recorded after the last call's uploads from the pinned buffer
   cudaStream_t side = nullptr;     // the sampled assigner's build next to the learned one; the warp finisher
   cudaEvent_t fork = nullptr, join = nullptr, fork2 = nullptr, join2 = nullptr;
+  long long barrier_limit = 0;     // cycles a grid barrier may take (0: the default; < 0: none)
   // autotuner: launch shapes and bucket counts picked per shape class
   struct Tuned {
     uint64_t key[4];
@@ -81,8 +82,14 @@ static int cuda_status(cudaError_t e) {
 
 // Every layout of the arena begins with the call's counters and, at
 // ARENA_BAR, the words the barriers of cooperative launches count on: one for
-// the whole grid, and one for every team of the batched path.
+// the whole grid, and one for every team of the batched path; the last word
+// counts the CTAs that have left such a launch (leave_body).
 constexpr size_t ARENA_BAR = 256, ARENA_BAR_BYTES = 8192;
+
+// Cycles a grid barrier waits before it gives up: about two seconds.
+constexpr long long BARRIER_CYCLES = 1ll << 32;
+
+static long long barrier_limit(const Context* c) { return c->barrier_limit ? c->barrier_limit : BARRIER_CYCLES; }
 
 static int ensure_arena(Context* c, size_t bytes) {
   if (c->arena_bytes >= bytes) return GGMS_OK;

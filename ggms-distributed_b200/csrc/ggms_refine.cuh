@@ -27,6 +27,8 @@ struct RefineArgs {
   using K = typename KeyOf<T>::K;
   Counters* C;
   uint32_t* bar;               // the arena's barrier word
+  uint32_t* left;              // CTAs that have left the launch
+  long long limit;             // cycles a barrier may take
   K* cand[2];
   Seg<K>* segs[2];
   TileRef* tiles[2];
@@ -52,8 +54,9 @@ GGMS_BEGIN
 // them the leader.  It adds 2^31 - (ncta - 1), the others 1: when all have arrived the top bit
 // has flipped and the low bits are back where they were, so the word needs no
 // reset between barriers or launches.  In two halves: what the CTA did before
-// arrive() is visible to a CTA after its wait().  The wait is bounded (about
-// two seconds): false for the whole CTA, with the status set, when it ran out.
+// arrive() is visible to a CTA after its wait().  The wait is bounded by `limit`
+// cycles (negative: it gives up at once): false for the whole CTA, with the
+// status set, when it ran out.
 struct GridBarrier {
   uint32_t old;  // thread 0's
   __device__ __forceinline__ void arrive(uint32_t* bar, uint32_t ncta, bool leader) {
@@ -63,30 +66,29 @@ struct GridBarrier {
       old = atomicAdd(bar, leader ? 0x80000000u - (ncta - 1u) : 1u);
     }
   }
-  __device__ __forceinline__ bool wait(uint32_t* bar, uint32_t ncta, Counters* C) {
+  __device__ __forceinline__ bool wait(uint32_t* bar, uint32_t ncta, Counters* C, long long limit) {
     bool good = true;
     if (threadIdx.x == 0 && ncta > 1u) {
       const long long t0 = clock64();
-      for (;;) {
+      good = limit >= 0;
+      while (good) {
         uint32_t now;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(bar) : "memory");
         if ((now ^ old) & 0x80000000u) break;
-        if (clock64() - t0 > (1ll << 32)) {
-          good = false;
-          set_status(C, GGMS_E_INTERNAL);
-          break;
-        }
+        good = clock64() - t0 <= limit;
       }
+      if (!good) set_status(C, GGMS_E_INTERNAL);
       __threadfence();
     }
     return __syncthreads_and(good) != 0;
   }
 };
 
-__device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t ncta, bool leader, Counters* C) {
+__device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t ncta, bool leader, Counters* C,
+                                             long long limit) {
   GridBarrier b;
   b.arrive(bar, ncta, leader);
-  return b.wait(bar, ncta, C);
+  return b.wait(bar, ncta, C, limit);
 }
 
 // Every k's answer; a k that is not resolved is an error.  out may be pinned
@@ -100,18 +102,23 @@ __device__ __forceinline__ void write_out_body(const typename KeyOf<T>::K* k_key
   }
 }
 
-// The last CTA to get here copies the counters to pinned host memory (the
-// host reads the status and statistics after its sync).  All threads call it.
-__device__ __forceinline__ void report_body(Counters* C, Counters* report, uint32_t ncta) {
+// The end of a cooperative launch: every CTA comes here, also one whose barrier
+// ran out, and the last copies the counters to pinned host memory (the host
+// reads the status and statistics after its sync).  *left is 0 before and
+// after; it is no counter of the call, whose zeroing a CTA may still have
+// before it when another one gives up.  All threads call it.
+__device__ __forceinline__ void leave_body(const Counters* C, uint32_t* left, Counters* report, uint32_t ncta) {
   __shared__ uint32_t last;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    last = atomicAdd(&C->ticket, 1u) + 1u == ncta ? 1u : 0u;
+    last = atomicAdd(left, 1u) + 1u == ncta ? 1u : 0u;
     __threadfence();
   }
   __syncthreads();
-  if (last && report)
+  if (!last) return;
+  if (threadIdx.x == 0) *left = 0u;
+  if (report)
     for (uint32_t w = threadIdx.x; w < sizeof(Counters) / 4; w += blockDim.x)
       reinterpret_cast<uint32_t*>(report)[w] = __ldcg(reinterpret_cast<const uint32_t*>(C) + w);
 }
@@ -138,18 +145,18 @@ __device__ __forceinline__ bool refine_body(const RefineArgs<T>& a, uint8_t* sme
     const K* src = a.cand[(l - 1) & 1];
     K* dst = a.cand[l & 1];
     prep_body(a.rows[p], a.aflag[p], C, p, a.caps, cta, ncta);
-    if (!grid_barrier(a.bar, ncta, cta == 0u, C)) return false;
+    if (!grid_barrier(a.bar, ncta, cta == 0u, C, a.limit)) return false;
     count_body<K, NT>(src, a.segs[p], a.tiles[p], C, p, a.rows[p], a.caps, bins, cta, ncta);
-    if (!grid_barrier(a.bar, ncta, cta == 0u, C)) return false;
+    if (!grid_barrier(a.bar, ncta, cta == 0u, C, a.limit)) return false;
     scan_body<NT>(a.rows[p], C, p, a.caps, red, cta, ncta);
-    if (!grid_barrier(a.bar, ncta, cta == 0u, C)) return false;
+    if (!grid_barrier(a.bar, ncta, cta == 0u, C, a.limit)) return false;
     for (uint32_t i = cta * NT + threadIdx.x; i < a.nk; i += ncta * NT)
       locate_in_row(i, a.rows[p], NBIN, a.krank, a.kseg, &a.segs[p]->row, sizeof(Seg<K>) / 4, a.kbin, a.aflag[p],
                     NBIN_WORDS, C, nullptr);
-    if (!grid_barrier(a.bar, ncta, cta == 0u, C)) return false;
+    if (!grid_barrier(a.bar, ncta, cta == 0u, C, a.limit)) return false;
     children_body<K, NT>(a.rows[p], a.aflag[p], a.segs[p], C, p, a.segs[q], a.cursor[q], a.tiles[q], a.points,
                          a.khead[q], a.smalls, a.tinies, a.bigs[p], a.bigs[q], a.caps, cta, ncta);
-    if (!grid_barrier(a.bar, ncta, cta == 0u, C)) return false;
+    if (!grid_barrier(a.bar, ncta, cta == 0u, C, a.limit)) return false;
     for (uint32_t i = cta * NT + threadIdx.x; i < a.nk; i += ncta * NT) {
       const uint32_t s = a.kseg[i];
       if (s != K_DONE)
@@ -159,7 +166,7 @@ __device__ __forceinline__ bool refine_body(const RefineArgs<T>& a, uint8_t* sme
     if (l < MAXLEV)
       compact_body<K, NT>(src, a.segs[p], a.tiles[p], C, p, a.rows[p], a.segs[q], a.cursor[q], dst, a.caps, bins,
                           cta, ncta);
-    if (!grid_barrier(a.bar, ncta, cta == 0u, C)) return false;
+    if (!grid_barrier(a.bar, ncta, cta == 0u, C, a.limit)) return false;
     if (l < MAXLEV) {
       // children of up to RF_TINY bytes: a warp each, in the space of the CTA
       // finisher (2^28 keys, 2^14 ks: 16 K children of ~500 keys, 260 us at a
@@ -173,7 +180,7 @@ __device__ __forceinline__ bool refine_body(const RefineArgs<T>& a, uint8_t* sme
       __syncthreads();
       small_select_body<K, NT>(dst, a.segs[q], a.smalls, C, a.khead[q], a.knext, a.krank, a.kseg, a.kkey,
                                a.caps.small_keys, a.caps, smem, cta, ncta);
-      if (!grid_barrier(a.bar, ncta, cta == 0u, C)) return false;
+      if (!grid_barrier(a.bar, ncta, cta == 0u, C, a.limit)) return false;
     }
   }
   return true;
@@ -182,9 +189,9 @@ __device__ __forceinline__ bool refine_body(const RefineArgs<T>& a, uint8_t* sme
 template <typename T>
 __global__ __launch_bounds__(RF_NT, 2) void refine_levels(const __grid_constant__ RefineArgs<T> a) {
   extern __shared__ __align__(128) uint8_t smem[];
-  if (!refine_body<T, RF_NT>(a, smem)) return;
-  write_out_body<T>(a.kkey, a.kseg, a.nk, a.out, a.C, blockIdx.x, gridDim.x);
-  report_body(a.C, a.report, gridDim.x);
+  if (refine_body<T, RF_NT>(a, smem))
+    write_out_body<T>(a.kkey, a.kseg, a.nk, a.out, a.C, blockIdx.x, gridDim.x);
+  leave_body(a.C, a.left, a.report, gridDim.x);
 }
 
 GGMS_END

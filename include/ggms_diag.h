@@ -45,6 +45,11 @@ GGMS_API int ggms_diag_fit(const uint32_t* sorted_keys, int S, int kind, int ste
  * arithmetic only: no CUDA call. */
 GGMS_API int ggms_diag_pinned_layout(int64_t nk, int elem, int host_k, int host_out, int64_t* out);
 
+/* Limit, in GPU cycles, of every wait at a grid barrier of this context's later
+ * calls: 0 the library's own, negative: every wait gives up at once.  A wait
+ * that runs out ends the call with GGMS_E_INTERNAL and no answers. */
+GGMS_API int ggms_diag_barrier_limit(ggms_context* ctx, int64_t cycles);
+
 #ifdef __cplusplus
 }
 #endif
