@@ -982,7 +982,7 @@ __global__ __launch_bounds__(DR_NT, 1) void direct_select(const __grid_constant_
   if (good && __ldcg(&C->nbig[1]))
     good = refine_body<T, DR_NT>(r, smem) && grid_barrier(r.bar, ncta, cta == 0u, C, r.limit);
   if (good) write_out_body<T>(r.kkey, r.kseg, r.nk, r.out, C, cta, ncta);
-  leave_body(C, r.left, r.report, ncta);
+  leave_body(C, r.bar, r.left, r.report, ncta);
   GGMS_TRACE(10);
 }
 

@@ -428,6 +428,7 @@ struct Counters {
   uint32_t nbig[2];           // segments of pool p that a level refines (listed in bigs[p])
   uint32_t coarse;            // level 0 copies NGRP groups of buckets (most buckets hold a k)
   uint32_t passes;            // launches that read the whole input (counted by the kernels themselves)
+  uint32_t failed;            // a grid barrier of the call ran out
   uint32_t nlist[BT_CLASSES]; // batched path: segments per class
 };
 

@@ -27,7 +27,7 @@ struct RefineArgs {
   using K = typename KeyOf<T>::K;
   Counters* C;
   uint32_t* bar;               // the arena's barrier word
-  uint32_t* left;              // CTAs that have left the launch
+  uint32_t* left;              // CTAs that have left the launch (the word after the barriers' words)
   long long limit;             // cycles a barrier may take
   K* cand[2];
   Seg<K>* segs[2];
@@ -77,7 +77,10 @@ struct GridBarrier {
         if ((now ^ old) & 0x80000000u) break;
         good = clock64() - t0 <= limit;
       }
-      if (!good) set_status(C, GGMS_E_INTERNAL);
+      if (!good) {
+        set_status(C, GGMS_E_INTERNAL);
+        atomicExch(&C->failed, 1u);
+      }
       __threadfence();
     }
     return __syncthreads_and(good) != 0;
@@ -102,12 +105,15 @@ __device__ __forceinline__ void write_out_body(const typename KeyOf<T>::K* k_key
   }
 }
 
-// The end of a cooperative launch: every CTA comes here, also one whose barrier
-// ran out, and the last copies the counters to pinned host memory (the host
-// reads the status and statistics after its sync).  *left is 0 before and
-// after; it is no counter of the call, whose zeroing a CTA may still have
-// before it when another one gives up.  All threads call it.
-__device__ __forceinline__ void leave_body(const Counters* C, uint32_t* left, Counters* report, uint32_t ncta) {
+// The end of a call's last cooperative launch: every CTA comes here, also one
+// whose barrier ran out, and the last copies the counters to pinned host memory
+// (the host reads the status and statistics after its sync).  A barrier that
+// ran out, here or in batch_teams, has left its word between two barriers;
+// nobody waits any more, so the last CTA zeroes the words for the next call.
+// *left is 0 before and after; it is no counter of the call, whose zeroing a
+// CTA may still have before it when another one gives up.  All threads call it.
+__device__ __forceinline__ void leave_body(const Counters* C, uint32_t* bar, uint32_t* left, Counters* report,
+                                           uint32_t ncta) {
   __shared__ uint32_t last;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -117,6 +123,8 @@ __device__ __forceinline__ void leave_body(const Counters* C, uint32_t* left, Co
   }
   __syncthreads();
   if (!last) return;
+  if (__ldcg(&C->failed))
+    for (uint32_t* w = bar + threadIdx.x; w < left; w += blockDim.x) *w = 0u;
   if (threadIdx.x == 0) *left = 0u;
   if (report)
     for (uint32_t w = threadIdx.x; w < sizeof(Counters) / 4; w += blockDim.x)
@@ -189,9 +197,10 @@ __device__ __forceinline__ bool refine_body(const RefineArgs<T>& a, uint8_t* sme
 template <typename T>
 __global__ __launch_bounds__(RF_NT, 2) void refine_levels(const __grid_constant__ RefineArgs<T> a) {
   extern __shared__ __align__(128) uint8_t smem[];
-  if (refine_body<T, RF_NT>(a, smem))
+  // (after a team's barrier ran out the segments are incomplete and its words unusable)
+  if (!__ldcg(&a.C->failed) && refine_body<T, RF_NT>(a, smem))
     write_out_body<T>(a.kkey, a.kseg, a.nk, a.out, a.C, blockIdx.x, gridDim.x);
-  leave_body(a.C, a.left, a.report, gridDim.x);
+  leave_body(a.C, a.bar, a.left, a.report, gridDim.x);
 }
 
 GGMS_END

@@ -50,3 +50,70 @@ def test_the_host_sees_a_barrier_that_ran_out(path):
     assert host_call(ctx, d, ks, out, **PATHS[path]) == G.GGMS_E_INTERNAL
     assert (out == 123.0).all()  # no answers of an earlier call
     ctx.close()
+
+
+def device_call(ctx, d, dk, dout, **kw):
+    o = G.default_opts(ks_on_device=1, out_on_device=1, **kw)
+    assert G.multiselect_ex(ctx, d.data_ptr(), N, dk.data_ptr(), len(dk), dout.data_ptr(), np.float32, o) == 0
+
+
+@pytest.mark.parametrize("cycles", [-1, 1, 2000])
+@pytest.mark.parametrize("path", PATHS)
+def test_calls_after_a_barrier_that_ran_out(path, cycles):
+    """... and leaves the context as it was: the calls after it are exact.  With
+    a limit of some cycles the CTAs give up at different barriers (or not at
+    all: then the answers are exact)."""
+    import torch
+    ctx = G.Context(0)
+    v = vector(3)
+    d, ks = to_device(v), D.ks_uniform(N, 101, 4)
+    dk, dout = to_device(ks), torch.empty(len(ks), dtype=torch.float32, device="cuda")
+    exp = orc.bits(orc.select(v, ks))
+    out = np.empty(len(ks), np.float32)
+    for _ in range(4):  # run directly, captured, replayed
+        limit(ctx, cycles)
+        rc = host_call(ctx, d, ks, out, **PATHS[path])
+        assert rc == G.GGMS_E_INTERNAL or (cycles > 0 and rc == 0 and (orc.bits(out) == exp).all())
+        device_call(ctx, d, dk, dout, **PATHS[path])
+        assert ctx.status() == G.GGMS_E_INTERNAL or cycles > 0
+        device_call(ctx, d, dk, dout, **PATHS[path])  # nobody asks for this one's status
+        limit(ctx, 0)
+        device_call(ctx, d, dk, dout, **PATHS[path])
+        assert ctx.status() == 0
+        np.testing.assert_array_equal(orc.bits(dout.cpu().numpy()), exp)
+        assert host_call(ctx, d, ks, out, **PATHS[path]) == 0
+        np.testing.assert_array_equal(orc.bits(out), exp)
+    ctx.close()
+
+
+@pytest.mark.parametrize("cycles", [-1, 1, 2000])
+def test_batched_calls_after_a_barrier_that_ran_out(cycles):
+    """Teams of every size (a long segment among equal ones), then single CTAs, sorts and rows."""
+    import torch
+    ctx = G.Context(0)
+    g = np.random.default_rng(5)
+    lens = np.array([1 << 22] + [(1 << 19) + 7] * 6 + [100_003] * 5 + [5000] * 7 + [700] * 9)
+    off = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    v = g.integers(0, 1 << 32, off[-1], dtype=np.uint64).astype(np.uint32)
+    v[g.random(len(v)) < 0.3] = 12345
+    v[g.random(len(v)) < 0.3] = 12346
+    ks = np.concatenate([g.integers(1, n + 1, 30) for n in lens]).astype(np.uint32)
+    k_off = (np.arange(len(lens) + 1) * 30).astype(np.int64)
+    dv, dk, do, dko = to_device(v), to_device(ks), to_device(off), to_device(k_off)
+    out = torch.empty(len(ks), dtype=torch.int32, device="cuda")
+
+    def call():
+        assert G.segmented(ctx, dv.data_ptr(), do.data_ptr(), len(lens), dk.data_ptr(), dko.data_ptr(),
+                           out.data_ptr(), np.uint32) == 0
+    exp = orc.select_segmented(v, off, ks, k_off)
+    for _ in range(3):
+        limit(ctx, cycles)
+        call()
+        st = ctx.status()
+        assert st == G.GGMS_E_INTERNAL or (cycles > 0 and st == 0)
+        call()
+        limit(ctx, 0)
+        call()
+        assert ctx.status() == 0
+        np.testing.assert_array_equal(out.cpu().numpy().view(np.uint32), exp)
+    ctx.close()
