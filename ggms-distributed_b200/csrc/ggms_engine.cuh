@@ -145,13 +145,13 @@ static Workspace<K> layout(const Plan& p, uint8_t* base) {
 // The arguments of refine_levels over a workspace: the levels from 1 on, then
 // the answers to `out` (device or pinned memory).
 template <typename T>
-static RefineArgs<T> refine_args(const Workspace<typename KeyOf<T>::K>& w, const Context* c, uint32_t nk, Caps caps,
+static RefineArgs<T> refine_args(const Workspace<typename KeyOf<T>::K>& w, const Context* c, uint64_t n, uint32_t nk, Caps caps,
                                  T* out, Counters* report) {
   RefineArgs<T> a;
   a.C = w.C;
   a.bar = (uint32_t*)(c->arena + ARENA_BAR);
   a.left = a.bar + ARENA_BAR_BYTES / 4 - 1;
-  a.limit = barrier_limit(c);
+  a.limit = barrier_limit(c, n, nk);
   for (int i = 0; i < 2; ++i) {
     a.cand[i] = w.cand[i];
     a.segs[i] = w.segs[i];
@@ -463,14 +463,14 @@ static int run_direct(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
     a.gact = w.aflag0;
     a.ghist = w.hist0;
     a.gcur = w.cmap0;
-    a.r = refine_args<T>(w, ctx, nk, caps, host_out ? pin_out : out, host_out ? pin_C : nullptr);
+    a.r = refine_args<T>(w, ctx, n, nk, caps, host_out ? pin_out : out, host_out ? pin_C : nullptr);
     return launch_direct<T>(ctx, a, ctas, s);
   };
   const uint64_t key[] = {0xD17ull + sizeof(T) + (topk ? 256u : 0u) + (std::is_signed<T>::value ? 16u : 0u) +
                               (std::is_floating_point<T>::value ? 32u : 0u),
                           (uint64_t)(uintptr_t)d_in, n, host_k ? 1ull : (uint64_t)(uintptr_t)ks, nk,
                           host_out ? 1ull : (uint64_t)(uintptr_t)out, p.seed, (uint64_t)(uintptr_t)ctx->arena,
-                          (uint64_t)(uintptr_t)ctx->pinned, (uint64_t)barrier_limit(ctx)};
+                          (uint64_t)(uintptr_t)ctx->pinned, (uint64_t)ctx->barrier_limit};
   if (host_out) pin_C->status = GGMS_E_INTERNAL;  // until the launch reports
   rc = run_graphed(ctx, key, (int)(sizeof(key) / sizeof(key[0])), st, enqueue);
   if (rc) return rc;
@@ -655,7 +655,7 @@ static int run_single(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
 
     // ---- refinement levels over candidates, answers
     prof_rec(prof, 8, s);
-    rc = launch_refine<T>(ctx, refine_args<T>(w, ctx, nk, caps, host_out ? (T*)pin_out : out,
+    rc = launch_refine<T>(ctx, refine_args<T>(w, ctx, n, nk, caps, host_out ? (T*)pin_out : out,
                                               host_out || o.stats ? pin_C : nullptr), s);
     if (rc) return rc;
     if (cudaGetLastError() != cudaSuccess) return GGMS_E_CUDA;
@@ -674,7 +674,7 @@ static int run_single(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
                             p.seed, (uint64_t)(uint32_t)p.train_steps | ((uint64_t)pv->nt << 32),
                             (uint64_t)pv->unroll | ((uint64_t)float_bits(p.bound) << 8),
                             (uint64_t)float_bits(p.window_z), (uint64_t)(uintptr_t)ctx->arena,
-                            (uint64_t)(uintptr_t)ctx->pinned, (uint64_t)p.pl_knots, (uint64_t)barrier_limit(ctx)};
+                            (uint64_t)(uintptr_t)ctx->pinned, (uint64_t)p.pl_knots, (uint64_t)ctx->barrier_limit};
     rc = run_graphed(ctx, key, (int)(sizeof(key) / sizeof(key[0])), st, enqueue);
   }
   if (rc) return rc;
@@ -863,7 +863,7 @@ static int run_segmented(Context* ctx, const T* d_in, const int64_t* seg_off, in
     a.seed = p.seed ^ 0x5E6A11ull;
     a.lists = w.lists;
     a.scratch = w.scratch;
-    a.r = refine_args<T>(w, ctx, nk, caps, out, nullptr);
+    a.r = refine_args<T>(w, ctx, n, nk, caps, out, nullptr);
     if (const int r = launch_batch<T>(ctx, a, s)) return r;
     return launch_refine<T>(ctx, a.r, s);
   };
@@ -873,7 +873,7 @@ static int run_segmented(Context* ctx, const T* d_in, const int64_t* seg_off, in
     const uint64_t key[] = {0x5E6ull + sizeof(T), (uint64_t)(uintptr_t)d_in, (uint64_t)(uintptr_t)seg_off, nseg,
                             (uint64_t)(uintptr_t)ks, (uint64_t)(uintptr_t)k_off, (uint64_t)(uintptr_t)out, n,
                             nk, (uint64_t)(uintptr_t)ctx->arena, (uint64_t)std::is_signed<T>::value,
-                            (uint64_t)std::is_floating_point<T>::value, p.seed, (uint64_t)barrier_limit(ctx)};
+                            (uint64_t)std::is_floating_point<T>::value, p.seed, (uint64_t)ctx->barrier_limit};
     rc = run_graphed(ctx, key, (int)(sizeof(key) / sizeof(key[0])), st, enqueue);
   }
   if (rc) return rc;

@@ -86,10 +86,13 @@ static int cuda_status(cudaError_t e) {
 // counts the CTAs that have left such a launch (leave_body).
 constexpr size_t ARENA_BAR = 256, ARENA_BAR_BYTES = 8192;
 
-// Cycles a grid barrier waits before it gives up: about two seconds.
-constexpr long long BARRIER_CYCLES = 1ll << 32;
-
-static long long barrier_limit(const Context* c) { return c->barrier_limit ? c->barrier_limit : BARRIER_CYCLES; }
+// Cycles a grid barrier waits before it gives up: about two seconds, and what
+// one CTA may have to do between two barriers while the others wait -- walk a
+// list of all the ks (a k takes two dependent loads, under 2000 cycles) or
+// finish its share of the keys.
+static long long barrier_limit(const Context* c, uint64_t n, uint64_t nk) {
+  return c->barrier_limit ? c->barrier_limit : (1ll << 32) + 4096ll * (long long)nk + (long long)n;
+}
 
 static int ensure_arena(Context* c, size_t bytes) {
   if (c->arena_bytes >= bytes) return GGMS_OK;

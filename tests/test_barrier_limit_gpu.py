@@ -117,3 +117,18 @@ def test_batched_calls_after_a_barrier_that_ran_out(cycles):
         assert ctx.status() == 0
         np.testing.assert_array_equal(out.cpu().numpy().view(np.uint32), exp)
     ctx.close()
+
+
+def test_a_long_list_of_ks_between_barriers():
+    """One refinement level's child holds all 8 M ks (the same k many times): one
+    warp walks their list while the other CTAs wait at the barrier behind it, for
+    longer than a wait without ks may take.  fp32, 2^25 keys in 1024 buckets:
+    every bucket takes a level, its bins hold some 16 keys."""
+    ctx = G.Context(0)
+    n, nk = 1 << 25, 8_000_000
+    v = D.normal_f32(n, 6)
+    k = n // 3
+    got = G.select(ctx, to_device(v).data_ptr(), n, np.full(nk, k, np.uint32), np.float32,
+                   assigner=G.ASSIGNER_SAMPLED, num_buckets=1024)
+    assert (orc.bits(got) == orc.bits(np.sort(v)[n - k:n - k + 1])[0]).all()
+    ctx.close()
