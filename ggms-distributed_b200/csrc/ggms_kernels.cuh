@@ -2175,12 +2175,22 @@ __device__ __forceinline__ void count_body(const K* src, const Seg<K>* segs, con
     }
     const uint64_t beg = s.off + (uint64_t)tr.no * TILE;
     const uint64_t end = min(beg + TILE, s.off + s.cnt);
-    tile_stream<K, NT>(src, beg, end, [&](const K* k, uint32_t mask) {
+    // (16-byte loads with a mask test per key, as in compact_body, counted at
+    // half the rate: 375 us against 237 for 2^28 fp32 keys, and spilled)
+    constexpr int U = 8;  // independent loads in flight per thread
+    for (uint64_t o = beg + threadIdx.x; o < end; o += (uint64_t)NT * U) {
+      K x[U];
 #pragma unroll
-      for (int t = 0; t < 16 / (int)sizeof(K); ++t)
-        if ((mask >> t) & 1u)
-          atomicAdd(&h[min((uint32_t)((K)(k[t] - s.lo) >> s.shift), (uint32_t)NBIN - 1u)], 1u);
-    });
+      for (int u = 0; u < U; ++u) {
+        const uint64_t i = o + (uint64_t)u * NT;
+        x[u] = i < end ? src[i] : (K)0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (o + (uint64_t)u * NT >= end) break;
+        atomicAdd(&h[min((uint32_t)((K)(x[u] - s.lo) >> s.shift), (uint32_t)NBIN - 1u)], 1u);
+      }
+    }
     open_keys += end - beg;
   }
   if (open != 0xFFFFFFFFu) flush();
