@@ -2595,6 +2595,7 @@ __global__ __launch_bounds__(NT) void small_select(const InT* __restrict__ src,
 // segment's range (one warp-private 256-bin histogram per digit), or, with more
 // than TS_SORT_ABOVE ks, one bitonic sort.  The ks come from the segment's list.
 constexpr int TS_NT = 128;
+constexpr uint32_t TS_WALK = 64;
 
 template <typename K>
 __device__ __forceinline__ K warp_radix_select(const K* v, uint32_t cnt, int bits, uint32_t r, uint32_t* h,
@@ -2652,15 +2653,22 @@ __device__ __forceinline__ K warp_radix_select(const K* v, uint32_t cnt, int bit
 }
 
 // buf, hist: TK keys (a power of two) and 256 words of shared memory per warp.
+// nk: all ks of the call if a segment's list may hold many of them, else 0
+// (level 0 gives one warp TS_SORT_ABOVE ks at most).  A list is walked at 0.2
+// to 0.5 us a k; behind TS_WALK of its ks, or 1/64 of all, the others are found
+// in k_seg instead: few segments can have as many, so the scans stay few
+// (2^25 fp32, equal ks in one bin of a level: 10^6 ks 483 ms by the list, 19
+// with the scan; 1000 ks 0.69 and 0.25).
 template <typename InT, int NW, uint32_t TK>
 __device__ __forceinline__ void tiny_select_body(const InT* src, const Seg<typename KeyOf<InT>::K>* segs_q,
                                                  const uint32_t* tinies, Counters* C, const uint32_t* khead_q,
                                                  const uint32_t* knext, const uint32_t* k_rank, uint32_t* k_seg,
                                                  typename KeyOf<InT>::K* k_key, const Caps& caps,
                                                  typename KeyOf<InT>::K* buf, uint32_t* hist, uint32_t cta,
-                                                 uint32_t ncta) {
+                                                 uint32_t ncta, uint32_t nk) {
   using K = typename KeyOf<InT>::K;
   const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint32_t walk = nk ? max(TS_WALK, nk / 64u) : 0xFFFFFFFFu;
   K* v = buf + wid * TK;
   uint32_t* h = hist + wid * 256u;
   auto sort_slice = [&](uint32_t cnt) {  // bitonic; N <= TK
@@ -2758,7 +2766,8 @@ __device__ __forceinline__ void tiny_select_body(const InT* src, const Seg<typen
         for (uint32_t k = khead; k != K_NIL && some <= TS_SORT_ABOVE; k = knext[k]) ++some;
       const bool sorted = some > TS_SORT_ABOVE;
       if (sorted) sort_slice(cnt);
-      for (uint32_t k = khead; k != K_NIL; k = knext[k]) {
+      uint32_t k = khead;
+      for (uint32_t steps = 0; k != K_NIL && steps < walk; ++steps, k = knext[k]) {
         bool ok = false;
         const uint32_t r = k_rank[k];
         K pre = 0;
@@ -2767,6 +2776,27 @@ __device__ __forceinline__ void tiny_select_body(const InT* src, const Seg<typen
         if (lane == 0) {
           if (ok) k_key[k] = (K)(s.lo + pre); else set_status(C, GGMS_E_INTERNAL);
           k_seg[k] = K_DONE;
+        }
+      }
+      if (nk && k != K_NIL) {  // a long list: the slice in order, and every k of the call that is here
+        if (by_rank) {
+          __syncwarp();
+          if (lane < cnt) v[ra] = ka;
+          if (lane + 32u < cnt) v[rb] = kb;
+        }
+        __syncwarp();  // (also: the answered ks are marked)
+        for (uint32_t i0 = lane; i0 < nk; i0 += 32u * 8u) {
+          uint32_t at[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) at[q] = i0 + q * 32u < nk ? k_seg[i0 + q * 32u] : K_DONE;
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const uint32_t i = i0 + q * 32u;
+            if (at[q] != id) continue;
+            const uint32_t r = k_rank[i];
+            if (r < cnt) k_key[i] = (K)(s.lo + v[r]); else set_status(C, GGMS_E_INTERNAL);
+            k_seg[i] = K_DONE;
+          }
         }
       }
       __syncwarp();  // the slice is reloaded by the warp's next segment
@@ -2794,7 +2824,7 @@ __global__ __launch_bounds__(NT) void tiny_select(const InT* __restrict__ src,
   __shared__ K buf[NT / 32 * tiny_keys<K>()];
   __shared__ uint32_t hist[NT / 32 * 256];
   tiny_select_body<InT, NT / 32, tiny_keys<K>()>(src, segs_q, tinies, const_cast<Counters*>(C), khead_q, knext,
-                                                 k_rank, k_seg, k_key, caps, buf, hist, blockIdx.x, gridDim.x);
+                                                 k_rank, k_seg, k_key, caps, buf, hist, blockIdx.x, gridDim.x, 0u);
   pdl_wait();
 }
 

@@ -184,7 +184,7 @@ __device__ __forceinline__ bool refine_body(const RefineArgs<T>& a, uint8_t* sme
       if (threadIdx.x < RF_WARPS * 32)
         tiny_select_body<K, RF_WARPS, TK>(dst, a.segs[q], a.tinies, C, a.khead[q], a.knext, a.krank, a.kseg,
                                         a.kkey, a.caps, slices,
-                                        reinterpret_cast<uint32_t*>(slices + RF_WARPS * TK), cta, ncta);
+                                        reinterpret_cast<uint32_t*>(slices + RF_WARPS * TK), cta, ncta, a.nk);
       __syncthreads();
       small_select_body<K, NT>(dst, a.segs[q], a.smalls, C, a.khead[q], a.knext, a.krank, a.kseg, a.kkey,
                                a.caps.small_keys, a.caps, smem, cta, ncta);
