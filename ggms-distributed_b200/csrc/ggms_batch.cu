@@ -39,13 +39,16 @@ int launch_batch(Context* ctx, const BatchArgs<T>& a, cudaStream_t s) {
   ctx->launches += 4;
   batch_init<T><<<std::min<unsigned>(cdiv(std::max(a.nseg, a.r.nk), 256), (unsigned)ctx->sms * 8), 256, 0, s>>>(
       a, (uint32_t)ctx->sms);
+  GGMS_CU(cudaGetLastError());
   if (const int r = launch_rows<T, BT_ROW0>(ctx, a, s)) return r;
   if (const int r = launch_rows<T, BT_ROW0 * 2>(ctx, a, s)) return r;
   batch_sorts<T><<<(unsigned)ctx->sms, DR_NT, sort_smem, s>>>(a);
+  GGMS_CU(cudaGetLastError());
   GGMS_CU(launch_coop(batch_teams<T>, (unsigned)ctx->sms, DR_NT, team_smem<T>(), s, a));
   // a single's segment has more than direct_cap keys
   const unsigned most = (unsigned)std::min<uint64_t>(a.nseg, a.n / direct_cap<K>());
   if (most) batch_singles<T><<<most, DR_NT, smem, s>>>(a);
+  GGMS_CU(cudaGetLastError());
   return GGMS_OK;
 }
 
