@@ -89,14 +89,14 @@ __device__ __forceinline__ uint32_t team_level(uint64_t cnt, uint64_t n, uint32_
   return l;
 }
 
-// Every segment into its class's list; an unresolved k counts as an error, so
-// the ks start as resolved to key 0 and invalid ones stay that way.
+// Every segment into its class's list.  The ks start as taken by nobody, which
+// the answers' kernel reports as an error; the answer of an invalid k is key 0.
 template <typename T>
 __global__ void batch_init(const __grid_constant__ BatchArgs<T> a, uint32_t ncta) {
   Counters* C = a.r.C;
   const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x, gs = gridDim.x * blockDim.x;
   for (uint32_t i = gt; i < a.r.nk; i += gs) {
-    a.r.kseg[i] = K_DONE;
+    a.r.kseg[i] = K_OPEN;
     a.r.kkey[i] = 0;
   }
   const uint32_t lane = threadIdx.x & 31;
@@ -261,6 +261,7 @@ __global__ __launch_bounds__(DR_NT, 1) void batch_sorts(const __grid_constant__ 
       const uint32_t k = a.ks[g.k0 + i];
       if (k >= 1u && k <= g.cnt) a.r.kkey[g.k0 + i] = sorted[g.cnt - k];
       else set_status(a.r.C, GGMS_E_INVALID_ARG);
+      a.r.kseg[g.k0 + i] = K_DONE;
     }
     __syncthreads();
   }
@@ -426,6 +427,7 @@ __global__ __launch_bounds__(RW_NT) void rows_select(const __grid_constant__ Bat
         const uint32_t k = a.ks[k0 + i];
         if (k >= 1u && k <= cnt) a.r.kkey[k0 + i] = sorted[cnt - k];
         else set_status(C, GGMS_E_INVALID_ARG);
+        a.r.kseg[k0 + i] = K_DONE;
       }
       __syncwarp();
     }

@@ -171,6 +171,7 @@ constexpr int ASG_MAXM = 1024;                  // max segments of a PL model
 constexpr int ASG_CELL_BITS = 12;
 constexpr int ASG_NCELL = 1 << ASG_CELL_BITS;   // uniform lookup cells over the knot range
 constexpr uint32_t K_DONE = 0xFFFFFFFFu;        // k_seg value of a resolved k
+constexpr uint32_t K_OPEN = 0xFFFFFFFDu;        // ... of a k whose segment no kernel has taken (batched path); segments are below
 constexpr uint32_t CM_NONE = 0xFFFFFFFFu;       // child-map entry: bin holds no requested k
 constexpr uint32_t CM_POINT = 0x80000000u;      // child-map flag: bin is one key; low bits index points[]
 

@@ -1202,7 +1202,7 @@ __device__ __forceinline__ void locate_in_row(uint32_t i, const uint32_t* rows, 
                                               uint32_t* k_bin, uint32_t* aflag, uint32_t flag_words, Counters* C,
                                               uint32_t* kcnt) {
   uint32_t s = k_seg[i];
-  if (s == K_DONE) return;
+  if (s >= K_OPEN) return;
   if (row_of) s = row_of[(size_t)s * row_stride];
   uint32_t r = k_rank[i];
   const uint32_t lo = locate_one(rows + (size_t)s * row_len, row_len, r, C);

@@ -167,7 +167,7 @@ __device__ __forceinline__ bool refine_body(const RefineArgs<T>& a, uint8_t* sme
     if (!grid_barrier(a.bar, ncta, cta == 0u, C, a.limit)) return false;
     for (uint32_t i = cta * NT + threadIdx.x; i < a.nk; i += ncta * NT) {
       const uint32_t s = a.kseg[i];
-      if (s != K_DONE)
+      if (s < K_OPEN)
         relabel_one<K>(i, a.rows[p][(size_t)a.segs[p][s].row * NBIN + a.kbin[i]], a.kseg, a.kkey, a.points, C, a.segs[q],
                        a.khead[q], a.knext);
     }
