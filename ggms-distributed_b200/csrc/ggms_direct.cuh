@@ -800,6 +800,12 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
   auto is_big = [&](uint32_t b) { return (sm.big[b >> 5] >> (b & 31)) & 1u; };
   auto big_of = [&](uint32_t b) { return sm.bpre[b >> 5] + __popc(sm.big[b >> 5] & ((1u << (b & 31)) - 1u)); };
   GGMS_TRACE(4);
+  // Where the cursors will end, as a weighted sum per warp: when the caller
+  // changes the vector between the count and the copy they end elsewhere, and
+  // the call fails.  The stores stay in the workspace: a vector's n keys lie
+  // below 2 n of its place in cand[0], which cand[1] follows.  (A bound tested
+  // for every copied key cost the batched path 2 to 3 %.)
+  uint32_t ends = 0;
   for (uint32_t b0 = tid; b0 < B; b0 += 8u * DR_NT) {
     // this CTA's range of every child it holds keys of: one reservation each,
     // eight in flight per thread
@@ -814,10 +820,13 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
     for (int u = 0; u < 8; ++u) {
       const uint32_t b = b0 + u * DR_NT;
       if (b >= B || !active(b)) continue;
-      const uint32_t off = b ? sm.J[pz(b - 1)] : 0u;
-      sm.hist[b] = off + base[u];
+      const uint32_t at = (b ? sm.J[pz(b - 1)] : 0u) + base[u];
+      ends += (at + sm.hist[b]) * (2u * b + 1u);
+      sm.hist[b] = at;
     }
   }
+  ends = __reduce_add_sync(FULL, ends);
+  if (lane == 0) red[warp] = ends;
   // ids of the large children: a range of the list of all vectors'
   if (cta == 0 && tid == 0 && nbig) {
     atomicAdd(&r.C->nsegs[1], nbig);
@@ -836,6 +845,12 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
       if (active(b)) cand[atomicAdd(&sm.hist[b], 1u)] = key;
     });
   });
+  __syncthreads();
+  ends = 0;
+  for (uint32_t b = tid; b < B; b += DR_NT)
+    if (active(b)) ends += sm.hist[b] * (2u * b + 1u);
+  ends = __reduce_add_sync(FULL, ends);
+  if (lane == 0 && ends != red[warp]) set_status(r.C, GGMS_E_INTERNAL);
   GGMS_TRACE(6);
   if (!grid_barrier(a.bar, ncta, cta == 0u, r.C, r.limit)) return false;
   GGMS_TRACE(7);
