@@ -724,13 +724,15 @@ static int run_single_tuned(Context* c, const T* d_in, uint64_t n, const uint32_
                             const ggms_opts& o, cudaStream_t st, bool topk = false) {
   if (!o.autotune || o.num_buckets || o.pass_threads || o.pass_unroll || n == 0 || nk == 0)
     return run_single<T>(c, d_in, n, ks, nk, out, o, st, topk);
+  ggms_opts b = o;
+  b.autotune = 0;
+  const bool direct = direct_ok(c, b, n, nk, sizeof(T), topk);  // the one launch is a candidate
   const uint64_t key[4] = {sizeof(T) | (std::is_signed<T>::value ? 16u : 0u) |
                                (std::is_floating_point<T>::value ? 32u : 0u) | (topk ? 64u : 0u),
                            (uint64_t)bitlen64(n) | ((uint64_t)bitlen64(nk) << 8),
-                           (uint64_t)o.assigner | ((uint64_t)o.ks_on_device << 8) | ((uint64_t)o.out_on_device << 9),
+                           (uint64_t)o.assigner | ((uint64_t)o.ks_on_device << 8) | ((uint64_t)o.out_on_device << 9) |
+                               ((uint64_t)direct << 10),
                            (uint64_t)float_bits(o.window_z)};
-  ggms_opts b = o;
-  b.autotune = 0;
   if (const Context::Tuned* t = tuned_find(c, key)) {
     b.num_buckets = t->B;
     b.pass_threads = t->nt;
@@ -741,6 +743,11 @@ static int run_single_tuned(Context* c, const T* d_in, uint64_t n, const uint32_
   static const int shapes[][2] = {{1024, 4}, {1024, -2}, {512, 4}, {512, 8}};
   float best = 3.4e38f;
   Context::Tuned pick{{key[0], key[1], key[2], key[3]}, 8192, DEFAULT_PASS_NT, DEFAULT_PASS_UNROLL};
+  if (direct) {
+    const int rc = time_calls(st, [&] { return run_single<T>(c, d_in, n, ks, nk, out, b, st, topk); }, &best);
+    if (rc) return rc;
+    pick.B = pick.nt = pick.unroll = 0;
+  }
   for (int B : Bs) {
     for (const auto& sh : shapes) {
       ggms_opts t = b;

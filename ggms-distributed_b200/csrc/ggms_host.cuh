@@ -438,7 +438,8 @@ static int mark_done(Context* c, cudaStream_t st) {
 // where ks and answers live) times every candidate on the caller's own data --
 // each candidate a full, correct call: 1 warm-up + 2 timed with CUDA events on
 // the caller's stream -- and keeps the fastest in the context; later calls of
-// the class use it.  (The batched path has nothing to tune: its launch shapes
+// the class use it.  Where a call that tunes nothing takes the one-launch path,
+// that is a candidate too (kept as zeros).  (The batched path has nothing to tune: its launch shapes
 // follow the segments' lengths.)
 static const Context::Tuned* tuned_find(Context* c, const uint64_t* key) {
   for (const auto& t : c->tuned)

@@ -1,6 +1,6 @@
-"""A launch that fails makes the call return an error, whichever launch of the
-call it is.  The library's own objects are linked to a CUDA runtime without a
-GPU (tests/launch_shim/fake_cudart.cpp) that fails one launch."""
+"""The host code's launches.  The library's own objects are linked to a CUDA
+runtime without a GPU (tests/launch_shim/fake_cudart.cpp).  A launch that fails
+makes the call return an error, whichever launch of the call it is."""
 import ctypes
 import os
 import subprocess
@@ -63,3 +63,25 @@ def test_every_failing_launch_is_reported(lib, entry, kw):
     for i in range(launches):
         lib.fake_reset(i, 0)
         assert call(lib, entry, **kw) == G.GGMS_E_CUDA, f"launch {i} of {launches}"
+
+
+def test_the_one_launch_path_is_a_candidate_of_the_autotuner(lib):
+    """With every candidate as fast (the runtime's clock says 1 ms each) the first
+    one is kept: the call that the library makes without tuning."""
+    lib.fake_reset(-1, 0)
+    n, nk = 1 << 20, 100
+    ctx = ctypes.c_void_p()
+    assert lib.ggms_create(ctypes.byref(ctx), 0) == 0
+    o = G.Opts()
+    lib.ggms_default_opts(ctypes.byref(o))
+    o.ks_on_device = o.out_on_device = o.autotune = 1
+    v, out, ks = np.zeros(n, np.float32), np.zeros(nk, np.float32), np.ones(nk, np.uint32)
+    p = lambda a: ctypes.c_void_p(a.ctypes.data)
+    per_call = []
+    for _ in range(2):
+        before = lib.fake_launches()
+        assert lib.ggms_multiselect_f32_ex(ctx, p(v), ctypes.c_int64(n), p(ks), ctypes.c_int64(nk), p(out),
+                                           ctypes.byref(o), None) == G.GGMS_OK
+        per_call.append(lib.fake_launches() - before)
+    lib.ggms_destroy(ctx)
+    assert per_call[0] > 100 and per_call[1] == 1  # tunes, then calls as tuned
