@@ -31,7 +31,7 @@ int launch_batch(Context* ctx, const BatchArgs<T>& a, cudaStream_t s) {
   using K = typename KeyOf<T>::K;
   constexpr size_t smem = sizeof(DirectSmem<K>), sort_smem = sizeof(SortSmem<K>) + direct_cap<K>() * sizeof(K);
   if (!ready[ctx->device]) {
-    GGMS_CU(cudaFuncSetAttribute(batch_teams<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)team_smem<T>()));
+    GGMS_CU(cudaFuncSetAttribute(batch_teams<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     GGMS_CU(cudaFuncSetAttribute(batch_singles<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     GGMS_CU(cudaFuncSetAttribute(batch_sorts<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_smem));
     ready[ctx->device] = 1;
@@ -44,7 +44,7 @@ int launch_batch(Context* ctx, const BatchArgs<T>& a, cudaStream_t s) {
   if (const int r = launch_rows<T, BT_ROW0 * 2>(ctx, a, s)) return r;
   batch_sorts<T><<<(unsigned)ctx->sms, DR_NT, sort_smem, s>>>(a);
   GGMS_CU(cudaGetLastError());
-  GGMS_CU(launch_coop(batch_teams<T>, (unsigned)ctx->sms, DR_NT, team_smem<T>(), s, a));
+  GGMS_CU(launch_coop(batch_teams<T>, std::min<unsigned>((unsigned)ctx->sms, TEAM_MAX_CTAS), DR_NT, smem, s, a, 0u));
   // a single's segment has more than direct_cap keys
   const unsigned most = (unsigned)std::min<uint64_t>(a.nseg, a.n / direct_cap<K>());
   if (most) batch_singles<T><<<most, DR_NT, smem, s>>>(a);

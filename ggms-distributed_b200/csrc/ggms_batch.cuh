@@ -4,9 +4,10 @@
 // batch_init sorts the segments into classes by length, each with a persistent
 // kernel of one CTA per SM:
 //
-//   teams    a segment long against an equal share of the batch goes to a team
-//            of CTAs (half, a quarter, ... of the grid): the one-vector steps of
-//            ggms_direct.cuh with the barriers among the team;
+//   teams    a segment longer than a CTA's equal share of the batch goes to a
+//            team of CTAs: the one-vector steps of ggms_direct.cuh with the
+//            barriers among the team.  All teams work at once, each with CTAs
+//            for its length;
 //   singles  a segment beyond one CTA's sort: the same steps by one CTA (its
 //            barriers are CTA barriers), taken from a shared list, longer ones
 //            first, so that the CTAs end together;
@@ -57,8 +58,6 @@ int launch_batch(Context* ctx, const BatchArgs<T>& a, cudaStream_t s);
 
 GGMS_BEGIN
 
-constexpr uint32_t NONE_YET = 0xFFFFFFFFu;
-
 // A segment's keys and ks; every range is clamped into its array.
 struct SegRange {
   uint64_t off;
@@ -74,19 +73,9 @@ __device__ __forceinline__ SegRange seg_range(const BatchArgs<T>& a, uint32_t s,
 }
 
 // A CTA's equal share of the batch, but no fewer keys than repay a team's
-// barriers.
+// barriers.  Fewer segments than CTAs are longer than it.
 __device__ __forceinline__ uint64_t batch_share(uint64_t n, uint32_t ncta) {
   return max((uint64_t)(1u << 18), n / ncta);
-}
-// Team level of a segment (BT_TEAMS: a single CTA): CTAs for about a share
-// each.  A single CTA is the cheapest per key (no barriers, no global
-// histogram); it takes segments of up to two shares, the longest first.
-__device__ __forceinline__ uint32_t team_level(uint64_t cnt, uint64_t n, uint32_t ncta) {
-  const uint64_t t = cnt / batch_share(n, ncta);
-  if (t <= 1u) return BT_TEAMS;
-  uint32_t l = 0;
-  while (l + 1u < BT_TEAMS && (uint64_t)(ncta >> (l + 1u)) >= t) ++l;
-  return l;
 }
 
 // Every segment into its class's list.  The ks start as taken by nobody, which
@@ -114,10 +103,11 @@ __global__ void batch_init(const __grid_constant__ BatchArgs<T> a, uint32_t ncta
         } else if (g.cnt <= CAP) {
           cls = BT_SORT;
         } else {
-          cls = team_level(g.cnt, a.n, ncta);
-          if (cls == BT_TEAMS) {  // single: halves of the longest a single CTA gets
-            const uint64_t most = 2u * batch_share(a.n, ncta);
-            while (cls + 1u < BT_SORT && (uint64_t)g.cnt << (cls + 1u - BT_TEAMS) <= most) ++cls;
+          const uint64_t share = batch_share(a.n, ncta);
+          cls = BT_TEAM;
+          if (g.cnt <= share) {  // single: halves of the longest a single CTA gets
+            cls = BT_SINGLE;
+            while (cls + 1u < BT_SORT && (uint64_t)g.cnt << (cls + 1u - BT_SINGLE) <= share) ++cls;
           }
         }
       }
@@ -160,67 +150,72 @@ __device__ __forceinline__ void batch_task(const BatchArgs<T>& a, uint32_t s, ui
   t.k0 = g.k0;
 }
 
-// What batch_teams hands to team_vector, behind direct_body's shared memory.
-template <typename T>
-struct TeamShared {
-  DirectTask<T> task;
-  RefineArgs<T> r;
-  uint32_t cls, next;  // the loop's state
-};
-template <typename T>
-constexpr size_t team_smem() {
-  return direct_smem<typename KeyOf<T>::K>() + sizeof(TeamShared<T>);
-}
+constexpr uint32_t TEAM_PER = 8, TEAM_MAX_CTAS = 32 * TEAM_PER;  // segments per lane of the plan below
 
-// A function of its own, so that the loop over the segments holds no registers
-// while a segment is worked on.  It names the shared memory itself: handed a
-// pointer, every access would be a generic one (the count ran at half speed).
+// Segments of teams, in a cooperative launch: the segments [nc round,
+// nc (round + 1)) of the list (nc = gridDim.x; one round where the launch has
+// the CTAs it asks for).  Every CTA computes who works on what: with
+// ceil(length / T) CTAs a segment, for the smallest T (to 1/64) that the CTAs
+// suffice for, no CTA has more than T keys to read.  (Teams of a half, a
+// quarter, ... of the grid, one size after the other, and up to two shares to
+// a single CTA: 64 segments of 2^20 u32 968 us, and 5 of 6 M 353; 303 and 159.)
 template <typename T>
-__device__ __noinline__ bool team_vector() {
+__global__ __launch_bounds__(DR_NT, 1) void batch_teams(const __grid_constant__ BatchArgs<T> a, uint32_t round) {
   extern __shared__ __align__(128) uint8_t smem[];
-  const TeamShared<T>& b = *reinterpret_cast<const TeamShared<T>*>(smem + direct_smem<typename KeyOf<T>::K>());
-  return direct_body<T, false, 2>(b.task, b.r, smem);
-}
-
-// Segments of teams: a cooperative launch of gridDim.x CTAs.  Level l has 2^l
-// teams; team i is the CTAs [gridDim.x i / 2^l, gridDim.x (i + 1) / 2^l): every
-// team lies inside one team of the level above, so its CTAs come to it together
-// and no barrier waits for a CTA that is still in another team's segment.
-template <typename T>
-__global__ __launch_bounds__(DR_NT, 1) void batch_teams(const __grid_constant__ BatchArgs<T> a) {
-  using K = typename KeyOf<T>::K;
-  extern __shared__ __align__(128) uint8_t smem[];
-  TeamShared<T>& sh = *reinterpret_cast<TeamShared<T>*>(smem + direct_smem<K>());
+  __shared__ DirectTask<T> task;
+  __shared__ uint32_t seg_s, first_s, size_s;
   Counters* C = a.r.C;
-  if (threadIdx.x == 0) {
-    sh.r = a.r;
-    sh.cls = 0u;
-    sh.next = NONE_YET;
-    if (blockIdx.x == 0) {  // the count and the copy read the segments beyond one CTA's sort
-      uint32_t m = 0;
-      for (uint32_t c = 0; c < BT_SORT; ++c) m += C->nlist[c];
-      if (m) atomicAdd(&C->passes, 2u);
-    }
+  const uint32_t me = blockIdx.x, nc = gridDim.x, lane = threadIdx.x & 31;
+  if (me == 0 && threadIdx.x == 0 && round == 0) {  // the count and the copy read the segments beyond one CTA's sort
+    uint32_t m = 0;
+    for (uint32_t c = 0; c < BT_SORT; ++c) m += C->nlist[c];
+    if (m) atomicAdd(&C->passes, 2u);
   }
-  for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const uint32_t me = blockIdx.x, nc = gridDim.x;
-      for (; sh.cls < BT_TEAMS; ++sh.cls, sh.next = NONE_YET) {
-        const uint32_t cls = sh.cls, teams = 1u << cls, i = ((me + 1u) * teams - 1u) / nc;
-        const uint32_t j = sh.next == NONE_YET ? i : sh.next;
-        if (j >= C->nlist[cls]) continue;
-        sh.next = j + teams;
-        const uint32_t first = nc * i / teams, size = nc * (i + 1u) / teams - first;
-        batch_task<T>(a, a.lists[(size_t)cls * a.nseg + j], first, me - first, size, a.r.bar + cls * nc + first,
-                      sh.task);
-        break;
+  const uint32_t all = C->nlist[BT_TEAM], m = min(nc, all - min(all, nc * round));
+  if (m == 0) return;
+  if (threadIdx.x < 32) {
+    if (lane == 0) size_s = 0u;
+    const uint32_t* list = a.lists + (size_t)BT_TEAM * a.nseg + nc * round;
+    uint32_t cnt[TEAM_PER], sum = 0, most = 0;  // (all segments together: n < 2^32 keys)
+#pragma unroll
+    for (uint32_t i = 0; i < TEAM_PER; ++i) {
+      const uint32_t j = lane * TEAM_PER + i;
+      bool bad = false;
+      cnt[i] = j < m ? seg_range(a, list[j], &bad).cnt : 0u;
+      sum += cnt[i];
+      most = max(most, cnt[i]);
+    }
+    sum = __reduce_add_sync(FULL, sum);
+    most = __reduce_max_sync(FULL, most);
+    auto ctas = [&](uint32_t c, uint32_t t) { return c / t + (c % t ? 1u : 0u); };
+    uint32_t lo = ctas(sum, nc), hi = most;  // hi suffices: a CTA each
+    while (hi > lo && hi - lo > lo / 64u) {
+      const uint32_t mid = lo + (hi - lo) / 2u;
+      uint32_t need = 0;
+#pragma unroll
+      for (uint32_t i = 0; i < TEAM_PER; ++i) need += ctas(cnt[i], mid);
+      if (__reduce_add_sync(FULL, need) <= nc) hi = mid; else lo = mid + 1u;
+    }
+    uint32_t mine = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < TEAM_PER; ++i) mine += ctas(cnt[i], hi);
+    uint32_t first = warp_incl_scan_u32(mine, lane) - mine;
+    __syncwarp();
+#pragma unroll
+    for (uint32_t i = 0; i < TEAM_PER; ++i) {
+      const uint32_t size = ctas(cnt[i], hi);
+      if (me >= first && me < first + size) {
+        seg_s = list[lane * TEAM_PER + i];
+        first_s = first;
+        size_s = size;
       }
+      first += size;
     }
-    __syncthreads();
-    if (sh.cls == BT_TEAMS) return;
-    if (!team_vector<T>()) return;
+    __syncwarp();
+    if (lane == 0 && size_s) batch_task<T>(a, seg_s, first_s, me - first_s, size_s, a.r.bar + first_s, task);
   }
+  __syncthreads();
+  if (size_s) direct_body<T, false, 4>(task, a.r, smem);
 }
 
 // Segments of single CTAs: CTA j takes the j-th, longest class first, so the
@@ -230,7 +225,7 @@ template <typename T>
 __global__ __launch_bounds__(DR_NT, 1) void batch_singles(const __grid_constant__ BatchArgs<T> a) {
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ DirectTask<T> task;
-  uint32_t cls = BT_TEAMS, j = blockIdx.x;
+  uint32_t cls = BT_SINGLE, j = blockIdx.x;
   for (; cls < BT_SORT; ++cls) {
     const uint32_t m = a.r.C->nlist[cls];
     if (j < m) break;

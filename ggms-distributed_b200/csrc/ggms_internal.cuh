@@ -404,10 +404,9 @@ struct TileRef {
 };
 
 // Classes of caller segments in the batched path (ggms_batch.cuh): teams of
-// CTAs of BT_TEAMS sizes, single CTAs by length (BT_SINGLES lists), one CTA's
-// sort, one warp (two lengths).
-constexpr uint32_t BT_TEAMS = 7, BT_SINGLES = 4;
-constexpr uint32_t BT_SORT = BT_TEAMS + BT_SINGLES, BT_WARP = BT_SORT + 1, BT_CLASSES = BT_WARP + 2;
+// CTAs, single CTAs by length (four lists), one CTA's sort, one warp (two
+// lengths).
+constexpr uint32_t BT_TEAM = 0, BT_SINGLE = 1, BT_SORT = BT_SINGLE + 4, BT_WARP = BT_SORT + 1, BT_CLASSES = BT_WARP + 2;
 
 // Device counters (one small block of memory, zeroed per call).
 struct Counters {
