@@ -44,7 +44,12 @@ int launch_batch(Context* ctx, const BatchArgs<T>& a, cudaStream_t s) {
   if (const int r = launch_rows<T, BT_ROW0 * 2>(ctx, a, s)) return r;
   batch_sorts<T><<<(unsigned)ctx->sms, DR_NT, sort_smem, s>>>(a);
   GGMS_CU(cudaGetLastError());
-  GGMS_CU(launch_coop(batch_teams<T>, std::min<unsigned>((unsigned)ctx->sms, TEAM_MAX_CTAS), DR_NT, smem, s, a, 0u));
+  // fewer than ctx->sms segments are longer than a share: one round with that many CTAs
+  unsigned grid = std::min<unsigned>((unsigned)ctx->sms, TEAM_MAX_CTAS);
+  for (uint32_t round = 0; round * grid < (uint32_t)ctx->sms; ++round) {
+    if (round) ++ctx->launches;
+    GGMS_CU(launch_coop(batch_teams<T>, grid, DR_NT, smem, s, a, round));
+  }
   // a single's segment has more than direct_cap keys
   const unsigned most = (unsigned)std::min<uint64_t>(a.nseg, a.n / direct_cap<K>());
   if (most) batch_singles<T><<<most, DR_NT, smem, s>>>(a);

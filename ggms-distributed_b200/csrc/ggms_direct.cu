@@ -20,7 +20,8 @@ int launch_direct(Context* ctx, const DirectArgs<T>& a, unsigned ctas, cudaStrea
     direct_sort<T><<<1, DR_NT, sort_smem, s>>>(a);
     return cudaGetLastError() == cudaSuccess ? GGMS_OK : GGMS_E_CUDA;
   }
-  GGMS_CU(launch_coop(direct_select<T>, std::min<unsigned>(ctas, (unsigned)ctx->sms), DR_NT, direct_smem<K>(), s, a));
+  unsigned grid = std::min<unsigned>(ctas, (unsigned)ctx->sms);
+  GGMS_CU(launch_coop(direct_select<T>, grid, DR_NT, direct_smem<K>(), s, a));
   return GGMS_OK;
 }
 

@@ -201,12 +201,13 @@ static cudaError_t launch_pdl(void (*k)(P...), unsigned grid, unsigned block, si
 }
 
 // Launch whose CTAs meet at grid barriers: all of them are resident at once, or
-// the launch waits until they can be (or fails when they never can).
+// the launch waits until they can be.  Where the stream has fewer SMs (a green
+// context, a share of the device) it is refused at once; `grid` is then lowered
+// by an eighth until it is taken, and holds what was.
 template <typename... P, typename... A>
-static cudaError_t launch_coop(void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
-                               A&&... args) {
+static cudaError_t launch_coop(void (*k)(P...), unsigned& grid, unsigned block, size_t smem, cudaStream_t s,
+                               const A&... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
@@ -215,7 +216,13 @@ static cudaError_t launch_coop(void (*k)(P...), unsigned grid, unsigned block, s
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
+  for (;;) {
+    cfg.gridDim = dim3(grid);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k, args...);
+    if (e != cudaErrorCooperativeLaunchTooLarge || grid <= 1) return e;
+    cudaGetLastError();
+    grid -= (grid + 7) / 8;
+  }
 }
 
 // The side stream and its fork / join events (created on first use).

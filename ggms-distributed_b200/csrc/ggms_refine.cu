@@ -17,7 +17,8 @@ int launch_refine(Context* ctx, const RefineArgs<T>& a, cudaStream_t s) {
     per_sm = std::min(o, 2);
   }
   ++ctx->launches;
-  GGMS_CU(launch_coop(refine_levels<T>, (unsigned)(ctx->sms * per_sm), RF_NT, SMALL_SELECT_SMEM, s, a));
+  unsigned grid = (unsigned)(ctx->sms * per_sm);
+  GGMS_CU(launch_coop(refine_levels<T>, grid, RF_NT, SMALL_SELECT_SMEM, s, a));
   return GGMS_OK;
 }
 

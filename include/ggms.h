@@ -116,7 +116,14 @@ GGMS_API int ggms_version(void);
 
 /* A context owns a device workspace (grown on demand and reused), pinned
  * staging buffers and events.  One context must not be used by two host threads
- * at once; distinct contexts are independent. */
+ * at once; distinct contexts are independent.
+ *
+ * Some kernels are cooperative launches: their CTAs meet at barriers, so such a
+ * kernel starts when all of them have room, and beside a long kernel of another
+ * stream it waits for that.  Vectors of up to 160 MB and batched calls take one
+ * CTA of 1024 threads and up to 225 KB of shared memory on every SM (fewer for
+ * vectors below 148 K elements), the refinement levels two of 512 threads and
+ * 80 KB.  On a stream with fewer SMs (a green context) they take what it has. */
 typedef struct ggms_context ggms_context;
 GGMS_API int ggms_create(ggms_context** ctx, int device);
 GGMS_API int ggms_destroy(ggms_context* ctx);

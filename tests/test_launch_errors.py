@@ -85,3 +85,15 @@ def test_the_one_launch_path_is_a_candidate_of_the_autotuner(lib):
         per_call.append(lib.fake_launches() - before)
     lib.ggms_destroy(ctx)
     assert per_call[0] > 100 and per_call[1] == 1  # tunes, then calls as tuned
+
+
+@pytest.mark.parametrize("entry,kw", CALLS)
+@pytest.mark.parametrize("ctas", [1, 16, 147])
+def test_fewer_sms_than_the_device_has(lib, entry, kw, ctas):
+    """Cooperative launches are refused where fewer CTAs can be resident: the call
+    makes smaller ones."""
+    lib.fake_reset(-1, ctas)
+    assert call(lib, entry, **kw) == G.GGMS_OK
+    assert lib.fake_coop_grid() <= ctas
+    if kw.get("n", ctas) >= 1 << 20:
+        assert lib.fake_coop_grid() > ctas * 3 // 4
