@@ -264,14 +264,15 @@ __global__ __launch_bounds__(DR_NT, 1) void batch_sorts(const __grid_constant__ 
 
 // One warp per segment of at most ROW keys: the keys are counted into ROW / 2
 // bins uniform in key between the segment's extremes (for floats without the
-// gap around zero, as in DirectMap), placed by bin, and each bin put in order
-// by one lane; every k then reads its rank.  The cost does not depend on the
-// number of ks, where a radix select pays four rounds per k (rows of 600 keys
-// with 4-5 ks: 386 us for 12 M keys).  Up to 64 keys: every key's rank by
-// comparison.
+// gap around zero, as in DirectMap), placed by bin, and each bin that holds a k
+// put in order by one lane; every k then reads its rank.  The cost hardly
+// depends on the number of ks, where a radix select pays four rounds per k (rows
+// of 600 keys with 4-5 ks: 386 us for 12 M keys).  Up to 64 keys: every key's
+// rank by comparison.
 constexpr int RW_NT = 160;  // 5 warps: 4 and 2 CTAs per SM by shared memory
 constexpr int RW_U = 4;     // keys in flight per lane (a lane's accesses are one long chain otherwise)
 constexpr uint32_t RW_LANE = 24;
+constexpr uint32_t RW_BISECT = 6;  // keys of a bin that repay counting them for a bit of one k, not sorting
 template <typename K, uint32_t ROW>
 struct RowSmem {
   K v[ROW], w[ROW];
@@ -379,41 +380,125 @@ __global__ __launch_bounds__(RW_NT) void rows_select(const __grid_constant__ Bat
             if (i0 + q * 32u < cnt) sm.w[at[q]] = k[q];
         }
         __syncwarp();
-        // h[b] is now the end of bin b.  Bins of up to RW_LANE keys: one lane
-        // each, insertion sort.  Larger ones (a dense spot of the keys): the
-        // warp, one by one, unless all their keys are equal
+        // h[b] is now the end of bin b
+        auto sort_few = [&](uint32_t s0, uint32_t e) {  // one lane: insertion sort
+          for (uint32_t i = s0 + 1u; i < e; ++i) {
+            const K x = sm.w[i];
+            uint32_t p = i;
+            for (; p > s0 && sm.w[p - 1u] > x; --p) sm.w[p] = sm.w[p - 1u];
+            sm.w[p] = x;
+          }
+        };
+        auto sort_bin = [&](uint32_t c0, uint32_t len) {  // the warp: bitonic, in v (the row's copy is no longer needed)
+          uint32_t N = 64;
+          while (N < len) N <<= 1;
+          for (uint32_t i = lane; i < N; i += 32u) sm.v[i] = i < len ? sm.w[c0 + i] : key_max<K>();
+          __syncwarp();
+          for (uint32_t kk = 2; kk <= N; kk <<= 1)
+            for (uint32_t jj = kk >> 1; jj > 0; jj >>= 1) {
+              for (uint32_t t = lane; t < N / 2; t += 32u) {  // pair t: i has bit jj clear
+                const uint32_t i = ((t & ~(jj - 1u)) << 1) | (t & (jj - 1u));
+                const K x = sm.v[i], y = sm.v[i | jj];
+                if ((x > y) == ((i & kk) == 0)) { sm.v[i] = y; sm.v[i | jj] = x; }
+              }
+              __syncwarp();
+            }
+          for (uint32_t i = lane; i < len; i += 32u) sm.w[c0 + i] = sm.v[i];
+          __syncwarp();
+        };
+        auto extremes = [&](uint32_t c0, uint32_t len, K& mn, K& mx) {
+          mn = key_max<K>();
+          mx = 0;
+          for (uint32_t i = lane; i < len; i += 32u) {
+            mn = min(mn, sm.w[c0 + i]);
+            mx = max(mx, sm.w[c0 + i]);
+          }
+          mn = warp_min(mn);
+          mx = warp_max(mx);
+        };
+        if (nk <= 32u) {
+          // lane j puts the j-th k's bin in order (the first of the lanes with
+          // the same bin); a larger bin, a dense spot of the keys, is the
+          // warp's.  20,000 rows of 600 keys with one k each: 101 us, and 142 when
+          // half of the keys are zero; ordering all bins took 203 and 478.
+          const uint32_t k = lane < nk ? a.ks[k0 + lane] : 0u, r = cnt - k;
+          const bool ok = k >= 1u && k <= cnt;
+          uint32_t b = RW_BINS + lane, s0 = 0, e = 0;
+          if (ok) {
+            uint32_t l = 0, u = RW_BINS - 1u;
+            while (l < u) {
+              const uint32_t mid = (l + u) >> 1;
+              if (sm.h[mid] > r) u = mid; else l = mid + 1u;
+            }
+            b = l;
+            s0 = b ? sm.h[b - 1u] : 0u;
+            e = sm.h[b];
+          }
+          const uint32_t peers = __match_any_sync(FULL, b);
+          const bool first = ok && __ffs(peers) - 1 == (int)lane;
+          if (first && e - s0 <= RW_LANE) sort_few(s0, e);
+          bool found = false;
+          K ans = 0;
+          for (uint32_t todo = __ballot_sync(FULL, first && e - s0 > RW_LANE); todo; todo &= todo - 1u) {
+            const int src = __ffs(todo) - 1;
+            const uint32_t c0 = __shfl_sync(FULL, s0, src), len = __shfl_sync(FULL, e, src) - c0;
+            uint32_t who = __shfl_sync(FULL, peers, src);
+            K mn, mx;
+            extremes(c0, len, mn, mx);
+            if (mn == mx) continue;
+            if ((uint32_t)(__popc(who) * bitlen((K)(mx - mn))) * RW_BISECT > len) {
+              sort_bin(c0, len);
+              continue;
+            }
+            for (; who; who &= who - 1u) {  // the smallest key with more than `at` keys up to it
+              const int j = __ffs(who) - 1;
+              const uint32_t at = __shfl_sync(FULL, r, j) - c0;
+              K lo_k = mn, hi_k = mx;
+              while (lo_k < hi_k) {  // two bits a round: the loads are what it waits for
+                const K q = (K)((hi_k - lo_k) / 4u), h = (K)((hi_k - lo_k) / 2u);
+                const K p1 = (K)(lo_k + q), p2 = (K)(lo_k + h), p3 = (K)(lo_k + h + q);
+                uint32_t n1 = 0, n2 = 0, n3 = 0;
+#pragma unroll 4
+                for (uint32_t i = lane; i < len; i += 32u) {
+                  const K x = sm.w[c0 + i];
+                  n1 += x <= p1 ? 1u : 0u;
+                  n2 += x <= p2 ? 1u : 0u;
+                  n3 += x <= p3 ? 1u : 0u;
+                }
+                n1 = __reduce_add_sync(FULL, n1);
+                n2 = __reduce_add_sync(FULL, n2);
+                n3 = __reduce_add_sync(FULL, n3);
+                if (n3 <= at) lo_k = (K)(p3 + 1u);
+                else if (n2 <= at) { lo_k = (K)(p2 + 1u); hi_k = p3; }
+                else if (n1 <= at) { lo_k = (K)(p1 + 1u); hi_k = p2; }
+                else hi_k = p1;
+              }
+              if ((int)lane == j) {
+                ans = lo_k;
+                found = true;
+              }
+            }
+          }
+          __syncwarp();
+          if (lane < nk) {
+            if (ok) a.r.kkey[k0 + lane] = found ? ans : sm.w[r];
+            else set_status(C, GGMS_E_INVALID_ARG);
+            a.r.kseg[k0 + lane] = K_DONE;
+          }
+          __syncwarp();
+          continue;
+        }
+        // many ks: every bin, a lane each (large ones: the warp, unless all their keys are equal)
         for (uint32_t b0 = 0; b0 < RW_BINS; b0 += 32u) {
           const uint32_t b = b0 + lane, e = sm.h[b], s0 = b ? sm.h[b - 1u] : 0u;
           const uint32_t large = __ballot_sync(FULL, e - s0 > RW_LANE);
-          if (e - s0 <= RW_LANE)
-            for (uint32_t i = s0 + 1u; i < e; ++i) {
-              const K x = sm.w[i];
-              uint32_t p = i;
-              for (; p > s0 && sm.w[p - 1u] > x; --p) sm.w[p] = sm.w[p - 1u];
-              sm.w[p] = x;
-            }
+          if (e - s0 <= RW_LANE) sort_few(s0, e);
           for (uint32_t todo = large; todo; todo &= todo - 1u) {
             const int src = __ffs(todo) - 1;
-            const uint32_t c0 = __shfl_sync(FULL, s0, src), c1 = __shfl_sync(FULL, e, src), len = c1 - c0;
-            const K x0 = sm.w[c0];
-            bool equal = true;
-            for (uint32_t i = lane; i < len; i += 32u) equal = equal && sm.w[c0 + i] == x0;
-            if (__all_sync(FULL, equal)) continue;
-            uint32_t N = 64;  // bitonic sort in v (the row's copy is no longer needed)
-            while (N < len) N <<= 1;
-            for (uint32_t i = lane; i < N; i += 32u) sm.v[i] = i < len ? sm.w[c0 + i] : key_max<K>();
-            __syncwarp();
-            for (uint32_t kk = 2; kk <= N; kk <<= 1)
-              for (uint32_t jj = kk >> 1; jj > 0; jj >>= 1) {
-                for (uint32_t t = lane; t < N / 2; t += 32u) {  // pair t: i has bit jj clear
-                  const uint32_t i = ((t & ~(jj - 1u)) << 1) | (t & (jj - 1u));
-                  const K x = sm.v[i], y = sm.v[i | jj];
-                  if ((x > y) == ((i & kk) == 0)) { sm.v[i] = y; sm.v[i | jj] = x; }
-                }
-                __syncwarp();
-              }
-            for (uint32_t i = lane; i < len; i += 32u) sm.w[c0 + i] = sm.v[i];
-            __syncwarp();
+            const uint32_t c0 = __shfl_sync(FULL, s0, src), len = __shfl_sync(FULL, e, src) - c0;
+            K mn, mx;
+            extremes(c0, len, mn, mx);
+            if (mn != mx) sort_bin(c0, len);
           }
         }
         __syncwarp();
