@@ -48,7 +48,7 @@ struct BatchArgs {
   uint32_t* scratch;           // per CTA: BT_SCRATCH words (a team uses its first CTA's)
   RefineArgs<T> r;
 };
-constexpr uint32_t BT_SCRATCH = 2 * DIRECT_MAX_B + DIRECT_MAX_B / 32 + 32;
+constexpr uint32_t BT_SCRATCH = 3 * DIRECT_MAX_B + 2 * (DIRECT_MAX_B / 32) + 32;
 
 // Enqueues batch_init and the classes' kernels (ggms_batch.cu).
 template <typename T>
@@ -143,6 +143,7 @@ __device__ __forceinline__ void batch_task(const BatchArgs<T>& a, uint32_t s, ui
   t.ghist = a.scratch + (size_t)first * BT_SCRATCH;
   t.gcur = t.ghist + DIRECT_MAX_B;
   t.gact = t.gcur + DIRECT_MAX_B;
+  t.gpt = t.gact + DIRECT_MAX_B / 32 + 32;
   t.bar = bar;
   t.cta = cta;
   t.ncta = ncta;

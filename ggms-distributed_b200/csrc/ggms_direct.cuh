@@ -29,7 +29,9 @@
 // fp32, 2^14 ks: 390 us of finishing against 30 us), and ks that share a child
 // cost nothing extra.  A child of more than 32 KB goes to the
 // refinement levels.
-// Buckets whose keys turn out to be one value (heavy duplicates) cost one
+// A bucket that only one key can be in (integers of a small range, floats in a
+// few units of the last place: more buckets than keys) is no child: its key is
+// its ks' answer.  Buckets whose keys turn out to be one value cost one
 // refinement level: the level starts from the children's true key range.
 //
 // A vector that fits one CTA's sort (32 KB) is sorted by it (direct_sort):
@@ -67,6 +69,7 @@ struct DirectArgs {
   uint32_t slices;             // 1: every CTA locates its own ks only (one more barrier)
   uint32_t *ghist, *gcur;      // [B] bucket counts, keys copied so far
   uint32_t* gact;              // [B / 32] buckets holding a k (slices)
+  uint32_t* gpt;               // [B / 32 + B] buckets of one key, a sampled position of each
   RefineArgs<T> r;             // workspace of the large children (pool 1) and where the answers go
 };
 
@@ -215,6 +218,7 @@ struct DirectSmem {
   uint32_t J[pz(DIRECT_MAX_B)];     // inclusive counts of the children alone (padded)
   uint32_t act[DIRECT_MAX_B / 32];  // buckets holding a k
   uint32_t big[DIRECT_MAX_B / 32];  // ... and more than direct_cap keys
+  uint32_t pt[DIRECT_MAX_B / 32];   // ... and one key only (before the ks are located: one key only)
   uint32_t bpre[DIRECT_MAX_B / 32]; // large children before each word
 };
 template <typename K>
@@ -476,7 +480,7 @@ struct DirectTask {
   uint32_t nk;
   uint64_t seed;
   uint32_t B, focus, slices;
-  uint32_t *ghist, *gcur, *gact;  // [B], [B], [B / 32 + 1]; one CTA: unused
+  uint32_t *ghist, *gcur, *gact, *gpt;  // [B], [B], [B / 32 + 2], [B / 32 + B]; one CTA: unused
   uint32_t* bar;               // the barrier word of the vector's CTAs
   uint32_t cta, ncta;          // this CTA among them
   uint64_t off;                // the vector's n candidates: r.cand[0] + off
@@ -524,20 +528,21 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
 
   // ---- the map, from a sample every CTA draws for itself
   const uint32_t S = (uint32_t)min(a.n, (uint64_t)DIRECT_SAMPLE);
+  auto sampled = [&](uint32_t i) __attribute__((always_inline)) -> K {
+    uint64_t pos = i;
+    if (a.n > DIRECT_SAMPLE) {  // one key per stratum, at a hashed offset
+      const uint64_t p0 = a.n * i / DIRECT_SAMPLE, p1 = a.n * (i + 1) / DIRECT_SAMPLE;
+      pos = p0 + (((mix64(a.seed ^ i) >> 32) * (p1 - p0)) >> 32);
+    }
+    return KeyOf<T>::to(__ldg(a.in + pos));
+  };
   K sv[DIRECT_SAMPLE / DR_NT];
   K lo = key_max<K>(), hi = 0, hn = 0, lp = key_max<K>();
   constexpr K MID = (K)((K)1 << (sizeof(K) * 8 - 1));  // floating types: the keys below are negative
 #pragma unroll
   for (int j = 0; j < (int)(DIRECT_SAMPLE / DR_NT); ++j) {
     const uint32_t i = tid + j * DR_NT;
-    if (i < S) {
-      uint64_t pos = i;
-      if (a.n > DIRECT_SAMPLE) {  // one key per stratum, at a hashed offset
-        const uint64_t p0 = a.n * i / DIRECT_SAMPLE, p1 = a.n * (i + 1) / DIRECT_SAMPLE;
-        pos = p0 + (((mix64(a.seed ^ i) >> 32) * (p1 - p0)) >> 32);
-      }
-      sv[j] = KeyOf<T>::to(__ldg(a.in + pos));
-    }
+    if (i < S) sv[j] = sampled(i);
   }
 #pragma unroll
   for (int j = 0; j < (int)(DIRECT_SAMPLE / DR_NT); ++j)
@@ -549,6 +554,7 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
     }
   for (uint32_t i = tid; i < DIRECT_CELLS; i += DR_NT) sm.I[i] = 0u;
   for (uint32_t i = tid; i < B; i += DR_NT) sm.hist[i] = 0u;
+  for (uint32_t w = tid; w < B / 32; w += DR_NT) sm.pt[w] = 0u;
   lo = warp_min(lo);
   hi = warp_max(hi);
   if (FP) {
@@ -684,7 +690,11 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
     block_scan_regs<2>(w2, red);
     nfirst = w2[0] - nfirst;
   }
-  if (tid == DR_NT - 1) red[70] = w2[1];
+  if (tid == DR_NT - 1) {
+    red[70] = w2[1];
+    red[71] = 0u;
+    red[68] = 0u;
+  }
   __syncthreads();
   const uint32_t W = (red[70] & 0xFFFFu) + (red[70] >> 16);
   if (focus) hot = red[70] & 0xFFFFu;
@@ -701,6 +711,8 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
     const uint32_t b0 = first_bucket(nfirst), b1 = first_bucket(w2[0]), b2 = first_bucket(w2[1]);
     sm.tab[2 * tid] = min(b0, B - 1u) | (b1 - b0) << 16;  // b0 == B only past the last weight
     sm.tab[2 * tid + 1] = min(b1, B - 1u) | (b2 - b1) << 16;
+    // some cell has a bucket or more per key
+    if (!hi32 && map.csh < 16u && max(b1 - b0, b2 - b1) >> (map.csh & 31u) != 0u) red[71] = 1u;
   }
   __syncthreads();
   // use(m): m is the map in its cheapest form for this sample (the same for every CTA)
@@ -728,6 +740,27 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
   GGMS_TRACE(2);
   if (a.focus) __syncthreads();
   else if (!zeroed.wait(a.bar, ncta, r.C, r.limit)) return false;  // (a CTA barrier too)
+  // Buckets of one key, decided by the first CTA for all: the map is monotone, so
+  // a bucket that a key's neighbours on both sides miss is that key's alone.
+  // (Here and not before the count: there it cost every call 0.5 us.)
+  if (cta == 0u) {
+    if (red[71]) {
+      with_map([&](const auto& m) {
+#pragma unroll 1
+        for (uint32_t i = tid; i < min(a.n, (uint64_t)DIRECT_SAMPLE); i += DR_NT) {
+          const K x = sampled(i);
+          const uint32_t b = m(x);
+          if ((x != 0 && m((K)(x - 1u)) == b) || (x != key_max<K>() && m((K)(x + 1u)) == b)) continue;
+          atomicOr(&sm.pt[b >> 5], 1u << (b & 31));
+          if (ONE) sm.J[pz(b)] = i; else a.gpt[B / 32 + b] = i;  // (any of the key's)
+        }
+      });
+      __syncthreads();
+      if (ncta > 1u)
+        for (uint32_t w = tid; w < B / 32; w += DR_NT) a.gpt[w] = sm.pt[w];
+    }
+    if (tid == 0 && ncta > 1u) a.gact[B / 32 + 1] = red[71];
+  }
   if (ncta > 1u)
     for (uint32_t i = tid; i < B; i += DR_NT) {
       const uint32_t v = sm.hist[i];
@@ -737,6 +770,7 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
 
   GGMS_TRACE(3);
   // ---- scan, locate
+  const uint32_t points = ncta > 1u && tid == 0 ? __ldcg(&a.gact[B / 32 + 1]) : 0u;  // (one thread: all of them meet at one word)
   for (uint32_t w = tid; w < B / 32; w += DR_NT) {
     sm.act[w] = 0u;
     sm.big[w] = 0u;
@@ -750,6 +784,7 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
     default: scan_counts<16>(counts, sm.hist, sm.I, red); break;
   }
   static_assert(DIRECT_MAX_B == 16 * DR_NT, "the largest scan above");
+  if (ncta > 1u && tid == 0) red[71] = points;  // read behind the ks
   auto bucket_of = [&](uint32_t rank) {  // the smallest b with I[b] > rank
     uint32_t l = 0, h = B - 1u;
     while (l < h) {
@@ -776,6 +811,19 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
     for (uint32_t w = tid; w < B / 32; w += DR_NT) sm.act[w] = __ldcg(&a.gact[w]);
   }
   __syncthreads();
+  // a bucket of one key is no child; its place in hist holds a sampled position of the key
+  if (__builtin_expect(red[71] != 0u, 0)) {
+    for (uint32_t w = tid; w < B / 32; w += DR_NT) {
+      const uint32_t one = sm.act[w] & (ncta > 1u ? __ldcg(&a.gpt[w]) : sm.pt[w]);
+      sm.pt[w] = one;
+      sm.act[w] &= ~one;
+      for (uint32_t m = one; m; m &= m - 1u) {
+        const uint32_t b = w * 32u + __ffs(m) - 1u;
+        sm.hist[b] = ONE ? sm.J[pz(b)] : __ldcg(&a.gpt[B / 32 + b]);
+      }
+    }
+    __syncthreads();
+  }
   constexpr uint32_t CAP = direct_cap<K>();
   switch (B / DR_NT) {
     case 1: child_counts<1>(sm.I, sm.act, sm.J, sm.big, CAP, red); break;
@@ -800,7 +848,7 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
   auto is_big = [&](uint32_t b) { return (sm.big[b >> 5] >> (b & 31)) & 1u; };
   auto big_of = [&](uint32_t b) { return sm.bpre[b >> 5] + __popc(sm.big[b >> 5] & ((1u << (b & 31)) - 1u)); };
   GGMS_TRACE(4);
-  // Where the cursors will end, as a weighted sum per warp: when the caller
+  // Where the cursors will end, as a weighted sum: when the caller
   // changes the vector between the count and the copy they end elsewhere, and
   // the call fails.  The stores stay in the workspace: a vector's n keys lie
   // below 2 n of its place in cand[0], which cand[1] follows.  (A bound tested
@@ -826,7 +874,7 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
     }
   }
   ends = __reduce_add_sync(FULL, ends);
-  if (lane == 0) red[warp] = ends;
+  if (lane == 0) atomicAdd(&red[68], ends);
   // ids of the large children: a range of the list of all vectors'
   if (cta == 0 && tid == 0 && nbig) {
     atomicAdd(&r.C->nsegs[1], nbig);
@@ -838,21 +886,28 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
 
   GGMS_TRACE(5);
   // ---- copy
-  with_map([&](const auto& m) {
+  if (total) with_map([&](const auto& m) {
     K* cand = r.cand[0] + a.off;
     direct_stream<T, U>(a.in, a.n, cta, ncta, [&](K key) {
       const uint32_t b = m(key);
       if (active(b)) cand[atomicAdd(&sm.hist[b], 1u)] = key;
     });
   });
-  __syncthreads();
-  ends = 0;
-  for (uint32_t b = tid; b < B; b += DR_NT)
-    if (active(b)) ends += sm.hist[b] * (2u * b + 1u);
-  ends = __reduce_add_sync(FULL, ends);
-  if (lane == 0 && ends != red[warp]) set_status(r.C, GGMS_E_INTERNAL);
   GGMS_TRACE(6);
-  if (!grid_barrier(a.bar, ncta, cta == 0u, r.C, r.limit)) return false;
+  GridBarrier copied;
+  copied.arrive(a.bar, ncta, cta == 0u);
+  ends = 0;
+  for (uint32_t b = 4u * tid; b < B; b += 4u * DR_NT) {
+    const uint32_t some = (sm.act[b >> 5] >> (b & 31)) & 15u;
+    if (!some) continue;
+    const uint4 h = *reinterpret_cast<const uint4*>(&sm.hist[b]);
+    ends += (some & 1u ? h.x * (2u * b + 1u) : 0u) + (some & 2u ? h.y * (2u * b + 3u) : 0u) +
+            (some & 4u ? h.z * (2u * b + 5u) : 0u) + (some & 8u ? h.w * (2u * b + 7u) : 0u);
+  }
+  ends = __reduce_add_sync(FULL, ends);
+  if (lane == 0) atomicSub(&red[68], ends);
+  if (!copied.wait(a.bar, ncta, r.C, r.limit)) return false;
+  if (tid == 0 && red[68]) set_status(r.C, GGMS_E_INTERNAL);
   GGMS_TRACE(7);
   GGMS_TRACE_CTA(0);
 
@@ -867,6 +922,11 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
       continue;
     }
     const uint32_t b = bucket_of(rank), in = rank - (b ? sm.I[pz(b - 1)] : 0u);
+    if (__builtin_expect((sm.pt[b >> 5] >> (b & 31)) & 1u, 0)) {
+      kkey(i) = sampled(sm.hist[b]);
+      kseg(i) = K_DONE;
+      continue;
+    }
     const bool lg = is_big(b);
     krank(i) = lg ? in : (b ? sm.J[pz(b - 1)] : 0u) + in;
     kseg(i) = lg ? first_big + big_of(b) : K_SORTED;
@@ -988,6 +1048,7 @@ __global__ __launch_bounds__(DR_NT, 1) void direct_select(const __grid_constant_
   t.ghist = a.ghist;
   t.gcur = a.gcur;
   t.gact = a.gact;
+  t.gpt = a.gpt;
   t.bar = r.bar;
   t.cta = cta;
   t.ncta = ncta;

@@ -81,7 +81,7 @@ static Workspace<K> layout(const Plan& p, uint8_t* base) {
   size_t o_h0 = b.take(4ull * p.B);
   size_t o_a0 = b.take(4ull * (p.B / 32) + 4ull * p.B);
   size_t o_c0 = b.take(4ull * p.B);
-  size_t o_crow = b.take(4ull * p.B * (p.ncta ? p.ncta : 1));
+  size_t o_crow = b.take(4ull * p.B * (p.ncta ? p.ncta : 2));  // (0: the other paths' buckets of one key)
   size_t o_ic = b.take(4ull * NGRP);
   size_t o_afc = b.take(4ull * (NGRP / 32));
   size_t o_segs[2], o_cur[2], o_tiles[2], o_rows[2], o_af[2], o_cand[2], o_kh[2];
@@ -463,6 +463,7 @@ static int run_direct(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
     a.gact = w.aflag0;
     a.ghist = w.hist0;
     a.gcur = w.cmap0;
+    a.gpt = w.crow;
     a.r = refine_args<T>(w, ctx, n, nk, caps, host_out ? pin_out : out, host_out ? pin_C : nullptr);
     return launch_direct<T>(ctx, a, ctas, s);
   };
