@@ -655,11 +655,11 @@ static int run_single(Context* ctx, const T* d_in, uint64_t n, const uint32_t* k
     if (rc) return rc;
 
     // ---- refinement levels over candidates, answers
-    prof_rec(prof, 8, s);
     rc = launch_refine<T>(ctx, refine_args<T>(w, ctx, n, nk, caps, host_out ? (T*)pin_out : out,
                                               host_out || o.stats ? pin_C : nullptr), s);
     if (rc) return rc;
     if (cudaGetLastError() != cudaSuccess) return GGMS_E_CUDA;
+    prof_rec(prof, 8, s);  // nothing follows: the levels' launch writes the answers
     prof_rec(prof, 5, s);
     return GGMS_OK;
   };

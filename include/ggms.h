@@ -147,8 +147,9 @@ GGMS_API int ggms_context_pass_times(ggms_context* ctx, float* pass1_ms, float* 
  *   2 PASS 1 windows                     3 PASS 1 (count)
  *   4 between the passes (scan, locate, children, write cursors)
  *   5 PASS 2 (copy)                      6 finishing (in-shared-memory select,
- *                                          refinement levels)
- *   7 answers (write-out, copies)
+ *                                          refinement levels and, in their
+ *                                          launch, the answers)
+ *   7 what follows the answers (nothing today)
  * Returns the number of calls written (at most `max`), or -status. */
 #define GGMS_PHASES 8
 GGMS_API int ggms_context_phase_times(ggms_context* ctx, float* ms, int max);

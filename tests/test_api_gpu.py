@@ -105,6 +105,26 @@ def test_phase_times_cover_the_call():
     ctx.close()
 
 
+def test_phase_times_count_the_levels_as_finishing():
+    """2^26 keys of a mixture, 2^14 ks: nearly all keys go through a refinement
+    level, which takes far longer than what follows the answers."""
+    import torch
+    ctx = G.Context(0)
+    n = 1 << 26
+    v = D.mixture8_f32(n, 31)
+    ks = D.ks_uniform(n, 1 << 14, 5)
+    d, dk = to_device(v), to_device(ks)
+    dout = torch.empty(len(ks), dtype=torch.float32, device="cuda")
+    _, st = G.select(ctx, d.data_ptr(), n, ks, np.float32, stats=True)
+    assert st["refine_elements"] > 1 << 25
+    G.load().ggms_context_profile(ctx.ptr, 1)
+    for _ in range(3):
+        assert _dev_call(ctx, d, n, dk, len(ks), dout) == G.GGMS_OK
+    for c in ctx.phase_times(8):
+        assert c["finish"] > c["answers"]
+    ctx.close()
+
+
 @pytest.mark.parametrize("assigner", [G.ASSIGNER_SAMPLED, G.ASSIGNER_AUTO])
 def test_full_passes_are_counted(ctx, assigner):
     n = 1 << 22
