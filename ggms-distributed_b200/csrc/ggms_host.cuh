@@ -57,8 +57,8 @@ struct Context {
   uint64_t clock = 0;
   cudaStream_t capture = nullptr;  // private stream the graphs are captured on
   cudaEvent_t pin_busy = nullptr;  // recorded after the last call's uploads from the pinned buffer
-  cudaStream_t side = nullptr;     // the sampled assigner's build next to the learned one; the warp finisher
-  cudaEvent_t fork = nullptr, join = nullptr, fork2 = nullptr, join2 = nullptr;
+  cudaStream_t side = nullptr;     // the sampled assigner's build next to the learned one
+  cudaEvent_t fork = nullptr, join = nullptr;
   long long barrier_limit = 0;     // cycles a grid barrier may take (0: the default; < 0: none)
   // autotuner: launch shapes and bucket counts picked per shape class
   struct Tuned {
@@ -175,7 +175,7 @@ static void destroy_context(Context* c) {
   if (c->capture) cudaStreamDestroy(c->capture);
   if (c->pin_busy) cudaEventDestroy(c->pin_busy);
   if (c->side) cudaStreamDestroy(c->side);
-  for (cudaEvent_t e : {c->fork, c->join, c->fork2, c->join2})
+  for (cudaEvent_t e : {c->fork, c->join})
     if (e) cudaEventDestroy(e);
   cudaSetDevice(prev);
   delete c;
@@ -228,7 +228,7 @@ static cudaError_t launch_coop(void (*k)(P...), unsigned& grid, unsigned block, 
 // The side stream and its fork / join events (created on first use).
 static int ensure_side(Context* c) {
   if (!c->side) GGMS_CU(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
-  for (cudaEvent_t* e : {&c->fork, &c->join, &c->fork2, &c->join2})
+  for (cudaEvent_t* e : {&c->fork, &c->join})
     if (!*e) GGMS_CU(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   return GGMS_OK;
 }

@@ -1335,7 +1335,7 @@ __global__ __launch_bounds__(1024) void l0_children(const uint32_t* __restrict__
   sg.hi = hi;
   sg.shift = (uint32_t)max(0, bitlen((K)(hi - lo)) - RADIX_BITS);
   sg.row = kind != C_BIG ? SEG_SMALL : cbase[N_BIG] + li;
-  sg.pad = b;  // the level-0 bucket or group (l0_bases needs it)
+  sg.pad = b;  // the level-0 bucket or group (bases_body needs it)
   segs1[id] = sg;
   cursor1[id] = 0u;
   khead1[id] = K_NIL;
@@ -1523,15 +1523,8 @@ __device__ __forceinline__ void bases_body(uint32_t* crow, uint32_t B, uint32_t 
   }
 }
 
-template <typename K>
-__global__ void l0_bases(uint32_t* crow, uint32_t B, uint32_t ncta, const Seg<K>* __restrict__ segs1,
-                         const Counters* __restrict__ C, Caps caps) {
-  pdl_entry();
-  bases_body<K>(crow, B, ncta, segs1, C, caps);
-}
-
 // After l0_children: the ks follow their level-0 child (relabel_one) and the
-// per-CTA write cursors of PASS 2 are formed (l0_bases), in one launch --
+// per-CTA write cursors of PASS 2 are formed (bases_body), in one launch --
 // threads [0, nk) relabel, all warps then take children for the cursors.
 template <typename K>
 __global__ void l0_relabel_bases(const uint32_t* __restrict__ cmap0, uint32_t nk,
@@ -1899,7 +1892,7 @@ __host__ __device__ constexpr uint32_t coarse_chunk() {
 }
 
 // PASS 2 of the coarse mode.  Same element -> CTA assignment as PASS 1; CTA
-// c's range of group g starts at crow[c][g << gsh] (l0_bases).  Per chunk: the
+// c's range of group g starts at crow[c][g << gsh] (bases_body).  Per chunk: the
 // group of every key (bucket >> gsh), its rank among the chunk's keys of that
 // group (a shared atomic), a scan of the NGRP counts, the keys into shared
 // memory in group order, then thread i stores staged key i -- consecutive
@@ -2076,9 +2069,8 @@ __global__ __launch_bounds__(NT, PASS_MIN_CTAS(NT)) void l0_compact_coarse(const
 // ------------------------------------------------------------------ refinement levels
 // Level l works on the segments of pool p = l & 1 and creates children in pool
 // q = p ^ 1.  Keys are read from `src` and children are written to `dst`.
-// The steps are device functions over (cta, ncta), so that the batched level 0
-// can launch them as kernels and refine_levels runs them all in one launch.
-// In that launch one step reads what another CTA wrote in an earlier one, so
+// The steps are device functions over (cta, ncta): refine_body runs them all in
+// one launch, in which one step reads what another CTA wrote in an earlier one, so
 // their pointers to scratch are not __restrict__ (no non-coherent loads).
 
 // zero this level's histogram rows / flags (segments that small_select or
