@@ -1,28 +1,31 @@
-// ggms_direct.cuh -- one vector in one launch: the path of vectors that fit
-// the L2 cache.
+// ggms_direct.cuh -- one vector in one launch: the path of vectors whose second
+// read comes from the L2 cache, all or most of it (up to 160 MB; fewer keys with
+// many ks: direct_ok).
 //
 // The two-pass pipeline (ggms_engine.cuh) spends ~100 us around its passes on
 // chains of one-CTA kernels (sample sort, model, windows, scan, children,
-// finishers), which is repaid only when the passes themselves are long.  For a
-// vector that the L2 cache holds a re-read costs little, so this path keeps
-// the shape (sample -> buckets -> count -> copy -> finish) and drops the
-// chain: one cooperative launch, three grid barriers, and between the barriers
-// every CTA computes the same small things for itself instead of waiting for
-// one CTA to compute them.
+// finishers), which is repaid only when the passes themselves are long.  For
+// such a vector a re-read costs little, so this path keeps the shape (sample ->
+// buckets -> count -> copy -> finish) and drops the chain: one cooperative
+// launch of four grid barriers (five with many ks, more when large children are
+// left), and between the barriers every CTA computes the same small things for
+// itself instead of waiting for one CTA to compute them.
 //
 //   1. every CTA draws the same sample (up to 4096 keys), histograms it over
 //      2048 cells uniform in key between its extremes, and turns the cells'
 //      prefix sums into a piecewise-linear map key -> bucket (DirectMap);
 //   2. it counts its share of the input into a shared-memory histogram and
-//      adds that to the global one (barrier);
-//   3. it scans the global histogram, locates the ks, and knows the buckets
+//      adds that to the global one, which all have zeroed meanwhile (a barrier
+//      before and one after);
+//   3. it scans the global histogram, locates the ks (many ks: its own, and a
+//      barrier), and knows the buckets
 //      holding a k (the children) and where each child's keys go in a compact
 //      candidate array;
 //   4. it reserves a range of every child it holds keys of (one global atomic
 //      per child), re-reads its share and copies the keys (barrier);
 //   5. the candidate array is in key order up to the order inside each child:
-//      every CTA sorts an equal part of it, whole children at a time, and every
-//      k reads its answer at its position (barrier).
+//      every CTA sorts an equal part of it, whole children at a time (barrier),
+//      and every k reads its answer at its position.
 //
 // Step 5 sorts where a selection would do: with children of a few dozen keys a
 // selection per k pays for its k lists and histograms whatever the size (2^22

@@ -50,7 +50,9 @@ enum {
 /* ---- level-0 bucket assigners ---- */
 enum {
   GGMS_ASSIGNER_AUTO = 0,        /* learned PL-CDF, sampled pivots if its imbalance is over the bound; vectors
-                                    of up to 160 MB with no other field set: one launch, sampled cells */
+                                    of up to 160 MB (20 Mi elements with more than 512 ks, 12 Mi with
+                                    more than 2048, but for top-k) and up to 65536 ks, with no other
+                                    field set: one launch, sampled cells */
   GGMS_ASSIGNER_SAMPLED = 1,     /* sampled pivots + per-segment slopes (the reference's method) */
   GGMS_ASSIGNER_LEARNED_PL = 2,  /* monotone piecewise-linear CDF, trained on the GPU */
   GGMS_ASSIGNER_LEARNED_MLP = 3  /* monotone 1-32-32-1 MLP CDF, trained on the GPU */
@@ -99,7 +101,7 @@ typedef struct ggms_opts {
   float window_z;               /* PASS 1 windows: safety margin of the predicted k positions in
                                    binomial standard deviations; 0 = 6; < 0 = no windows */
   int32_t autotune;             /* 1: when num_buckets and the pass shape are left at 0, the first call of a
-                                   shape class times the candidates on the caller's data and the context
+                                   shape class times the candidates (the one launch among them) on the caller's data and the context
                                    keeps the fastest (the batched path has nothing to tune) */
   ggms_stats* stats;            /* optional host pointer */
   int32_t pl_knots;             /* segments of the learned piecewise-linear CDF model: 16..1024;
@@ -120,7 +122,7 @@ GGMS_API int ggms_version(void);
  *
  * Some kernels are cooperative launches: their CTAs meet at barriers, so such a
  * kernel starts when all of them have room, and beside a long kernel of another
- * stream it waits for that.  Vectors of up to 160 MB and batched calls take one
+ * stream it waits for that.  Calls of one launch (AUTO) and batched calls take one
  * CTA of 1024 threads and up to 225 KB of shared memory on every SM (fewer for
  * vectors below 148 K elements), the refinement levels two of 512 threads and
  * 80 KB.  On a stream with fewer SMs (a green context) they take what it has. */
