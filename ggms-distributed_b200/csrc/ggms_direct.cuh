@@ -34,8 +34,11 @@
 // refinement levels.
 // A bucket that only one key can be in (integers of a small range, floats in a
 // few units of the last place: more buckets than keys) is no child: its key is
-// its ks' answer.  Buckets whose keys turn out to be one value cost one
-// refinement level: the level starts from the children's true key range.
+// its ks' answer.  A large child whose keys turn out to be one value (floats of
+// 16-bit precision) answers its ks once its true key range is known, and the
+// levels, which start from that range, do not read it (40 M fp32, half of them
+// zero, one k: 289 us, 329 with a level over them; 19 M of bfloat16 precision,
+// 2000 ks: 835 and 919).
 //
 // A vector that fits one CTA's sort (32 KB) is sorted by it (direct_sort):
 // nothing else is as short.
@@ -1007,15 +1010,16 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
       const uint32_t b = w * 32u + __ffs(m) - 1u, id = first_big + big_of(b);
       if (id >= r.caps.rows || id >= r.caps.segs) continue;
       const uint32_t off = b ? sm.J[pz(b - 1)] : 0u, cnt = sm.J[pz(b)] - off;
-      const uint32_t nt = (cnt + TILE - 1) / TILE;
+      const uint32_t nt = (cnt + TILE - 1) / TILE, t0 = (cta + ncta - dealt % ncta) % ncta;
+      dealt += nt;
+      if (t0 >= nt) continue;
       K mn = key_max<K>(), mx = 0;
-      for (uint32_t t = (cta + ncta - dealt % ncta) % ncta; t < nt; t += ncta)
+      for (uint32_t t = t0; t < nt; t += ncta)
         for (uint32_t i = t * TILE + tid; i < min(cnt, (t + 1u) * TILE); i += DR_NT) {
           const K x = r.cand[0][a.off + off + i];
           mn = min(mn, x);
           mx = max(mx, x);
         }
-      dealt += nt;
       mn = warp_min(mn);
       mx = warp_max(mx);
       if (lane == 0 && mn <= mx) {
@@ -1027,6 +1031,15 @@ __device__ __forceinline__ bool direct_body(const DirectTask<T>& a, const Refine
   for (uint32_t j = first_big + gt; j < min(first_big + nbig, min(r.caps.rows, r.caps.segs)); j += gs) {
     Seg<K>& s = r.segs[1][j];
     s.shift = (uint32_t)max(0, bitlen((K)(__ldcg(&s.hi) - __ldcg(&s.lo))) - RADIX_BITS);
+  }
+  // a child of one value answers its ks; the levels skip its tiles
+  for (uint32_t i = gt; i < nk; i += gs) {
+    const uint32_t id = kseg(i);
+    if (id >= min(r.caps.rows, r.caps.segs)) continue;  // resolved
+    const K lo1 = __ldcg(&r.segs[1][id].lo);
+    if (lo1 != __ldcg(&r.segs[1][id].hi)) continue;
+    kkey(i) = lo1;
+    kseg(i) = K_DONE;
   }
   return true;
 }

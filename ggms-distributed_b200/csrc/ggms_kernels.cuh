@@ -2154,6 +2154,7 @@ __device__ __forceinline__ void count_body(const K* src, const Seg<K>* segs, con
     const TileRef tr = tiles[t];
     if (tr.seg >= ns) continue;  // only after a capacity error (status already set)
     const Seg<K> s = segs[tr.seg];
+    if (s.lo == s.hi) continue;  // one value: its ks are answered (direct_body)
     if (tr.seg != open) {  // (no barrier between a segment's tiles: the warps run on into the next one's loads)
       if (open != 0xFFFFFFFFu) {
         flush();
@@ -2309,6 +2310,7 @@ __device__ __forceinline__ void compact_body(const K* src, const Seg<K>* segs, c
     const TileRef tr = tiles[t];
     if (tr.seg >= ns) continue;  // only after a capacity error (status already set)
     const Seg<K> s = segs[tr.seg];
+    if (s.lo == s.hi) continue;  // one value
     if (tr.seg != loaded) {
       const uint32_t* row = rows + (size_t)s.row * NBIN;
       __syncthreads();
