@@ -37,6 +37,11 @@ namespace ggms {
 // BT_FEW rows per SM only for the shortest (126 rows of 900 fp32 keys: 52 us by
 // warps, 8 by CTAs).
 constexpr uint32_t BT_ROW0 = 1024, BT_ROW_FEW = 256, BT_FEW = 4;
+// ks of a segment that one CTA selects one by one, where it would sort the
+// segment for more.  3000 segments of 3000 fp32 keys, us for 1 / 2 / 3 ks and for
+// the sort: normal 134 / 176 / 221 / 261, with ties 164 / 238 / 311 / 331; of 8000
+// keys 159 / 213 / 262 / 462.
+constexpr uint32_t BT_SELECT_KS = 3;
 
 template <typename T>
 struct BatchArgs {
@@ -241,19 +246,102 @@ __global__ __launch_bounds__(DR_NT, 1) void batch_singles(const __grid_constant_
   direct_body<T, true, 4>(task, a.r, smem);
 }
 
-// Segments of one CTA's sort.
+// The m keys of the CTA's registers that lie in [lo, hi], counted into 1024 bins
+// uniform in key; thread t gets bin t's count and the inclusive count up to it.
+// h: 1024 words, red: 32.  All threads call it; ends with a barrier.
+template <typename K, int R>
+__device__ __forceinline__ uint2 cta_bins(const K (&k)[R], uint32_t m, K lo, K hi, uint32_t* h, uint32_t* red) {
+  const uint32_t tid = threadIdx.x;
+  static_assert(DR_NT == 1 << 10, "a bin per thread");
+  const int sh = max(0, bitlen((K)(hi - lo)) - 10);
+  h[tid] = 0u;
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < R; ++j)
+    if (tid + j * DR_NT < m && k[j] >= lo && k[j] <= hi) atomicAdd(&h[(uint32_t)((K)(k[j] - lo) >> sh)], 1u);
+  __syncthreads();
+  const uint32_t c = h[tid];
+  uint32_t v[1] = {c};
+  block_scan_regs<1>(v, red);
+  return make_uint2(c, v[0]);
+}
+
+// The key of rank r among those m keys in [lo, hi], whose bins are `b`: the bin
+// of the rank is counted again, until it holds one key or one value.  red: 35.
+template <typename K, int R>
+__device__ __forceinline__ K cta_select(const K (&k)[R], uint32_t m, uint32_t r, K lo, K hi, uint2 b, uint32_t* h,
+                                        uint32_t* red, K* one) {
+  const uint32_t tid = threadIdx.x;
+  while (lo < hi) {
+    const int sh = max(0, bitlen((K)(hi - lo)) - 10);
+    __syncthreads();  // (red is read until here)
+    if (b.y > r && b.y - b.x <= r) {
+      red[32] = tid;
+      red[33] = b.y - b.x;
+      red[34] = b.x;
+    }
+    __syncthreads();
+    const K w = (K)(((K)1 << sh) - 1);
+    lo = (K)(lo + ((K)red[32] << sh));
+    if ((K)(hi - lo) > w) hi = (K)(lo + w);
+    r -= red[33];
+    if (red[34] == 1u && lo < hi) {
+#pragma unroll
+      for (int j = 0; j < R; ++j)
+        if (tid + j * DR_NT < m && k[j] >= lo && k[j] <= hi) *one = k[j];
+      __syncthreads();
+      return *one;
+    }
+    if (lo < hi) b = cta_bins(k, m, lo, hi, h, red);
+  }
+  return lo;
+}
+
+// Segments of one CTA's sort; with up to BT_SELECT_KS ks a selection each.
 template <typename T>
 __global__ __launch_bounds__(DR_NT, 1) void batch_sorts(const __grid_constant__ BatchArgs<T> a) {
   using K = typename KeyOf<T>::K;
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ K red_k[2][DR_NT / 32];
   SortSmem<K>& sm = *reinterpret_cast<SortSmem<K>*>(smem);
+  __shared__ uint32_t red[35], ks_s[BT_SELECT_KS];
+  __shared__ K one;
   K* sorted = reinterpret_cast<K*>(smem + sizeof(SortSmem<K>));
   const uint32_t m = a.r.C->nlist[BT_SORT];
   for (uint32_t j = blockIdx.x; j < m; j += gridDim.x) {
     bool bad = false;
     const SegRange g = seg_range(a, a.lists[(size_t)BT_SORT * a.nseg + j], &bad);
     const T* in = a.in + g.off;
+    if (g.nk <= BT_SELECT_KS) {
+      constexpr int R = (int)(direct_cap<K>() / DR_NT);
+      K k[R], mn = key_max<K>(), mx = 0;
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const uint32_t i = threadIdx.x + q * DR_NT;
+        if (i < g.cnt) k[q] = KeyOf<T>::to(in[i]);
+      }
+#pragma unroll
+      for (int q = 0; q < R; ++q)
+        if (threadIdx.x + q * DR_NT < g.cnt) {
+          mn = min(mn, k[q]);
+          mx = max(mx, k[q]);
+        }
+      if (threadIdx.x < g.nk) ks_s[threadIdx.x] = a.ks[g.k0 + threadIdx.x];  // (the same k for all threads)
+      block_extremes(mn, mx, red_k);
+      const uint2 all = cta_bins(k, g.cnt, mn, mx, &sm.hist[0][0], red);
+      for (uint32_t i = 0; i < g.nk; ++i) {
+        const uint32_t kk = ks_s[i];
+        const bool ok = kk >= 1u && kk <= g.cnt;
+        const K key = ok ? cta_select(k, g.cnt, g.cnt - kk, mn, mx, all, &sm.hist[0][0], red, &one) : (K)0;
+        if (threadIdx.x == 0) {
+          if (ok) a.r.kkey[g.k0 + i] = key;
+          else set_status(a.r.C, GGMS_E_INVALID_ARG);
+          a.r.kseg[g.k0 + i] = K_DONE;
+        }
+      }
+      __syncthreads();
+      continue;
+    }
     sort_keys<K>(sm, g.cnt, red_k, [&](uint32_t i) { return KeyOf<T>::to(in[i]); },
                  [&](uint32_t i, K key) { sorted[i] = key; });
     for (uint32_t i = threadIdx.x; i < g.nk; i += DR_NT) {
